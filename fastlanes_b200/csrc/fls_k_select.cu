@@ -31,7 +31,6 @@ constexpr int      K        = FLS_SEL_K;
 constexpr int      NF       = FLS_SEL_FEATURES;
 constexpr int      H        = FLS_SEL_HIDDEN;
 constexpr uint64_t kEmpty   = ~0ull;      // empty key of the hash tables; the value ~0 itself has a slot of its own
-constexpr uint32_t kNoPos   = 0xFFFFFFFFu;
 constexpr uint32_t kMaxVecPerChunk = 64;
 constexpr int      kWarps   = 8;
 
@@ -119,6 +118,7 @@ __device__ __forceinline__ void load_run(const Col& c, uint64_t v, uint32_t lane
 struct Parts {
 	uint32_t bw_f, bw_d, bw_i, runs;
 	uint32_t start_mask; // this thread's run starts (bit i: original position R(t) + i starts a run)
+	uint64_t lo, hi;     // lowest and highest value, in the column's order (signed: the top bit flipped)
 };
 
 template <int W>
@@ -137,6 +137,8 @@ __device__ __forceinline__ Parts vector_parts(const typename UT<W>::T (&x)[32], 
 	mn     = warp_min(mn);
 	mx     = warp_max(mx);
 	P.bw_f = bits_of(static_cast<uint64_t>(static_cast<T>(mx - mn)));
+	P.lo   = mn;
+	P.hi   = mx;
 	// DELTA: the unrsum chains of the transposed layout visit a lane's values in ascending original order, so
 	// a chain is a run of contiguous original positions (W = 32: this thread's 32; W = 64: 64, this thread's
 	// and its partner's); every chain's first difference is 0
@@ -353,29 +355,52 @@ __device__ void vector_features(const typename UT<W>::T (&x)[32], uint32_t lane,
 // ---------------------------------------------------------------------------------------------------------
 // Kernels over work items (warp per vector)
 // ---------------------------------------------------------------------------------------------------------
+// What k_parts notes of every vector for the chunk dictionary: in the column's order (signed columns with the top bit
+// flipped) its lowest, highest, first and last value, its runs and whether its values never fall.
+struct VecInfo {
+	uint64_t lo, hi, first, last;
+	uint32_t runs, sorted;
+};
+
+template <int W>
+__device__ __forceinline__ void note_vector(const typename UT<W>::T (&x)[32], uint32_t lane, bool sgn, const Parts& P,
+                                            VecInfo* out) {
+	using T         = typename UT<W>::T;
+	const T  flip   = sgn ? (T(1) << (W - 1)) : T(0);
+	const T  prev   = __shfl_sync(0xFFFFFFFFu, x[31], prev_run_lane(lane));
+	bool     falls  = lane > 0 && (x[0] ^ flip) < (prev ^ flip);
+#pragma unroll
+	for (int i = 1; i < 32; ++i) { falls |= (x[i] ^ flip) < (x[i - 1] ^ flip); }
+	falls        = __any_sync(0xFFFFFFFFu, falls);
+	const T last = __shfl_sync(0xFFFFFFFFu, x[31], lane_of_virtual(31));
+	if (lane == 0) { *out = VecInfo {P.lo, P.hi, static_cast<uint64_t>(x[0] ^ flip), static_cast<uint64_t>(last ^ flip), P.runs, falls ? 0u : 1u}; }
+}
+
 struct ItemArgs {
 	const Col*  cols;
 	const Item* items;
 	uint64_t    n_items;
 };
 
-__global__ void __launch_bounds__(kWarps * 32) k_parts(ItemArgs a, uint32_t* parts) {
+__global__ void __launch_bounds__(kWarps * 32) k_parts(ItemArgs a, uint32_t* parts, VecInfo* info) {
 	const uint32_t lane = threadIdx.x & 31u;
 	for (uint64_t it = blockIdx.x * static_cast<uint64_t>(kWarps) + (threadIdx.x >> 5); it < a.n_items;
 	     it += static_cast<uint64_t>(gridDim.x) * kWarps) {
 		const Item m = a.items[it];
 		const Col  c = a.cols[m.col];
-		uint32_t   pk;
 		if (c.width == 64) {
 			uint64_t x[32];
 			load_run<64>(c, m.vec, lane, x);
-			pk = pack_parts(vector_parts<64>(x, lane, c.sgn != 0));
+			const Parts P = vector_parts<64>(x, lane, c.sgn != 0);
+			if (lane == 0) { parts[it] = pack_parts(P); }
+			if (info) { note_vector<64>(x, lane, c.sgn != 0, P, info + it); }
 		} else {
 			uint32_t x[32];
 			load_run<32>(c, m.vec, lane, x);
-			pk = pack_parts(vector_parts<32>(x, lane, c.sgn != 0));
+			const Parts P = vector_parts<32>(x, lane, c.sgn != 0);
+			if (lane == 0) { parts[it] = pack_parts(P); }
+			if (info) { note_vector<32>(x, lane, c.sgn != 0, P, info + it); }
 		}
-		if (lane == 0) { parts[it] = pk; }
 	}
 }
 
@@ -412,31 +437,63 @@ __global__ void __launch_bounds__(kWarps * 32) k_features(ItemArgs a, float* fea
 
 // ---------------------------------------------------------------------------------------------------------
 // Dictionary of a chunk (wizard), one CTA per chunk: the chunk's distinct values, numbered in first-occurrence
-// order (src/cor/lyt/dic/dic_fac.cpp:19-40), give the dictionary size and every vector's code bit width.
-//   table     open addressing in shared memory (16 Ki slots), first position of every key by atomicMin.  A
-//             chunk with more than kCdCap distinct values is split by hash into kCdParts buckets instead: one
-//             read of the values scatters (key, position) pairs into the CTA's bucket scratch in global memory
-//             (each bucket has room for the whole chunk), and every bucket (about 1/8 of the keys) goes
-//             through the shared-memory table in turn, read back coalesced;
-//   ranks     every key's first position sets a bit in the chunk's position bitmap (64 Ki bits, shared memory);
-//             popcounts of the bitmap words, scanned, rank the first positions: a value's code;
-//   codes     every value's code (the values again, or the buckets again), the code range of each vector.
-// Exact for every chunk.
+// order (src/cor/lyt/dic/dic_fac.cpp:19-40), give the dictionary size and every vector's code bit width.  Codes
+// rise with the first position, so a vector's code range is the rank of the largest first position among its values
+// minus that of the smallest: two ranks a vector (popcounts of the bitmap of first positions), none a value.
+//   sorted    a chunk whose values never fall (k_parts says) needs no table: every run is a new code;
+//   direct    a chunk whose values span fewer than 47 Ki keeps first positions by value - lowest, no hash;
+//   unique    a chunk of nearly all different values: every run start sets a bit of a 1 Mbit filter by its hash; the
+//             few that find theirs set mark a coarser filter, and only the values whose mark is set (a few percent)
+//             need the table: the others are the only ones of their kind, their first position is their own;
+//   table     47 Ki slots of 32 bits in shared memory, open addressing: 16 bits of the key's hash and the 16-bit
+//             position of its first occurrence seen so far (the chunk's values stay in L2, so the key itself is read
+//             back from that position when the hash bits agree).  A slot of 4 bytes instead of a 64-bit key and a
+//             position (12) is what lets one table hold most of a chunk of distinct values;
+//   queue     a warp takes whole vectors, and every step looks at one slot for each of 32 keys from the warp's queue
+//             in shared memory; keys that have to look further go back on it.  So runs, other parts' keys and long
+//             probes cost no idle lanes (a loop of its own for every warp of keys went round for its unluckiest
+//             lane, 200 to 300 instructions a step);
+//   parts     a chunk of more distinct values goes through the table in parts of the hash space (2, then 4, ...);
+//             the count beside the rows done says early whether it will.
+// Exact for every chunk.  Instruction-bound.  28 integer columns (30 M values, 462
+// chunks): 1,855 us with 16 Ki slots of keys and positions and a bucket pass through global memory, 284 us so; 5.7 M
+// string hashes (90 chunks): 710 us, 138 us.
 // ---------------------------------------------------------------------------------------------------------
-constexpr uint32_t kCdSlots  = 1u << 14;
-constexpr uint32_t kCdCap    = 12288; // distinct values the shared-memory table takes (a load of 3/4)
-constexpr uint32_t kCdParts  = 8;     // buckets of a chunk of more distinct values (8 x 12288 > 65,536)
-constexpr uint32_t kCdBucket = kMaxVecPerChunk * 1024;  // room of a bucket: the whole chunk
-constexpr int      kCdWarps  = 16;
-constexpr uint32_t kCdWords  = kMaxVecPerChunk * 1024 / 32;
-constexpr uint32_t kCdSmem   = kCdSlots * 8 + (kCdSlots + 1) * 4 + 2 * kCdWords * 4 + 2 * kMaxVecPerChunk * 4;
-constexpr uint64_t kCdGBytes = static_cast<uint64_t>(kCdParts) * kCdBucket * 12; // per CTA: keys, then positions
-static_assert(kCdSmem <= 227 * 1024, "chunk dictionary tables fit one CTA");
-static_assert(kMaxVecPerChunk <= 4 * kCdWarps, "at most 4 vectors of a chunk per warp");
+constexpr uint32_t kCdThreads = 1024;
+constexpr uint32_t kCdWarps   = kCdThreads / 32;
+constexpr uint32_t kCdSlots   = 47 * 1024;
+constexpr uint32_t kCdCap     = 43 * 1024; // keys the table takes (eleven twelfths), and those in flight
+constexpr uint32_t kCdMaxParts = 256;
+constexpr uint32_t kCdMaxSteps = 1u << 20; // a warp's steps in a part; never reached: the table has free slots
+constexpr uint32_t kCdWords   = kMaxVecPerChunk * 1024 / 32;
+constexpr uint32_t kCdFree    = 0xFFFFFFFFu;
+constexpr uint64_t kCdGBytes  = kMaxVecPerChunk * 1024 * 2; // per CTA: the slots of every vector's keys
+// unique: the filter (2^20 bits) lies where the table of the marked values then goes; behind it the marks (2^18 bits)
+constexpr uint32_t kCdUniqueSlots = 32 * 1024;
+constexpr uint32_t kCdMarkWords   = 8 * 1024;
+constexpr uint32_t kCdUniqueMax   = 8 * 1024;  // values that may find their bit set; marked are about twice as many
+constexpr uint32_t kCdUniqueCap   = 28 * 1024; // keys its table takes (keys chosen to share marks could be more)
+static_assert(kCdUniqueSlots + kCdMarkWords <= kCdSlots, "filter and marks lie in the table's space");
+static_assert(kCdCap + 2 * kCdThreads < kCdSlots && kCdSlots < 0xFFFFu, "free slots always; slots in 16 bits");
+
+struct ChunkDictSmem {
+	uint32_t table[kCdSlots]; // at the end: the exclusive prefix of the bitmap words' popcounts
+	uint32_t bits[kCdWords];  // first positions
+	uint64_t qkey[kCdWarps][64];
+	uint16_t qpos[kCdWarps][64], qslot[kCdWarps][64], qtag[kCdWarps][64];
+	uint32_t vrange[kMaxVecPerChunk][2]; // smallest and largest first position of a vector's values
+	uint32_t wsum[33];
+	uint32_t chunk, over, count, mode, distinct;
+	uint64_t lo;    // direct: the lowest value
+	uint64_t dw[2]; // weights of the first positions
+};
+static_assert(sizeof(ChunkDictSmem) <= 227 * 1024, "chunk dictionary tables fit one CTA");
+enum : uint32_t { CD_SORTED, CD_DIRECT, CD_UNIQUE /* to be tried */, CD_TABLE };
 
 struct ChunkDictArgs {
 	const Col*      cols;
 	const Item*     items;       // the chunks' vectors, chunk by chunk
+	const VecInfo*  info;        // per item
 	const uint32_t* chunk_items; // item range of every chunk (n_chunks + 1)
 	uint32_t        n_chunks;
 	uint32_t*       dict_n;  // per chunk: distinct values
@@ -448,298 +505,439 @@ struct ChunkDictArgs {
 	const uint32_t* const* w0;
 	const uint32_t* const* w1;
 	uint64_t*       dict_w;
-	uint8_t*        gtab; // gridDim.x regions of kCdGBytes: the CTAs' bucket scratch
+	uint16_t*       gslots; // gridDim.x regions of kCdGBytes
+	uint32_t*       ticket; // zero: the next chunk to take
 };
 
-// 64-bit finaliser of MurmurHash3 (Appleby): the slot from the low bits.
-__device__ __forceinline__ uint64_t cd_mix(uint64_t x) {
-	x ^= x >> 33;
-	x *= 0xff51afd7ed558ccdull;
-	x ^= x >> 33;
-	x *= 0xc4ceb9fe1a85ec53ull;
-	x ^= x >> 33;
-	return x;
+// A key's hash: *place places it (its top bits choose the part), *tag is what its slot keeps in the upper half (never
+// all ones, so that no slot reads as free).  32-bit keys: the 32-bit finaliser of MurmurHash3 (Appleby), a bijection.
+__device__ __forceinline__ void cd_hash(uint32_t x, uint32_t* place, uint32_t* tag) {
+	x ^= x >> 16;
+	x *= 0x85ebca6bu;
+	x ^= x >> 13;
+	x *= 0xc2b2ae35u;
+	x ^= x >> 16;
+	*place           = x;
+	const uint32_t t = x << 16;
+	*tag             = t == 0xFFFF0000u ? 0u : t;
+}
+// 64-bit keys: two linear combinations of the halves by odd constants, the one that places mixed as above.
+__device__ __forceinline__ void cd_hash(uint64_t x, uint32_t* place, uint32_t* tag) {
+	const uint32_t lo = static_cast<uint32_t>(x), hi = static_cast<uint32_t>(x >> 32);
+	uint32_t       a  = lo * 0x9E3779B1u + hi * 0x85EBCA77u;
+	const uint32_t t  = (lo * 0xC2B2AE3Du + hi * 0x27D4EB2Fu) & 0xFFFF0000u;
+	a ^= a >> 15;
+	a *= 0x2C1B3C6Du;
+	a ^= a >> 13;
+	*place = a;
+	*tag   = t == 0xFFFF0000u ? 0u : t;
 }
 
-// Slot of x in a table of mask + 1 slots (inserted when absent; *count counts new keys): mask + 1 for the key
-// ~0 (a slot of its own), mask + 2 when `limit` probes found neither x nor an empty slot.
-__device__ __forceinline__ uint32_t cd_insert(uint64_t* keys, uint32_t mask, uint64_t x, uint32_t* count,
-                                              uint32_t limit) {
-	if (x == kEmpty) { return mask + 1; }
-	uint32_t s = static_cast<uint32_t>(cd_mix(x)) & mask;
-	for (uint32_t probe = 0; probe < limit; ++probe) {
-		const uint64_t k = *reinterpret_cast<volatile uint64_t*>(keys + s);
-		if (k == x) { return s; }
-		if (k == kEmpty) {
-			const uint64_t old = atomicCAS(reinterpret_cast<unsigned long long*>(keys + s), kEmpty, x);
-			if (old == kEmpty) {
-				atomicAdd(count, 1u);
-				return s;
-			}
-			if (old == x) { return s; }
+// One look at slot *s for value x at position pos: done (it is the key's slot now) or not (*s is the next one).
+template <class T>
+__device__ __forceinline__ bool cd_step(uint32_t* table, uint32_t n_slots, const T* vals, T x, uint32_t pos, uint32_t tag,
+                                        uint32_t* s, bool* fresh) {
+	uint32_t e = *reinterpret_cast<volatile uint32_t*>(table + *s);
+	if (e == kCdFree) {
+		e = atomicCAS(table + *s, kCdFree, tag | pos);
+		if (e == kCdFree) {
+			*fresh = true;
+			return true;
 		}
-		s = (s + 1) & mask;
 	}
-	return mask + 2;
+	if ((e ^ tag) < 0x10000u && __ldg(vals + (e & 0xFFFFu)) == x) {
+		if (pos < (e & 0xFFFFu)) { atomicMin(table + *s, tag | pos); }
+		return true;
+	}
+	*s = *s + 1 == n_slots ? 0 : *s + 1;
+	return false;
 }
 
-__device__ __forceinline__ uint32_t cd_find(const uint64_t* keys, uint32_t mask, uint64_t x) {
-	if (x == kEmpty) { return mask + 1; }
-	uint32_t s = static_cast<uint32_t>(cd_mix(x)) & mask;
-	for (uint32_t probe = 0; probe <= mask; ++probe) {
-		const uint64_t k = keys[s];
-		if (k == x) { return s; }
-		if (k == kEmpty) { break; }
-		s = (s + 1) & mask;
+// A warp's queue of keys on their way into the table, and the list of the slots they ended in (the current vector's).
+template <class T>
+struct CdQueue {
+	T*         key;
+	uint16_t * pos, *slot, *tag;
+	uint16_t*  list;
+	uint32_t   q, n; // keys queued, slots listed
+
+	__device__ __forceinline__ void push(bool take, T x, uint32_t at_pos, uint32_t s, uint32_t t, uint32_t lane) {
+		const uint32_t m = __ballot_sync(0xFFFFFFFFu, take);
+		if (take) {
+			const uint32_t at = q + __popc(m & ((1u << lane) - 1u));
+			key[at]           = x;
+			pos[at]           = static_cast<uint16_t>(at_pos);
+			slot[at]          = static_cast<uint16_t>(s);
+			tag[at]           = static_cast<uint16_t>(t >> 16);
+		}
+		q += __popc(m);
+		__syncwarp();
 	}
-	return mask + 2;
+	// One look for every lane's key (those of `have`); the unfinished ones go on the queue.  Returns the new keys.
+	__device__ __forceinline__ uint32_t look(uint32_t* table, uint32_t n_slots, const T* vals, bool have, T x,
+	                                         uint32_t at_pos, uint32_t s, uint32_t t, uint32_t lane) {
+		bool fresh = false, done = false;
+		if (have) { done = cd_step<T>(table, n_slots, vals, x, at_pos, t, &s, &fresh); }
+		const uint32_t m = __ballot_sync(0xFFFFFFFFu, done);
+		if (done) { list[n + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(s); }
+		n += __popc(m);
+		push(have && !done, x, at_pos, s, t, lane);
+		return __popc(__ballot_sync(0xFFFFFFFFu, fresh));
+	}
+	// The last up to 32 queued keys take a look each.
+	__device__ __forceinline__ uint32_t pop(uint32_t* table, uint32_t n_slots, const T* vals, uint32_t lane) {
+		const uint32_t take = q < 32 ? q : 32;
+		q -= take;
+		const bool     have = lane < take;
+		const uint32_t at   = q + (have ? lane : 0u);
+		const T        x    = key[at];
+		const uint32_t p = pos[at], s = slot[at], t = static_cast<uint32_t>(tag[at]) << 16;
+		__syncwarp(); // read before the unfinished ones are written back
+		return look(table, n_slots, vals, have, x, p, s, t, lane);
+	}
+};
+
+// How the chunk of items [i0, i0 + nv) is done (warp 0; CD_*), from its vectors' notes.
+__device__ __forceinline__ void cd_choose(const ChunkDictArgs& a, uint32_t i0, uint32_t nv, uint32_t lane,
+                                          ChunkDictSmem& S) {
+	uint64_t lo = ~0ull, hi = 0;
+	uint32_t runs = 0, borders = 0, unsorted = 0;
+	for (uint32_t v = lane; v < nv; v += 32) {
+		const VecInfo m = a.info[i0 + v];
+		lo              = m.lo < lo ? m.lo : lo;
+		hi              = m.hi > hi ? m.hi : hi;
+		runs += m.runs;
+		unsorted |= m.sorted ? 0u : 1u;
+		if (v + 1 < nv) { // a run across the border of two vectors is one code
+			const uint64_t next = a.info[i0 + v + 1].first;
+			unsorted |= next < m.last ? 1u : 0u;
+			borders += next == m.last ? 1u : 0u;
+		}
+	}
+	lo       = warp_min(lo);
+	hi       = warp_max(hi);
+	runs     = warp_sum(runs);
+	borders  = warp_sum(borders);
+	unsorted = __any_sync(0xFFFFFFFFu, unsorted != 0);
+	if (lane == 0) {
+		S.lo       = lo;
+		S.distinct = runs - borders; // of a sorted chunk
+		// fewer runs than the table takes in one part with room to spare go straight to it
+		S.mode = !unsorted && !a.w0 ? CD_SORTED : hi - lo < kCdSlots ? CD_DIRECT : runs > kCdCap / 2 ? CD_UNIQUE : CD_TABLE;
+	}
 }
 
 template <int W>
-__device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& col, uint32_t c, uint64_t* keys,
-                                           uint32_t* first, uint32_t* bits, uint32_t* pref, uint32_t* vrange,
-                                           uint32_t* s_count, uint32_t* s_over, uint32_t* s_wsum, uint64_t* s_dw) {
+__device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& col, uint32_t c, ChunkDictSmem& S) {
 	using T             = typename UT<W>::T;
-	const uint32_t tid  = threadIdx.x, nt = blockDim.x, lane = tid & 31u, warp = tid >> 5, nw = nt >> 5;
-	const uint32_t i0   = a.chunk_items[c], i1 = a.chunk_items[c + 1];
+	const uint32_t tid  = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
+	const uint32_t i0   = a.chunk_items[c], nv = a.chunk_items[c + 1] - i0;
 	const Item     m0   = a.items[i0];
-	const uint32_t v0   = m0.vec - m0.cpos; // the chunk's first vector
-	constexpr uint32_t mask = kCdSlots - 1;
-	uint64_t* bkeys = reinterpret_cast<uint64_t*>(a.gtab + blockIdx.x * kCdGBytes);
-	uint32_t* bpos  = reinterpret_cast<uint32_t*>(bkeys + static_cast<uint64_t>(kCdParts) * kCdBucket);
-	auto begin_insert = [&]() {
-		if (tid == 0) {
-			*s_count = 0;
-			*s_over  = 0;
+	const uint64_t row0 = static_cast<uint64_t>(m0.vec - m0.cpos) * 1024; // the chunk's first value
+	const T*       vals = reinterpret_cast<const T*>(col.values) + row0;
+	uint16_t*      slots = a.gslots + blockIdx.x * (kCdGBytes / 2);
+	if (warp == 0) { cd_choose(a, i0, nv, lane, S); }
+	__syncthreads();
+	const uint32_t mode = S.mode;
+	if (mode == CD_SORTED) {
+		if (tid < nv) { a.bw_code[i0 + tid] = bits_of(a.info[i0 + tid].runs - 1); }
+		if (tid == 0) { a.dict_n[c] = S.distinct; }
+		__syncthreads(); // S is read to the end before the next chunk's choice
+		return;
+	}
+	const T            flip = col.sgn ? (T(1) << (W - 1)) : T(0);
+	const T            low  = static_cast<T>(S.lo);
+	const uint32_t*    w0   = a.w0 ? a.w0[m0.col] + row0 : nullptr;
+	const uint32_t*    w1   = a.w0 ? a.w1[m0.col] + row0 : nullptr;
+	volatile uint32_t* over = &S.over;
+	uint64_t           sw0 = 0, sw1 = 0; // weights of the first positions this thread finds
+	CdQueue<T>         Q {reinterpret_cast<T*>(S.qkey[warp]), S.qpos[warp], S.qslot[warp], S.qtag[warp], nullptr, 0, 0};
+	constexpr uint32_t kPer = kMaxVecPerChunk / kCdWarps; // vectors of a warp: warp, warp + kCdWarps
+	uint32_t           listed[kPer];
+	auto clear = [&](uint32_t words) { // of the table
+		for (uint32_t k = tid; k < words / 4; k += kCdThreads) {
+			reinterpret_cast<uint4*>(S.table)[k] = make_uint4(kCdFree, kCdFree, kCdFree, kCdFree);
 		}
-		__syncthreads();
 	};
-	// limit: probes before an insert gives up (the first attempt gives up early: its table must never fill,
-	// or every insert into it walks all slots)
-	auto insert_one = [&](uint64_t key, uint32_t pos, uint32_t limit) {
-		const uint32_t sl = cd_insert(keys, mask, key, s_count, limit);
-		if (sl > mask + 1) {
-			*s_over = 1;
-		} else if (pos < first[sl]) {
-			atomicMin(first + sl, pos);
+	auto reset = [&]() { // before anything is found
+		for (uint32_t k = tid; k < kCdWords; k += kCdThreads) { S.bits[k] = 0; }
+		if (tid < kMaxVecPerChunk) {
+			S.vrange[tid][0] = ~0u;
+			S.vrange[tid][1] = 0u;
 		}
+		sw0 = sw1 = 0;
 	};
-	auto clear_table = [&]() {
-		for (uint32_t k = tid; k < kCdSlots; k += nt) { keys[k] = kEmpty; }
-		for (uint32_t k = tid; k <= kCdSlots; k += nt) { first[k] = kNoPos; }
-		__syncthreads();
+	// row r of vector v: this lane's value, and whether it starts a run (a vector's first value counts as one)
+	T    last = 0;
+	auto row  = [&](uint32_t v, uint32_t r, T* x) {
+		*x     = __ldg(vals + v * 1024 + r * 32 + lane);
+		T prev = __shfl_up_sync(0xFFFFFFFFu, *x, 1);
+		if (lane == 0) { prev = last; }
+		last = __shfl_sync(0xFFFFFFFFu, *x, 31);
+		return *x != prev || (r == 0 && lane == 0);
 	};
-	// every key's first position into the bitmap (and, for strings, its row's weights); the table emptied
-	auto harvest = [&]() {
-		uint64_t sw0 = 0, sw1 = 0;
-		for (uint32_t k = tid; k <= mask + 1; k += nt) {
-			const uint32_t f = first[k];
-			if (f != kNoPos) {
-				atomicOr(bits + (f >> 5), 1u << (f & 31u));
-				if (a.w0) {
-					const uint64_t row = static_cast<uint64_t>(v0) * 1024 + f;
-					sw0 += a.w0[m0.col][row];
-					sw1 += a.w1[m0.col][row];
+	// the ranges of the warp's vectors from their slots (the table holds the first positions), and the first positions
+	// themselves; the table is read to the end at the closing barrier
+	auto collect = [&](uint32_t n_slots) {
+#pragma unroll
+		for (uint32_t j = 0; j < kPer; ++j) {
+			const uint32_t  v    = warp + j * kCdWarps;
+			const uint16_t* list = slots + v * 1024;
+			uint32_t        lo = ~0u, hi = 0u;
+#pragma unroll 4
+			for (uint32_t i = lane; i < listed[j]; i += 32) {
+				const uint32_t f = S.table[list[i]] & 0xFFFFu;
+				lo               = min(lo, f);
+				hi               = max(hi, f);
+			}
+			lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+			hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+			if (lane == 0 && lo != ~0u) { // (the parts' turns are one after the other)
+				S.vrange[v][0] = min(S.vrange[v][0], lo);
+				S.vrange[v][1] = max(S.vrange[v][1], hi);
+			}
+		}
+#pragma unroll 4
+		for (uint32_t k = tid; k < n_slots; k += kCdThreads) {
+			const uint32_t e = S.table[k];
+			if (e != kCdFree) {
+				const uint32_t f = e & 0xFFFFu;
+				atomicOr(S.bits + (f >> 5), 1u << (f & 31u));
+				if (w0) {
+					sw0 += __ldg(w0 + f);
+					sw1 += __ldg(w1 + f);
 				}
 			}
 		}
-		if (a.w0) {
-			sw0 = warp_sum(sw0);
-			sw1 = warp_sum(sw1);
-			if (lane == 0) {
-				atomicAdd(reinterpret_cast<unsigned long long*>(s_dw), static_cast<unsigned long long>(sw0));
-				atomicAdd(reinterpret_cast<unsigned long long*>(s_dw + 1), static_cast<unsigned long long>(sw1));
-			}
-		}
 		__syncthreads();
 	};
-	auto code_of = [&](uint32_t f) { return pref[f >> 5] + __popc(bits[f >> 5] & ((1u << (f & 31u)) - 1u)); };
-	for (uint32_t k = tid; k < kCdWords; k += nt) { bits[k] = 0; }
-	for (uint32_t k = tid; k < 2 * kMaxVecPerChunk; k += nt) { vrange[k] = (k & 1u) ? 0u : ~0u; }
-	if (tid == 0) { s_dw[0] = s_dw[1] = 0; }
-	// first attempt: every key of the chunk in the shared-memory table.  A thread stops within 4 inserts of
-	// the count passing kCdCap (the table then holds at most kCdCap + 4 * 512 keys, 7/8 of its slots).
-	begin_insert();
-	volatile uint32_t* v_count = s_count;
-	volatile uint32_t* v_over  = s_over;
-	for (uint32_t j = i0 + warp; j < i1; j += nw) {
-		if (*v_over != 0 || *v_count > kCdCap) { break; } // too many: the buckets instead
-		const Item m = a.items[j];
-		T          x[32];
-		load_run<W>(col, m.vec, lane, x);
-		const uint32_t pos0 = m.cpos * 1024 + thread_run(lane);
-#pragma unroll
-		for (int i = 0; i < 32; ++i) {
-			if ((i & 3) == 0 && (*v_over != 0 || *v_count > kCdCap)) { break; }
-			insert_one(static_cast<uint64_t>(x[i]), pos0 + i, 256);
-		}
-	}
-	__syncthreads();
-	const bool small = *s_over == 0 && *s_count <= kCdCap;
-	__syncthreads();
-	uint32_t bcount[kCdParts];
-	if (small) {
-		harvest();
-	} else {
-		clear_table();
-		// one read of the values: (key, position) pairs into kCdParts buckets by hash
-		if (tid < kCdParts) { s_wsum[tid] = 0; }
+	if (tid < 2) { S.dw[tid] = 0; }
+	bool found = false;
+	if (mode == CD_DIRECT) {
+		reset();
+		clear(kCdSlots);
 		__syncthreads();
-		for (uint32_t j = i0 + warp; j < i1; j += nw) {
-			const Item m = a.items[j];
-			T          x[32];
-			load_run<W>(col, m.vec, lane, x);
-			const uint32_t pos0 = m.cpos * 1024 + thread_run(lane);
-#pragma unroll
-			for (int i = 0; i < 32; ++i) {
-				const uint64_t key  = static_cast<uint64_t>(x[i]);
-				const uint32_t b    = static_cast<uint32_t>(cd_mix(key) >> 61);
-				const uint32_t peer = __match_any_sync(0xFFFFFFFFu, b);
-				const uint32_t lead = __ffs(peer) - 1;
-				uint32_t       base = 0;
-				if (lane == lead) { base = atomicAdd(s_wsum + b, static_cast<uint32_t>(__popc(peer))); }
-				base                 = __shfl_sync(peer, base, lead);
-				const uint32_t slot  = base + __popc(peer & ((1u << lane) - 1u));
-				const uint64_t where = static_cast<uint64_t>(b) * kCdBucket + slot;
-				bkeys[where]         = key;
-				bpos[where]          = pos0 + i;
+		auto entry = [&](T x) { return S.table + static_cast<uint32_t>(static_cast<T>((x ^ flip) - low)); };
+		for (uint32_t v = warp; v < nv; v += kCdWarps) {
+#pragma unroll 8
+			for (uint32_t r = 0; r < 32; ++r) {
+				const uint32_t pos = v * 1024 + r * 32 + lane;
+				uint32_t*      e   = entry(__ldg(vals + pos));
+				if (pos < *reinterpret_cast<volatile uint32_t*>(e)) { atomicMin(e, pos); }
 			}
 		}
 		__syncthreads();
+		for (uint32_t v = warp; v < nv; v += kCdWarps) {
+			uint32_t lo = ~0u, hi = 0u;
+#pragma unroll 8
+			for (uint32_t r = 0; r < 32; ++r) {
+				const uint32_t f = *entry(__ldg(vals + v * 1024 + r * 32 + lane));
+				lo               = min(lo, f);
+				hi               = max(hi, f);
+			}
+			lo = __reduce_min_sync(0xFFFFFFFFu, lo);
+			hi = __reduce_max_sync(0xFFFFFFFFu, hi);
+			if (lane == 0) {
+				S.vrange[v][0] = lo;
+				S.vrange[v][1] = hi;
+			}
+		}
 #pragma unroll
-		for (uint32_t b = 0; b < kCdParts; ++b) { bcount[b] = s_wsum[b]; }
+		for (uint32_t j = 0; j < kPer; ++j) { listed[j] = 0; }
+		collect(kCdSlots);
+		found = true;
+	}
+	if (mode == CD_UNIQUE) {
+		uint32_t* filter = S.table;
+		uint32_t* marks  = S.table + kCdUniqueSlots;
+		reset();
+		for (uint32_t k = tid; k < kCdUniqueSlots + kCdMarkWords; k += kCdThreads) { S.table[k] = 0; }
+		if (tid == 0) { S.count = S.over = 0; }
 		__syncthreads();
-		// every bucket through the table; once a bucket's table is complete, every pair's key is replaced by its
-		// key's first position (high half) beside its own position, so the code pass needs no table
-		for (uint32_t b = 0; b < kCdParts; ++b) {
-			begin_insert();
-			for (uint32_t k = tid; k < bcount[b]; k += nt) {
-				const uint64_t where = static_cast<uint64_t>(b) * kCdBucket + k;
-				insert_one(bkeys[where], bpos[where], kCdSlots);
+		bool stop = false;
+		for (uint32_t v = warp; v < nv && !stop; v += kCdWarps) {
+			for (uint32_t r0 = 0; r0 < 32 && !stop; r0 += 4) {
+				uint32_t set = 0;
+#pragma unroll
+				for (uint32_t i = 0; i < 4; ++i) {
+					T          x;
+					const bool start = row(v, r0 + i, &x);
+					uint32_t   place, tag;
+					cd_hash(x, &place, &tag);
+					const uint32_t b = place >> 12;
+					if (start && ((atomicOr(filter + (b >> 5), 1u << (b & 31u)) >> (b & 31u)) & 1u)) {
+						atomicOr(marks + (b >> 7), 1u << ((b >> 2) & 31u));
+						++set;
+					}
+				}
+				set = __reduce_add_sync(0xFFFFFFFFu, set);
+				if (lane == 0) {
+					// too many already, or on the way there
+					const uint32_t now = atomicAdd(&S.count, (4u << 16) + set) + (4u << 16) + set;
+					const uint32_t n = now & 0xFFFFu, done = now >> 16;
+					if (n > kCdUniqueMax || (done >= 4 * nv && n * nv > done * (kCdUniqueMax / 32) * 2)) { *over = 1; }
+				}
+				stop = __any_sync(0xFFFFFFFFu, *over != 0);
+			}
+		}
+		__syncthreads();
+		found = S.over == 0;
+		__syncthreads(); // S.over is read before it is cleared
+		if (found) {
+			clear(kCdUniqueSlots);
+			if (tid == 0) { S.count = 0; }
+			__syncthreads();
+#pragma unroll
+			for (uint32_t j = 0; j < kPer; ++j) {
+				const uint32_t v = warp + j * kCdWarps;
+				uint32_t       lo = ~0u, hi = 0u, steps = 0;
+				Q.list = slots + v * 1024;
+				Q.q = Q.n = 0;
+				for (uint32_t r = 0; r < 32 && v < nv; ++r) {
+					if (__any_sync(0xFFFFFFFFu, *over != 0)) { break; } // one answer for the whole warp
+					T          x;
+					const bool start = row(v, r, &x);
+					uint32_t   place, tag;
+					cd_hash(x, &place, &tag);
+					const uint32_t pos  = v * 1024 + r * 32 + lane;
+					const bool     mark = start && ((marks[place >> 19] >> ((place >> 14) & 31u)) & 1u);
+					const uint32_t only = __ballot_sync(0xFFFFFFFFu, start && !mark);
+					if (lane == 0) { S.bits[pos >> 5] = only; }
+					if (only) {
+						lo = min(lo, pos - lane + __ffs(only) - 1);
+						hi = pos - lane + 31 - __clz(only);
+					}
+					if (w0 && start && !mark) {
+						sw0 += __ldg(w0 + pos);
+						sw1 += __ldg(w1 + pos);
+					}
+					Q.push(mark, x, pos, __umulhi(place, kCdUniqueSlots), tag, lane);
+					uint32_t fresh = 0;
+					while ((Q.q >= 32 || (r == 31 && Q.q > 0)) && ++steps < kCdMaxSteps) { fresh += Q.pop(S.table, kCdUniqueSlots, vals, lane); }
+					if (lane == 0 && fresh && atomicAdd(&S.count, fresh) + fresh > kCdUniqueCap) { *over = 1; }
+				}
+				listed[j] = Q.n;
+				if (lane == 0 && lo != ~0u) {
+					S.vrange[v][0] = lo;
+					S.vrange[v][1] = hi;
+				}
+				if (steps >= kCdMaxSteps && lane == 0) { atomicOr(a.status, STATUS_BAD_INDEX); }
 			}
 			__syncthreads();
-			if ((*s_over != 0 || *s_count > mask) && tid == 0) { atomicOr(a.status, STATUS_BAD_INDEX); } // never
-			for (uint32_t k = tid; k < bcount[b]; k += nt) {
-				const uint64_t where = static_cast<uint64_t>(b) * kCdBucket + k;
-				const uint32_t sl    = cd_find(keys, mask, bkeys[where]);
-				const uint32_t f     = sl > mask + 1 ? kNoPos : first[sl];
-				bkeys[where]         = (static_cast<uint64_t>(f) << 32) | bpos[where];
-			}
-			harvest(); // reads the table only; its closing barrier orders the clear after every find
-			clear_table();
+			found = S.over == 0;
+			__syncthreads(); // S.over is read before it is cleared
+			if (found) { collect(kCdUniqueSlots); }
 		}
 	}
-	// ranks: exclusive prefix of the bitmap words' popcounts (thread t: words [t * per, (t + 1) * per))
-	const uint32_t per = kCdWords / nt;
-	uint32_t       loc = 0;
-	for (uint32_t k = 0; k < per; ++k) { loc += __popc(bits[tid * per + k]); }
-	const uint32_t inc = warp_inclusive_scan(loc, lane);
-	if (lane == 31) { s_wsum[warp] = inc; }
+	for (uint32_t parts_log = 0; !found; ++parts_log) {
+		reset();
+		for (uint32_t part = 0; part < (1u << parts_log); ++part) {
+			clear(kCdSlots);
+			if (tid == 0) { S.count = S.over = 0; }
+			__syncthreads();
+			uint32_t steps = 0;
+#pragma unroll
+			for (uint32_t j = 0; j < kPer; ++j) {
+				const uint32_t v    = warp + j * kCdWarps;
+				uint32_t       rows = 0;
+				Q.list = slots + v * 1024;
+				Q.q = Q.n = 0;
+				for (uint32_t r = 0; r < 32 && v < nv; ++r) {
+					if (__any_sync(0xFFFFFFFFu, *over != 0)) { break; } // one answer for the whole warp
+					T        x;
+					bool     need = row(v, r, &x);
+					uint32_t place, tag;
+					cd_hash(x, &place, &tag);
+					if (parts_log) { need = need && (place >> (32 - parts_log)) == part; }
+					const uint32_t pos = v * 1024 + r * 32 + lane, s = __umulhi(place << parts_log, kCdSlots);
+					uint32_t       fresh = 0;
+					bool           looked = true;
+					if (Q.q == 0 && __all_sync(0xFFFFFFFFu, need)) { // a full warp as it is
+						fresh = Q.look(S.table, kCdSlots, vals, true, x, pos, s, tag, lane);
+						++steps;
+					} else {
+						Q.push(need, x, pos, s, tag, lane);
+						looked = Q.q >= 32;
+					}
+					while ((Q.q >= 32 || (r == 31 && Q.q > 0)) && ++steps < kCdMaxSteps) { fresh += Q.pop(S.table, kCdSlots, vals, lane); }
+					++rows;
+					if (lane == 0 && (looked || r == 31)) {
+						// room left, and room for the chunk if the keys go on coming at this rate?
+						const uint32_t now = atomicAdd(&S.count, (rows << 16) + fresh) + (rows << 16) + fresh;
+						const uint32_t n = now & 0xFFFFu, done = now >> 16;
+						if (n > kCdCap || (done >= 4 * nv && n * nv > done * (kCdCap / 32))) { *over = 1; }
+					}
+					if (looked) { rows = 0; }
+				}
+				listed[j] = Q.n;
+			}
+			if (steps >= kCdMaxSteps && lane == 0) { atomicOr(a.status, STATUS_BAD_INDEX); }
+			__syncthreads();
+			const bool full = S.over != 0;
+			__syncthreads(); // S.over is read before it is cleared
+			if (full) { break; }
+			collect(kCdSlots);
+			found = part + 1 == (1u << parts_log);
+		}
+		if (!found && (2u << parts_log) > kCdMaxParts) {
+			if (tid == 0) { atomicOr(a.status, STATUS_BAD_INDEX); } // never: 256 parts of 65,536 values
+			break;
+		}
+	}
+	if (w0) {
+		sw0 = warp_sum(sw0);
+		sw1 = warp_sum(sw1);
+		if (lane == 0) {
+			atomicAdd(reinterpret_cast<unsigned long long*>(S.dw), static_cast<unsigned long long>(sw0));
+			atomicAdd(reinterpret_cast<unsigned long long*>(S.dw + 1), static_cast<unsigned long long>(sw1));
+		}
+	}
+	// exclusive prefix of the bitmap words' popcounts: words 2 * tid, 2 * tid + 1
+	static_assert(kCdWords == 2 * kCdThreads, "two bitmap words a thread");
+	uint32_t*      pref = S.table;
+	const uint32_t p0 = __popc(S.bits[2 * tid]), p1 = __popc(S.bits[2 * tid + 1]);
+	const uint32_t inc = warp_inclusive_scan(p0 + p1, lane);
+	if (lane == 31) { S.wsum[warp] = inc; }
 	__syncthreads();
 	if (warp == 0) {
-		const uint32_t w  = lane < nw ? s_wsum[lane] : 0u;
+		const uint32_t w  = S.wsum[lane];
 		const uint32_t wi = warp_inclusive_scan(w, lane);
-		s_wsum[lane]      = wi - w;
-		if (lane == 31) { s_wsum[32] = wi; }
+		S.wsum[lane]      = wi - w;
+		if (lane == 31) { S.wsum[32] = wi; }
 	}
 	__syncthreads();
-	uint32_t run = s_wsum[warp] + inc - loc;
-	for (uint32_t k = 0; k < per; ++k) {
-		pref[tid * per + k] = run;
-		run += __popc(bits[tid * per + k]);
-	}
-	const uint32_t total = s_wsum[32];
+	pref[2 * tid]     = S.wsum[warp] + inc - p0 - p1;
+	pref[2 * tid + 1] = S.wsum[warp] + inc - p1;
 	__syncthreads();
-	// codes: the code range of every vector of the chunk
-	if (small) {
-#pragma unroll
-		for (uint32_t q = 0; q < 4; ++q) {
-			const uint32_t j  = i0 + warp + q * nw;
-			uint32_t       mn = ~0u, mx = 0u;
-			if (j < i1) {
-				const Item m = a.items[j];
-				T          x[32];
-				load_run<W>(col, m.vec, lane, x);
-#pragma unroll
-				for (int i = 0; i < 32; ++i) {
-					const uint32_t sl = cd_find(keys, mask, static_cast<uint64_t>(x[i]));
-					if (sl > mask + 1) { continue; }
-					const uint32_t code = code_of(first[sl]);
-					mn                  = min(mn, code);
-					mx                  = max(mx, code);
-				}
-			}
-			mn = warp_min(mn);
-			mx = warp_max(mx);
-			if (j < i1 && lane == 0) {
-				vrange[2 * (j - i0)]     = mn;
-				vrange[2 * (j - i0) + 1] = mx;
-			}
-		}
-		__syncthreads();
-		clear_table();
-	} else {
-		// codes from the recorded first positions; a warp whose pairs all belong to one vector (the usual case:
-		// a bucket keeps the scatter's order) folds them before one atomic pair
-		for (uint32_t b = 0; b < kCdParts; ++b) {
-			for (uint32_t kb = 0; kb < bcount[b]; kb += nt) {
-				const uint32_t k  = kb + tid;
-				uint32_t       vi = ~0u, code = 0;
-				if (k < bcount[b]) {
-					const uint64_t e = bkeys[static_cast<uint64_t>(b) * kCdBucket + k];
-					const uint32_t f = static_cast<uint32_t>(e >> 32);
-					if (f != kNoPos) {
-						vi   = static_cast<uint32_t>(e) >> 10; // the vector inside the chunk
-						code = code_of(f);
-					}
-				}
-				const uint32_t v0 = __shfl_sync(0xFFFFFFFFu, vi, 0);
-				if (__all_sync(0xFFFFFFFFu, vi == v0)) {
-					const uint32_t mn = warp_min(code), mx = warp_max(code);
-					if (lane == 0 && v0 != ~0u) {
-						atomicMin(vrange + 2 * v0, mn);
-						atomicMax(vrange + 2 * v0 + 1, mx);
-					}
-				} else if (vi != ~0u) {
-					atomicMin(vrange + 2 * vi, code);
-					atomicMax(vrange + 2 * vi + 1, code);
-				}
-			}
-		}
-		__syncthreads();
-	}
-	for (uint32_t j = i0 + tid; j < i1; j += nt) {
-		const uint32_t lo = vrange[2 * (j - i0)], hi = vrange[2 * (j - i0) + 1];
-		a.bw_code[j]      = hi >= lo ? bits_of(hi - lo) : 0u;
+	if (tid < nv) {
+		auto rank = [&](uint32_t f) { return pref[f >> 5] + __popc(S.bits[f >> 5] & ((1u << (f & 31u)) - 1u)); };
+		const uint32_t lo = S.vrange[tid][0], hi = S.vrange[tid][1];
+		a.bw_code[i0 + tid] = lo <= hi ? bits_of(rank(hi) - rank(lo)) : 0u;
 	}
 	if (tid == 0) {
-		a.dict_n[c] = total;
+		a.dict_n[c] = S.wsum[32];
 		if (a.dict_w) {
-			a.dict_w[2ull * c]     = s_dw[0];
-			a.dict_w[2ull * c + 1] = s_dw[1];
+			a.dict_w[2ull * c]     = S.dw[0];
+			a.dict_w[2ull * c + 1] = S.dw[1];
 		}
 	}
 	__syncthreads();
 }
 
-__global__ void __launch_bounds__(kCdWarps * 32) k_chunk_dict(ChunkDictArgs a) {
+__global__ void __launch_bounds__(kCdThreads) k_chunk_dict(ChunkDictArgs a) {
 	extern __shared__ __align__(16) uint8_t smem[];
-	__shared__ uint32_t s_count, s_over, s_wsum[33];
-	__shared__ uint64_t s_dw[2];
-	uint64_t*           keys   = reinterpret_cast<uint64_t*>(smem);
-	uint32_t*           first  = reinterpret_cast<uint32_t*>(keys + kCdSlots);
-	uint32_t*           bits   = first + kCdSlots + 1;
-	uint32_t*           pref   = bits + kCdWords;
-	uint32_t*           vrange = pref + kCdWords;
-	for (uint32_t k = threadIdx.x; k < kCdSlots; k += blockDim.x) { keys[k] = kEmpty; }
-	for (uint32_t k = threadIdx.x; k <= kCdSlots; k += blockDim.x) { first[k] = kNoPos; }
-	__syncthreads();
-	for (uint32_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
+	ChunkDictSmem&                          S = *reinterpret_cast<ChunkDictSmem*>(smem);
+	for (;;) {
+		// chunks differ in cost by their distinct values: the next free CTA takes the next one
+		if (threadIdx.x == 0) { S.chunk = atomicAdd(a.ticket, 1u); }
+		__syncthreads();
+		const uint32_t c = S.chunk;
+		if (c >= a.n_chunks) { return; }
 		const Col col = a.cols[a.items[a.chunk_items[c]].col];
 		if (col.width == 64) {
-			chunk_dict<64>(a, col, c, keys, first, bits, pref, vrange, &s_count, &s_over, s_wsum, s_dw);
+			chunk_dict<64>(a, col, c, S);
 		} else {
-			chunk_dict<32>(a, col, c, keys, first, bits, pref, vrange, &s_count, &s_over, s_wsum, s_dw);
+			chunk_dict<32>(a, col, c, S);
 		}
 	}
 }
@@ -1361,9 +1559,9 @@ struct fls_sel_plan {
 	std::vector<uint64_t> chunk_first;
 	uint64_t              n_chunks = 0;
 	uint32_t              chunk_vectors = 64;
-	// wizard scratch (gtab: the chunk dictionary's bucket scratch, one region per CTA; the subset lists of a
+	// wizard scratch (gtab: the chunk dictionary's slot scratch, one region per CTA; the subset lists of a
 	// wizard run over some chunks) and the learned selector's; all grow-only
-	Scratch bw_code, parts, dict_n, gtab, sub_items, sub_ranges, sub_ccol, sub_ids, sub_sizes, sub_best, vlen, vclen,
+	Scratch bw_code, parts, info, dict_n, gtab, sub_items, sub_ranges, sub_ccol, sub_ids, sub_sizes, sub_best, vlen, vclen,
 	    dict_w, l_work, l_conf;
 	// string columns (fls_sel_plan_create_strings): the plan's columns are the row hashes; these are the strings
 	bool                str = false;
@@ -1455,7 +1653,7 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 		ccol_d   = p->sub_ccol.as<uint32_t>();
 	}
 	if (n_items == 0) { return FLS_OK; }
-	if (!p->parts.need(n_items * 4) || !p->bw_code.need(n_items * 4) || !p->dict_n.need(chunks.size() * 4)) {
+	if (!p->parts.need(n_items * 4) || !p->bw_code.need(n_items * 4) || !p->info.need(n_items * sizeof(VecInfo)) || !p->dict_n.need(chunks.size() * 4)) {
 		return FLS_ERR_CUDA;
 	}
 	if (p->str) {
@@ -1468,31 +1666,33 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 		++launch_counter();
 	}
 	ItemArgs ia {p->cols_d.as<Col>(), items_d, n_items};
-	k_parts<<<grid_for(n_items), kWarps * 32, 0, s>>>(ia, p->parts.as<uint32_t>());
+	k_parts<<<grid_for(n_items), kWarps * 32, 0, s>>>(ia, p->parts.as<uint32_t>(), p->info.as<VecInfo>());
 	++launch_counter();
 	// dictionary of every chunk: one CTA per chunk, tables in shared memory
 	{
 		static bool attr[64] = {};
 		if (dev->ordinal < 0 || dev->ordinal >= 64) { return FLS_ERR_CUDA; }
 		if (!attr[dev->ordinal]) {
-			if (cudaFuncSetAttribute(k_chunk_dict, cudaFuncAttributeMaxDynamicSharedMemorySize, kCdSmem) != cudaSuccess) {
+			if (cudaFuncSetAttribute(k_chunk_dict, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ChunkDictSmem)) != cudaSuccess) {
 				return FLS_ERR_CUDA;
 			}
 			attr[dev->ordinal] = true;
 		}
-		// one CTA per SM, each with its own bucket scratch for chunks of many distinct values
+		// one CTA per SM, each with its own slot scratch
 		const uint32_t grid = static_cast<uint32_t>(std::min<size_t>(chunks.size(), static_cast<size_t>(dev->sm_count)));
-		if (!p->gtab.need(kCdGBytes * grid)) { return FLS_ERR_CUDA; }
-		ChunkDictArgs a {p->cols_d.as<Col>(), items_d, ranges_d,
+		if (!p->gtab.need(kCdGBytes * grid + 4)) { return FLS_ERR_CUDA; }
+		uint32_t* ticket = reinterpret_cast<uint32_t*>(p->gtab.as<uint8_t>() + kCdGBytes * grid);
+		if (cudaMemsetAsync(ticket, 0, 4, s) != cudaSuccess) { return FLS_ERR_CUDA; }
+		ChunkDictArgs a {p->cols_d.as<Col>(), items_d, p->info.as<VecInfo>(), ranges_d,
 		                 static_cast<uint32_t>(chunks.size()), p->dict_n.as<uint32_t>(), p->bw_code.as<uint32_t>(),
-		                 dev->status, nullptr, nullptr, nullptr, p->gtab.as<uint8_t>()};
+		                 dev->status, nullptr, nullptr, nullptr, p->gtab.as<uint16_t>(), ticket};
 		if (p->str) {
 			const uint32_t* const* wp = p->wptr_d.as<const uint32_t*>();
 			a.w0                      = wp;
 			a.w1                      = wp + p->scols.size();
 			a.dict_w                  = p->dict_w.as<uint64_t>();
 		}
-		k_chunk_dict<<<grid, kCdWarps * 32, kCdSmem, s>>>(a);
+		k_chunk_dict<<<grid, kCdThreads, sizeof(ChunkDictSmem), s>>>(a);
 		++launch_counter();
 		if (cudaGetLastError() != cudaSuccess) { return FLS_ERR_CUDA; }
 	}
@@ -1700,7 +1900,7 @@ int fls_sel_vector_parts(const fls_sel_plan* p, uint32_t* d_parts, void* stream)
 	if (p->items.empty()) { return FLS_OK; }
 	cudaStream_t s = static_cast<cudaStream_t>(stream);
 	ItemArgs     a {p->cols_d.as<Col>(), p->items_d.as<Item>(), p->items.size()};
-	k_parts<<<grid_for(p->items.size()), kWarps * 32, 0, s>>>(a, d_parts);
+	k_parts<<<grid_for(p->items.size()), kWarps * 32, 0, s>>>(a, d_parts, nullptr);
 	++launch_counter();
 	return cudaGetLastError() == cudaSuccess ? FLS_OK : FLS_ERR_CUDA;
 }

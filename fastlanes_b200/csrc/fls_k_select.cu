@@ -952,11 +952,24 @@ __global__ void __launch_bounds__(kCdThreads) k_chunk_dict(ChunkDictArgs a) {
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kStrK = FLS_SEL_STR_K;
 
-// An FSST symbol table arranged for greedy matching: symbols grouped by their first byte, longest first.
+// An FSST symbol table arranged for greedy matching by the next two bytes of a string:
+//   one    bitmap of the bytes that are symbols by themselves; two: the two-byte symbols;
+//   groups the longer symbols, grouped by their first two bytes (pair), longest first.  Group ids start at kStrGroup;
+//          g_short is what a string takes when none of the group's symbols matches: 2, 1 or 0 (an escape).  A table
+//          with more pairs than ids shares the id of another group with the same g_short: every symbol of a group
+//          is compared in full, so that only costs comparisons.
+constexpr uint32_t kStrGroup  = 3;
+constexpr uint32_t kStrGroups = 256 - kStrGroup;
 struct StrTab {
-	uint64_t val[256];
+	ulonglong2 sym[256]; // the groups' symbols: value, mask of its bytes
+	uint32_t one[8];
+	uint16_t two[256];
+	uint16_t pair[256];  // first two bytes (the first in the low byte)
+	uint16_t start[258]; // symbols of group g: [start[g], start[g + 1]), g counted from 0
+	uint16_t n_two, n_pair;
+	uint8_t  pair_group[256];
 	uint8_t  len[256];
-	uint16_t start[257]; // symbols starting with byte b: [start[b], start[b + 1])
+	uint8_t  g_short[256];
 };
 
 struct StrCol {
@@ -992,97 +1005,290 @@ __device__ __forceinline__ uint64_t str_load8(const StrCol& c, uint64_t p) {
 	return (static_cast<uint64_t>(hi) << 32) | lo;
 }
 
-// Block per item: hash and length of each of the vector's 1024 rows, and the compressed length of every rs-th
-// row (rs = 1: every row, the exact figure the wizard's sizes need; rs > 1, the learned selector's features:
-// the other rows' compressed lengths are written as 0 and the vector's sum is scaled by rs).  The column's
-// symbol table is copied to shared memory for the greedy match; the vector's sums (vlen, vclen) by a block
-// reduction.
-__global__ void __launch_bounds__(kWarps * 32) k_str_rows(const StrCol* cols, const Item* items, uint64_t n_items,
-                                                          uint64_t* vlen, uint64_t* vclen, uint32_t rs) {
-	__shared__ uint64_t t_val[256];
-	__shared__ uint8_t  t_len[256];
-	__shared__ uint16_t t_start[257];
-	__shared__ uint64_t red[2][kWarps];
-	constexpr uint32_t  nt   = kWarps * 32;
-	const uint32_t      tid  = threadIdx.x, lane = tid & 31u, warp = tid >> 5;
-	for (uint64_t it = blockIdx.x; it < n_items; it += gridDim.x) {
-		const Item   m = items[it];
-		const StrCol c = cols[m.col];
-		__syncthreads(); // the previous item's table reads and sums are done
-		for (uint32_t k = tid; k < 257; k += nt) {
-			if (k < 256) {
-				t_val[k] = c.tab->val[k];
-				t_len[k] = c.tab->len[k];
+// str_load8 for a row that ends at least 12 bytes before the column's last byte
+__device__ __forceinline__ uint64_t str_load8_inside(const StrCol& c, uint64_t p) {
+	const uintptr_t a  = reinterpret_cast<uintptr_t>(c.bytes) + p;
+	const uint32_t* w  = reinterpret_cast<const uint32_t*>(a & ~uintptr_t(3));
+	const uint32_t  x0 = __ldg(w), x1 = __ldg(w + 1), x2 = __ldg(w + 2);
+	const uint32_t  sh = 8u * static_cast<uint32_t>(a & 3u);
+	return (static_cast<uint64_t>(__funnelshift_r(x1, x2, sh)) << 32) | __funnelshift_r(x0, x1, sh);
+}
+
+// Hash and length of each of a vector's 1024 rows, and the compressed length of every rs-th row (rs = 1: every
+// row, the exact figure the wizard's sizes need; rs > 1, the learned selector's features: the other rows'
+// compressed lengths are written as 0 and the vector's sum is scaled by rs).  The CTAs go through the columns one
+// after the other, a warp taking units of kStrUnit rows.
+//   memo     rows whose hash another row of the column had before (dictionary-like columns: nearly all) take its
+//            compressed length from a table in global memory, 64-bit entries of the hash and the length, cleared for
+//            every call; rows are told apart by hash and length.  A first launch over
+//            every `stride`-th vector fills it: all units start at once, so that without it nothing would be found;
+//   match    greedy matching looks at the next two bytes in a 64 KB table in shared memory (what they start: nothing,
+//            a one- or two-byte symbol, or a group of longer ones), so that only the few symbols of one group are
+//            compared, where the symbols sharing a first byte were walked one after the other;
+//   lanes    draw rows from the warp's list as they finish (8 at a time), one code a step: rows of 1 to 20 codes
+//            would otherwise leave most lanes idle.
+// 5.7 M rows (a third of them all different, 17 codes each): 1,677 us by rows and first-byte lists, 128 + 481 us for the
+// two launches, of which the matching is 410 and the hashes 66; instruction-bound.
+constexpr int      kStrWarps = 16;
+constexpr uint32_t kStrUnit  = 128;          // rows a warp takes at a time
+constexpr uint32_t kStrMemo  = 1u << 17;     // entries (1 MB, in L2)
+constexpr uint32_t kStrMemoLen = 4094;       // longest compressed length an entry holds
+struct StrRowsSmem {
+	uint8_t  pair[65536]; // by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g
+	StrTab   t;
+	uint32_t off[kStrWarps][kStrUnit + 1]; // a unit's row offsets from its first row's
+	uint16_t list[kStrWarps][kStrUnit];    // rows to match
+};
+
+// Codes and their cost (1, or 2 for an escaped byte) of the string bytes in x, `left` of them still in the row: the
+// length of the next code's bytes; *cost grows by its compressed size.
+__device__ __forceinline__ uint32_t str_next_code(const StrRowsSmem& S, uint64_t x, uint64_t left, uint32_t* cost) {
+	uint32_t what = S.pair[x & 0xFFFFu], step = 0;
+	if (left == 1) { what = (S.t.one[(x & 0xFFu) >> 5] >> (x & 31u)) & 1u; }
+	if (what >= kStrGroup) {
+		const uint32_t g = what - kStrGroup;
+		for (uint32_t k = S.t.start[g]; k < S.t.start[g + 1]; ++k) {
+			const ulonglong2 m = S.t.sym[k];
+			if ((x & m.y) == m.x && S.t.len[k] <= left) {
+				step = S.t.len[k];
+				break;
 			}
-			t_start[k] = c.tab->start[k];
+		}
+		what = step ? 1u : S.t.g_short[g];
+	}
+	if (step == 0) { step = what == 2 ? 2u : 1u; }
+	*cost += what ? 1u : 2u;
+	return step;
+}
+
+__device__ __forceinline__ uint64_t str_hash_step(uint64_t h, uint64_t x, uint64_t left) {
+	const uint64_t k = left >= 8 ? x : (x & ((1ull << (8 * left)) - 1));
+	return str_mix(h ^ k) + 0x9E3779B97F4A7C15ull;
+}
+constexpr uint64_t kStrHashSeed = 0x243F6A8885A308D3ull;
+
+// A unit whose offsets do not fit 31 bits from its first one (rows of gigabytes, or corrupt offsets), row by row.
+__device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c, uint64_t r0, uint32_t rs, uint32_t lane,
+                                           uint64_t* sl, uint64_t* sc) {
+	for (uint32_t j = lane; j < kStrUnit; j += 32) {
+		const uint64_t r = r0 + j, b = __ldg(c.offsets + r), e = __ldg(c.offsets + r + 1), m = e >= b ? e - b : 0;
+		uint64_t       h = kStrHashSeed ^ m;
+		for (uint64_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_load8(c, b + p), m - p); }
+		uint32_t cl = 0;
+		if ((r & 1023u) % rs == 0) {
+			for (uint64_t p = 0; p < m;) { p += str_next_code(S, str_load8(c, b + p), m - p, &cl); }
+		}
+		c.hash[r] = h;
+		c.len[r]  = static_cast<uint32_t>(m);
+		c.clen[r] = cl;
+		*sl += m;
+		*sc += cl;
+	}
+}
+
+// A row's memo entry: its place, and the entry without the length (the low 12 bits hold length + 1); place and entry
+// together hold all 64 bits of the hash, mixed with the column (its lengths are by its own table) and the row's own
+// length (short rows of different lengths can share a hash: "a" and "b\0" do).
+__device__ __forceinline__ uint64_t str_memo_key(uint64_t h, uint32_t col, uint32_t m, uint32_t* at) {
+	h ^= (static_cast<uint64_t>(col) << 32 | m) * 0x9E3779B97F4A7C15ull;
+	*at = static_cast<uint32_t>(h) & (kStrMemo - 1);
+	return ((h >> 5) ^ (h << 47)) & ~0xFFFull; // bits 17-63 of the hash in bits 12-58
+}
+
+struct StrRowsArgs {
+	const StrCol* cols;
+	const Item*   items; // by column
+	uint64_t      n_items;
+	uint64_t *    vlen, *vclen; // optional: sums of every item, zero before the first launch
+	uint64_t*     memo;
+	uint32_t      rs;
+	uint32_t      stride; // every stride-th item in the launch that fills the memo, the others in the next one
+	uint32_t      fill;
+};
+
+__global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArgs a) {
+	extern __shared__ __align__(16) uint8_t smem[];
+	StrRowsSmem&       S  = *reinterpret_cast<StrRowsSmem*>(smem);
+	constexpr uint32_t nt = kStrWarps * 32, kPer = 1024 / kStrUnit; // units of a vector
+	const uint32_t     tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, rs = a.rs;
+	uint64_t* const    memo = a.memo;
+	// this launch's items: i * stride (fill), or the others in order; number i of them
+	const uint64_t n_fill = (a.n_items + a.stride - 1) / a.stride;
+	const uint64_t n      = a.fill ? n_fill : a.n_items - n_fill;
+	auto           item   = [&](uint64_t i) { return a.fill ? i * a.stride : a.stride == 1 ? i : i + i / (a.stride - 1) + 1; };
+	const uint64_t gw = static_cast<uint64_t>(blockIdx.x) * kStrWarps, nw = static_cast<uint64_t>(gridDim.x) * kStrWarps;
+	// units are dealt to the warps round robin, over the columns' borders
+	for (uint64_t first = 0; first < n;) {
+		const uint32_t col = a.items[item(first)].col;
+		uint64_t       lo = first + 1, hi = n; // the column's end among them: the first item of another column
+		while (lo < hi) {
+			const uint64_t mid = (lo + hi) / 2;
+			if (a.items[item(mid)].col == col) {
+				lo = mid + 1;
+			} else {
+				hi = mid;
+			}
+		}
+		const uint64_t u0 = first * kPer, u1 = lo * kPer;
+		first             = lo;
+		// the CTA's first unit of the column at or after u0: one of warp gw .. gw + kStrWarps - 1 (mod nw)
+		const uint64_t mine = u0 + (gw + kStrWarps - 1 + nw - u0 % nw) % nw; // of the CTA's last warp
+		if (mine >= u1 + kStrWarps - 1) { continue; }
+		const StrCol c = a.cols[col];
+		__syncthreads(); // the previous column's table is read to the end
+		for (uint32_t k = tid; k < sizeof(StrTab) / 4; k += nt) {
+			reinterpret_cast<uint32_t*>(&S.t)[k] = __ldg(reinterpret_cast<const uint32_t*>(c.tab) + k);
 		}
 		__syncthreads();
-		const uint64_t r0 = static_cast<uint64_t>(m.vec) * 1024;
-		uint64_t       sl = 0, sc = 0;
-		for (uint32_t j = tid; j < 1024; j += nt) {
-			const uint64_t r = r0 + j;
-			const uint64_t s = c.offsets[r], e = c.offsets[r + 1];
-			const uint64_t n = e >= s ? e - s : 0;
-			uint64_t       h = 0x243F6A8885A308D3ull ^ n;
-			for (uint64_t p = 0; p < n; p += 8) {
-				const uint64_t x = str_load8(c, s + p);
-				const uint64_t k = n - p >= 8 ? x : (x & ((1ull << (8 * (n - p))) - 1));
-				h                = str_mix(h ^ k) + 0x9E3779B97F4A7C15ull;
-			}
-			c.hash[r] = h;
-			c.len[r]  = static_cast<uint32_t>(n);
-			if (j % rs != 0) { c.clen[r] = 0; }
-			sl += n;
+		for (uint32_t k = tid; k < 65536 / 4; k += nt) { // bytes 4k .. 4k + 3: the low byte of the pair
+			const uint32_t m                       = S.t.one[(k & 63u) >> 3] >> (4 * (k & 7u));
+			reinterpret_cast<uint32_t*>(S.pair)[k] = (m & 1u) | ((m & 2u) << 7) | ((m & 4u) << 14) | ((m & 8u) << 21);
 		}
-		// compressed lengths: rows rs * (tid + nt * i), spread over every thread
-		for (uint32_t j = rs * tid; j < 1024; j += rs * nt) {
-			const uint64_t r = r0 + j;
-			const uint64_t s = c.offsets[r], e = c.offsets[r + 1];
-			const uint64_t n = e >= s ? e - s : 0;
-			uint64_t       cl = 0;
-			for (uint64_t p = 0; p < n;) {
-				const uint64_t x    = str_load8(c, s + p);
-				const uint32_t b    = static_cast<uint32_t>(x & 0xFFu);
-				const uint64_t left = n - p;
-				uint32_t       step = 0;
-				for (uint32_t k = t_start[b]; k < t_start[b + 1]; ++k) {
-					const uint32_t l = t_len[k];
-					if (l <= left && (l == 8 ? x : (x & ((1ull << (8 * l)) - 1))) == t_val[k]) {
-						step = l;
-						break;
+		__syncthreads();
+		for (uint32_t k = tid; k < S.t.n_two; k += nt) { S.pair[S.t.two[k]] = 2; }
+		__syncthreads();
+		for (uint32_t k = tid; k < S.t.n_pair; k += nt) { S.pair[S.t.pair[k]] = static_cast<uint8_t>(kStrGroup + S.t.pair_group[k]); }
+		__syncthreads();
+		for (uint64_t u = u0 + (gw + warp + nw - u0 % nw) % nw; u < u1; u += nw) {
+			const uint64_t it = item(u / kPer);
+			uint64_t       sl = 0, sc = 0;
+			{
+				const uint64_t r0   = static_cast<uint64_t>(a.items[it].vec) * 1024 + (u % kPer) * kStrUnit;
+				const uint64_t o0   = __ldg(c.offsets + r0);
+				uint32_t*      off  = S.off[warp];
+				uint16_t*      list = S.list[warp];
+				bool           wide = false;
+				__syncwarp(); // the warp's previous unit is read to the end
+				for (uint32_t j = lane; j <= kStrUnit; j += 32) {
+					const uint64_t o = __ldg(c.offsets + r0 + j) - o0;
+					wide |= o >= (1ull << 31);
+					off[j] = static_cast<uint32_t>(o);
+				}
+				__syncwarp();
+				if (__any_sync(0xFFFFFFFFu, wide)) {
+					str_unit_wide(S, c, r0, rs, lane, &sl, &sc);
+				} else {
+					// offsets from o0 below this lie at least 12 bytes before the column's end
+					const uint64_t room  = c.n_bytes > o0 ? c.n_bytes - o0 : 0;
+					const uint32_t limit = room < 12 ? 0u : room < (1u << 31) ? static_cast<uint32_t>(room) - 11 : 1u << 31;
+					auto load8 = [&](uint32_t p, bool inside) { return inside ? str_load8_inside(c, o0 + p) : str_load8(c, o0 + p); };
+					uint32_t todo = 0;
+					uint32_t at = 0, row = 0, ask = 0; // the look into the memo of the row before
+					uint64_t key = 0, seen = 0;
+					for (uint32_t j = lane; j < kStrUnit + 32; j += 32) {
+						uint32_t row_next = j, ask_next = 0, at_next = 0;
+						uint64_t key_next = 0, seen_next = 0;
+						if (j < kStrUnit) {
+							const uint32_t b = off[j], e = off[j + 1], m = e >= b ? e - b : 0;
+							const bool     inside = e < limit;
+							uint64_t       h = kStrHashSeed ^ m;
+							for (uint32_t p = 0; p < m; p += 8) { h = str_hash_step(h, load8(b + p, inside), m - p); }
+							const uint64_t r = r0 + j;
+							c.hash[r]        = h;
+							c.len[r]         = m;
+							sl += m;
+							if ((r & 1023u) % rs == 0) {
+								key_next  = str_memo_key(h, col, m, &at_next);
+								seen_next = __ldcg(memo + at_next);
+								ask_next  = 1;
+							} else {
+								c.clen[r] = 0;
+							}
+						}
+						const bool hit = ask && (seen & ~0xFFFull) == key && (seen & 0xFFFu) != 0;
+						if (hit) {
+							const uint32_t cl = static_cast<uint32_t>(seen & 0xFFFu) - 1;
+							c.clen[r0 + row]  = cl;
+							sc += cl;
+						}
+						const bool     miss = ask && !hit;
+						const uint32_t m    = __ballot_sync(0xFFFFFFFFu, miss);
+						if (miss) { list[todo + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(row); }
+						todo += __popc(m);
+						row = row_next, ask = ask_next, at = at_next, key = key_next, seen = seen_next;
+					}
+					__syncwarp();
+					uint32_t next = 0, j = 0, p = 0, left = 0, cl = 0;
+					bool     have = false, inside = false;
+					for (;;) {
+						const uint32_t idle = __ballot_sync(0xFFFFFFFFu, !have);
+						if (next < todo && (__popc(idle) >= 8 || idle == 0xFFFFFFFFu)) {
+							if (!have) {
+								const uint32_t k = next + __popc(idle & ((1u << lane) - 1u));
+								have             = k < todo;
+								if (have) {
+									j                = list[k];
+									p                = off[j];
+									const uint32_t e = off[j + 1];
+									left             = e >= p ? e - p : 0;
+									inside           = e < limit;
+									cl               = 0;
+								}
+							}
+							next += __popc(idle);
+						} else if (idle == 0xFFFFFFFFu) {
+							break;
+						}
+						if (have && left) {
+							const uint32_t step = str_next_code(S, load8(p, inside), left, &cl);
+							p += step;
+							left -= step;
+						}
+						if (have && left == 0) {
+							c.clen[r0 + j] = cl;
+							sc += cl;
+							have = false;
+						}
+					}
+					__syncwarp();
+					for (uint32_t k = lane; k < todo; k += 32) { // what was matched, for the rows to come
+						const uint64_t r = r0 + list[k];
+						const uint32_t l = c.clen[r];
+						const uint32_t b = off[list[k]], e = off[list[k] + 1];
+						key              = str_memo_key(c.hash[r], col, e >= b ? e - b : 0, &at);
+						if (l <= kStrMemoLen) { __stcg(memo + at, key | (l + 1)); }
 					}
 				}
-				cl += step ? 1 : 2;
-				p += step ? step : 1;
 			}
-			c.clen[r] = static_cast<uint32_t>(cl);
-			sc += cl;
-		}
-		sl = warp_sum(sl);
-		sc = warp_sum(sc);
-		if (lane == 0) {
-			red[0][warp] = sl;
-			red[1][warp] = sc;
-		}
-		__syncthreads();
-		if (tid == 0) {
-			uint64_t a = 0, b = 0;
-			for (int w = 0; w < kWarps; ++w) {
-				a += red[0][w];
-				b += red[1][w];
+			sl = warp_sum(sl);
+			sc = warp_sum(sc);
+			if (lane == 0) {
+				if (a.vlen) { atomicAdd(reinterpret_cast<unsigned long long*>(a.vlen + it), static_cast<unsigned long long>(sl)); }
+				if (a.vclen) { atomicAdd(reinterpret_cast<unsigned long long*>(a.vclen + it), static_cast<unsigned long long>(sc * rs)); }
 			}
-			if (vlen) { vlen[it] = a; }
-			if (vclen) { vclen[it] = b * rs; }
 		}
 	}
 }
 
-// blocks of k_str_rows (one item per block, at most 8 per SM)
-int str_rows_grid(uint64_t n_items) {
+// k_str_rows over n_items vectors, two CTAs a SM: the launch that fills the memo over as many vectors as give every
+// warp a unit, then the rest.
+cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_items, uint64_t* vlen, uint64_t* vclen,
+                            uint32_t rs, uint64_t* memo, cudaStream_t s) {
 	Device* d = current_device();
-	if (!d) { return 0; }
-	const uint64_t cap = static_cast<uint64_t>(d->sm_count) * 8;
-	return static_cast<int>(std::max<uint64_t>(1, std::min<uint64_t>(n_items, cap)));
+	if (!d || d->ordinal < 0 || d->ordinal >= 64) { return cudaErrorInvalidDevice; }
+	static bool set[64] = {};
+	if (!set[d->ordinal]) {
+		const cudaError_t e = cudaFuncSetAttribute(k_str_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(StrRowsSmem));
+		if (e != cudaSuccess) { return e; }
+		set[d->ordinal] = true;
+	}
+	cudaError_t e = cudaMemsetAsync(memo, 0, kStrMemo * 8, s);
+	if (e == cudaSuccess && vlen) { e = cudaMemsetAsync(vlen, 0, n_items * 8, s); }
+	if (e == cudaSuccess && vclen) { e = cudaMemsetAsync(vclen, 0, n_items * 8, s); }
+	if (e != cudaSuccess) { return e; }
+	const uint64_t warps = static_cast<uint64_t>(d->sm_count) * 2 * kStrWarps, per = 1024 / kStrUnit;
+	const uint64_t step  = (n_items * per + warps - 1) / warps;
+	StrRowsArgs    a {cols, items, n_items, vlen, vclen, memo, rs, static_cast<uint32_t>(std::max<uint64_t>(1, step)), 1};
+	for (const uint32_t fill : {1u, 0u}) {
+		const uint64_t n_fill = (n_items + a.stride - 1) / a.stride, n = fill ? n_fill : n_items - n_fill;
+		const uint64_t ctas   = std::min((n * per + kStrWarps - 1) / kStrWarps, static_cast<uint64_t>(d->sm_count) * 2);
+		a.fill                = fill;
+		if (ctas) {
+			k_str_rows<<<static_cast<unsigned>(ctas), kStrWarps * 32, sizeof(StrRowsSmem), s>>>(a);
+			++launch_counter();
+		}
+	}
+	return cudaGetLastError();
 }
 
 // The features of a string vector: those of its row hashes (distinct rows, runs, multiplicities), with the
@@ -1566,7 +1772,7 @@ struct fls_sel_plan {
 	// string columns (fls_sel_plan_create_strings): the plan's columns are the row hashes; these are the strings
 	bool                str = false;
 	std::vector<StrCol> scols;
-	DevMem              scols_d, tabs_d, hash_d, len_d, clen_d, wptr_d;
+	DevMem              scols_d, tabs_d, hash_d, len_d, clen_d, wptr_d, str_memo;
 	std::map<uint32_t, ItemSet> samples; // stride -> sampled items
 };
 
@@ -1661,9 +1867,10 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 		if (!p->vlen.need(n_items * 8) || !p->vclen.need(n_items * 8) || !p->dict_w.need(chunks.size() * 16)) {
 			return FLS_ERR_CUDA;
 		}
-		k_str_rows<<<str_rows_grid(n_items), kWarps * 32, 0, s>>>(p->scols_d.as<StrCol>(), items_d, n_items,
-		                                                          p->vlen.as<uint64_t>(), p->vclen.as<uint64_t>(), 1u);
-		++launch_counter();
+		if (launch_str_rows(p->scols_d.as<StrCol>(), items_d, n_items, p->vlen.as<uint64_t>(), p->vclen.as<uint64_t>(), 1u,
+		                    p->str_memo.as<uint64_t>(), s) != cudaSuccess) {
+			return FLS_ERR_CUDA;
+		}
 	}
 	ItemArgs ia {p->cols_d.as<Col>(), items_d, n_items};
 	k_parts<<<grid_for(n_items), kWarps * 32, 0, s>>>(ia, p->parts.as<uint32_t>(), p->info.as<VecInfo>());
@@ -1776,8 +1983,8 @@ int fsst_import_table(const uint8_t* buf, uint64_t avail, FsstTable* t, uint64_t
 }
 
 namespace {
-// An exported FSST table (fsst_export format) arranged for greedy matching: its symbols grouped by first byte,
-// longest first (the codes past the table's symbol count, which decode as "corrupt", are not symbols).
+// An exported FSST table (fsst_export format) arranged for greedy matching (StrTab); the codes past the table's
+// symbol count, which decode as "corrupt", are not symbols.
 int arrange_table(const uint8_t* tab, uint64_t n, StrTab* out) {
 	FsstTable t {};
 	const int rc = fsst_import_table(tab, n, &t, nullptr);
@@ -1788,21 +1995,49 @@ int arrange_table(const uint8_t* tab, uint64_t n, StrTab* out) {
 	if (zt && count) { --count; }
 	std::vector<uint32_t> codes;
 	for (uint32_t c = zt; c < zt + count && c < 255; ++c) { codes.push_back(c); }
-	std::stable_sort(codes.begin(), codes.end(), [&](uint32_t x, uint32_t y) {
-		const uint32_t bx = static_cast<uint32_t>(t.sym[x] & 0xFFu), by = static_cast<uint32_t>(t.sym[y] & 0xFFu);
-		return bx != by ? bx < by : t.len[x] > t.len[y];
-	});
 	std::memset(out, 0, sizeof(*out));
-	uint32_t k = 0;
-	for (uint32_t b = 0; b < 256; ++b) {
-		out->start[b] = static_cast<uint16_t>(k);
-		while (k < codes.size() && (t.sym[codes[k]] & 0xFFu) == b) {
-			out->val[k] = t.sym[codes[k]];
-			out->len[k] = t.len[codes[k]];
-			++k;
+	std::vector<uint32_t> longer;
+	std::vector<bool>     is_two(65536, false);
+	for (const uint32_t c : codes) {
+		const uint32_t b = static_cast<uint32_t>(t.sym[c]);
+		if (t.len[c] == 1) {
+			out->one[(b & 0xFFu) >> 5] |= 1u << (b & 31u);
+		} else if (t.len[c] == 2) {
+			out->two[out->n_two++] = static_cast<uint16_t>(b);
+			is_two[b & 0xFFFFu]    = true;
+		} else if (t.len[c] > 2) {
+			longer.push_back(c);
 		}
 	}
-	out->start[256] = static_cast<uint16_t>(k);
+	auto pair_of  = [&](uint32_t c) { return static_cast<uint32_t>(t.sym[c]) & 0xFFFFu; };
+	auto short_of = [&](uint32_t pair) { return is_two[pair] ? 2u : (out->one[(pair & 0xFFu) >> 5] >> (pair & 31u)) & 1u; };
+	// group id of every pair: its own while ids last, then one of the same g_short
+	std::map<uint32_t, uint32_t> id;
+	uint32_t                     groups = 0;
+	for (const uint32_t c : longer) {
+		const uint32_t pair = pair_of(c);
+		if (id.count(pair)) { continue; }
+		const uint32_t sh = short_of(pair);
+		uint32_t       g  = groups;
+		if (groups + 3 >= kStrGroups) { // the last three ids: one for each g_short
+			for (g = 0; g < groups && out->g_short[g] != sh; ++g) {}
+		}
+		if (g == groups) { ++groups; }
+		out->g_short[g]                 = static_cast<uint8_t>(sh);
+		out->pair[out->n_pair]          = static_cast<uint16_t>(pair);
+		out->pair_group[out->n_pair++]  = static_cast<uint8_t>(g);
+		id[pair]                        = g;
+	}
+	std::stable_sort(longer.begin(), longer.end(), [&](uint32_t x, uint32_t y) {
+		const uint32_t gx = id[pair_of(x)], gy = id[pair_of(y)];
+		return gx != gy ? gx < gy : t.len[x] > t.len[y];
+	});
+	for (size_t k = 0; k < longer.size(); ++k) {
+		out->len[k] = t.len[longer[k]];
+		out->sym[k] = make_ulonglong2(t.sym[longer[k]], ~0ull >> (64 - 8 * out->len[k]));
+		out->start[id[pair_of(longer[k])] + 1] = static_cast<uint16_t>(k + 1);
+	}
+	for (uint32_t g = 0; g < 257; ++g) { out->start[g + 1] = std::max(out->start[g], out->start[g + 1]); }
 	return FLS_OK;
 }
 } // namespace
@@ -1863,6 +2098,7 @@ int fls_sel_plan_create_strings(const fls_sel_str_column* cols, uint32_t n_cols,
 	               (rc = upload(own->wptr_d, wp.data(), sizeof(void*) * wp.size())) != FLS_OK)) {
 		return rc != FLS_OK ? rc : FLS_ERR_CUDA;
 	}
+	if (!own->str_memo.alloc(kStrMemo * 8)) { return FLS_ERR_CUDA; }
 	own->str   = true;
 	own->scols = sc;
 	own->hash_d.p = hash.p, hash.p = nullptr;
@@ -1919,9 +2155,10 @@ namespace {
 constexpr uint32_t kStrFeatRowStride = 4;
 cudaError_t        sample_features(fls_sel_plan* p, const ItemArgs& a, float* feat, cudaStream_t s) {
 	if (p->str) {
-		k_str_rows<<<str_rows_grid(a.n_items), kWarps * 32, 0, s>>>(p->scols_d.as<StrCol>(), a.items, a.n_items,
-		                                                            nullptr, nullptr, kStrFeatRowStride);
-		++launch_counter();
+		const cudaError_t e =
+		    launch_str_rows(p->scols_d.as<StrCol>(), a.items, a.n_items, nullptr, nullptr, kStrFeatRowStride,
+		                    p->str_memo.as<uint64_t>(), s);
+		if (e != cudaSuccess) { return e; }
 	}
 	cudaError_t e = launch_features(a, feat, s);
 	if (e != cudaSuccess || !p->str) { return e; }

@@ -24,6 +24,7 @@ _SIGS = {
     "fls_gpu_launch_count": (_u64, [_i]),
     "fls_gpu_test_stalled_copy": (_i, [_p, _p, _p, _p, _p, _u64, _u64, ctypes.c_uint32, _p]),
 }
+_SIGS["fls_gpu_pack_offsets"] = (_i, [_p, _u64, ctypes.c_uint32, _p, _p, _p])
 for w in (8, 16, 32, 64):
     _SIGS[f"fls_gpu_unpack_u{w}"] = (_i, [_p, _p, _p, _p, _u64, _i, _p])
     _SIGS[f"fls_gpu_unffor_u{w}"] = (_i, [_p, _p, _p, _p, _p, _u64, _i, _p])

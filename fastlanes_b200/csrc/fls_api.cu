@@ -179,116 +179,6 @@ void family_geometry(Family fam, const DecodeArgs& a, int variant, int* threads,
 	*ctas_per_sm = per;
 }
 
-// ---------------------------------------------------------------------------------------------------------
-// Encoder-side kernels (fixtures, trial encodes, benchmark data).  Thread per lane of a vector.
-// ---------------------------------------------------------------------------------------------------------
-__host__ __device__ __forceinline__ uint32_t transposed_index(uint32_t o) {
-	// inverse of original_index: o = 64a + 8b + c  ->  k = a + 16*O[b] + 128*c   (O is an involution)
-	return (o / 64) + 16 * fls_order((o / 8) % 8) + 128 * (o % 8);
-}
-
-template <typename T>
-__global__ void k_permute(const T* __restrict__ in, T* __restrict__ out, uint64_t n_vec, bool to_transposed) {
-	const uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-	if (i >= n_vec * kVec) { return; }
-	const uint64_t v = i / kVec;
-	const uint32_t k = static_cast<uint32_t>(i % kVec);
-	if (to_transposed) {
-		out[i] = in[v * kVec + original_index(k)];
-	} else {
-		out[v * kVec + original_index(k)] = in[i];
-	}
-}
-
-template <typename T, int W>
-__global__ void k_ffor(const T* __restrict__ in, T* __restrict__ out, const uint8_t* __restrict__ bw,
-                       const T* __restrict__ base, const uint64_t* __restrict__ byte_off, uint64_t n_vec) {
-	// Word-centric packing: word w of lane l gathers every value j whose bits [j*b, (j+1)*b) overlap
-	// [w*W, (w+1)*W).  Inverse of the unpack layout: lane l's word w lives at out[l + L*w].
-	constexpr uint32_t L = 1024 / W;
-	const uint64_t     i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-	if (i >= n_vec * L) { return; }
-	const uint64_t v = i / L;
-	const uint32_t l = static_cast<uint32_t>(i % L);
-	const uint32_t b = bw[v];
-	if (b == 0 || b > W) { return; }
-	T* o = reinterpret_cast<T*>(reinterpret_cast<uint8_t*>(out) + (byte_off ? byte_off[v] : v * b * 128ull));
-	const T        bs   = base ? base[v] : T(0);
-	const T*       src  = in + v * kVec;
-	const uint64_t mask = b >= 64 ? ~0ull : ((1ull << b) - 1ull);
-	for (uint32_t w = 0; w < b; ++w) {
-		const uint32_t lo_bit = w * W;
-		const uint32_t j0     = lo_bit / b;
-		const uint32_t j1     = (lo_bit + W - 1) / b;
-		uint64_t       word   = 0;
-		for (uint32_t j = j0; j <= j1 && j < static_cast<uint32_t>(W); ++j) {
-			const uint64_t x  = static_cast<uint64_t>(static_cast<T>(src[l + L * j] - bs)) & mask;
-			const int32_t  sh = static_cast<int32_t>(j * b) - static_cast<int32_t>(lo_bit);
-			if (sh >= 0) {
-				word |= sh >= 64 ? 0ull : (x << sh);
-			} else {
-				word |= (-sh) >= 64 ? 0ull : (x >> (-sh));
-			}
-		}
-		o[l + L * w] = static_cast<T>(word);
-	}
-}
-
-template <typename T, int W>
-__global__ void k_unrsum(const T* __restrict__ in, T* __restrict__ out, uint64_t n_vec) {
-	constexpr uint32_t L = 1024 / W;
-	const uint64_t     i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
-	if (i >= n_vec * L) { return; }
-	const uint64_t v = i / L;
-	const uint32_t l = static_cast<uint32_t>(i % L);
-	// lane l covers a contiguous run of original positions; walk it in order
-	uint32_t start;
-	if constexpr (W == 64) {
-		start = l * 64;
-	} else if constexpr (W == 32) {
-		start = (l % 16) * 64 + 32 * (l / 16);
-	} else {
-		start = (l % 16) * 64 + fls_order(l / 16) * 8;
-	}
-	const T* src  = in + v * kVec;
-	T*       dst  = out + v * kVec;
-	T        prev = 0;
-	for (uint32_t p = 0; p < static_cast<uint32_t>(W); ++p) {
-		const uint32_t k = transposed_index(start + p);
-		const T        x = src[k];
-		dst[k]           = p == 0 ? T(0) : static_cast<T>(x - prev);
-		prev             = x;
-	}
-}
-
-template <typename T, int W>
-__global__ void k_analyze(const T* __restrict__ in, uint8_t* __restrict__ bw, T* __restrict__ base, uint64_t n_vec,
-                          bool is_signed) {
-	// one warp per vector
-	const uint64_t v    = static_cast<uint64_t>(blockIdx.x) * (blockDim.x / 32) + threadIdx.x / 32;
-	const uint32_t lane = threadIdx.x & 31u;
-	if (v >= n_vec) { return; }
-	const T* src  = in + v * kVec;
-	const T  flip = is_signed ? static_cast<T>(T(1) << (W - 1)) : T(0);
-	T        mn = static_cast<T>(~T(0)), mx = 0;
-	for (uint32_t k = lane; k < kVec; k += 32) {
-		const T x = static_cast<T>(src[k] ^ flip);
-		mn        = x < mn ? x : mn;
-		mx        = x > mx ? x : mx;
-	}
-	for (int o = 16; o > 0; o >>= 1) {
-		const T a = __shfl_xor_sync(0xFFFFFFFFu, mn, o);
-		const T b = __shfl_xor_sync(0xFFFFFFFFu, mx, o);
-		mn        = a < mn ? a : mn;
-		mx        = b > mx ? b : mx;
-	}
-	if (lane == 0) {
-		const uint64_t d = static_cast<uint64_t>(static_cast<T>(mx - mn));
-		bw[v]            = static_cast<uint8_t>(d == 0 ? 0 : 64 - __clzll(static_cast<long long>(d)));
-		base[v]          = static_cast<T>(mn ^ flip);
-	}
-}
-
 } // namespace flsgpu
 
 // =========================================================================================================
@@ -358,49 +248,6 @@ int run_stalled(const uint32_t* in, uint32_t* out, const uint8_t* bw, const uint
 	return to_status(launch_decode(Family::NUM, a, static_cast<cudaStream_t>(stream)));
 }
 
-template <typename T>
-int run_permute(const T* in, T* out, uint64_t n_vec, bool to_transposed, fls_stream_t stream) {
-	if (n_vec == 0) { return FLS_OK; }
-	if (!in || !out) { return FLS_ERR_ARG; }
-	const uint64_t n = n_vec * kVec;
-	k_permute<T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(in, out, n_vec,
-	                                                                                                    to_transposed);
-	++launch_counter();
-	return to_status(cudaGetLastError());
-}
-
-template <typename T, int W>
-int run_ffor(const T* in, T* out, const uint8_t* bw, const T* base, const uint64_t* off, uint64_t n_vec,
-             fls_stream_t stream) {
-	if (n_vec == 0) { return FLS_OK; }
-	if (!in || !out || !bw) { return FLS_ERR_ARG; }
-	const uint64_t n = n_vec * (1024 / W);
-	k_ffor<T, W><<<static_cast<unsigned>((n + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(in, out, bw,
-	                                                                                                   base, off, n_vec);
-	++launch_counter();
-	return to_status(cudaGetLastError());
-}
-
-template <typename T, int W>
-int run_unrsum(const T* in, T* out, uint64_t n_vec, fls_stream_t stream) {
-	if (n_vec == 0) { return FLS_OK; }
-	if (!in || !out || in == out) { return FLS_ERR_ARG; }
-	const uint64_t n = n_vec * (1024 / W);
-	k_unrsum<T, W><<<static_cast<unsigned>((n + 127) / 128), 128, 0, static_cast<cudaStream_t>(stream)>>>(in, out,
-	                                                                                                     n_vec);
-	++launch_counter();
-	return to_status(cudaGetLastError());
-}
-
-template <typename T, int W>
-int run_analyze(const T* in, uint8_t* bw, T* base, uint64_t n_vec, int is_signed, fls_stream_t stream) {
-	if (n_vec == 0) { return FLS_OK; }
-	if (!in || !bw || !base) { return FLS_ERR_ARG; }
-	k_analyze<T, W><<<static_cast<unsigned>((n_vec + 7) / 8), 256, 0, static_cast<cudaStream_t>(stream)>>>(
-	    in, bw, base, n_vec, is_signed != 0);
-	++launch_counter();
-	return to_status(cudaGetLastError());
-}
 } // namespace
 
 extern "C" {
@@ -444,13 +291,6 @@ int fls_gpu_test_stalled_copy(const uint32_t* d_in, uint32_t* d_out, const uint8
 	}                                                                                                               \
 	int fls_gpu_untranspose_i_u##W(const T* in, T* out, uint64_t n, fls_stream_t s) {                               \
 		return run_primitive<W>(in, out, nullptr, W, nullptr, nullptr, nullptr, n, FLS_ORIGINAL, ENC_RAW, s);       \
-	}                                                                                                               \
-	int fls_gpu_transpose_i_u##W(const T* in, T* out, uint64_t n, fls_stream_t s) {                                 \
-		return run_permute<T>(in, out, n, true, s);                                                                 \
-	}                                                                                                               \
-	int fls_gpu_ffor_u##W(const T* in, T* out, const uint8_t* bw, const T* base, const uint64_t* off, uint64_t n,   \
-	                      fls_stream_t s) {                                                                         \
-		return run_ffor<T, W>(in, out, bw, base, off, n, s);                                                        \
 	}
 
 FLS_PRIM(uint8_t, 8)
@@ -463,10 +303,6 @@ FLS_PRIM(uint64_t, 64)
 	                             const uint64_t* off, uint64_t n, int order, fls_stream_t s) {                      \
 		if (!bw || !base || !lane_base) { return FLS_ERR_ARG; }                                                     \
 		return run_primitive<W>(in, out, bw, 0, base, lane_base, off, n, order, ENC_DELTA, s);                      \
-	}                                                                                                               \
-	int fls_gpu_unrsum_u##W(const T* in, T* out, uint64_t n, fls_stream_t s) { return run_unrsum<T, W>(in, out, n, s); } \
-	int fls_gpu_analyze_u##W(const T* in, uint8_t* bw, T* base, uint64_t n, int sg, fls_stream_t s) {               \
-		return run_analyze<T, W>(in, bw, base, n, sg, s);                                                           \
 	}
 
 FLS_PRIM2(uint16_t, 16)

@@ -106,9 +106,13 @@ def ffor(x, bw, base=None):
     """generated::ffor (base None = generated::pack): returns (packed bytes, byte offsets)."""
     w = width_of(x)
     n = x.numel() // 1024
-    off = packed_offsets(bw, w)
-    total = int((bw.to(torch.int64) * 128).sum().item())
-    out = torch.zeros(max(total, 16), dtype=torch.uint8, device=x.device)
+    off = torch.empty(bw.numel(), dtype=torch.uint64, device=x.device)
+    total = torch.empty(2, dtype=torch.int64, device=x.device)
+    check(lib.fls_gpu_pack_offsets(_ptr(bw), bw.numel(), w, _ptr(off), _ptr(total), _stream()), "pack_offsets")
+    size, bad = total.tolist()
+    # every byte is written by the packing, except for vectors of an impossible width
+    alloc = torch.zeros if bad or size < 16 else torch.empty
+    out = alloc(max(size, 16), dtype=torch.uint8, device=x.device)
     check(getattr(lib, f"fls_gpu_ffor_u{w}")(_ptr(x), _ptr(out), _ptr(bw), _ptr(base), _ptr(off), n, _stream()),
           "ffor")
     return out, off

@@ -133,6 +133,10 @@ int fls_gpu_ffor_u32(const uint32_t* d_in, uint32_t* d_out, const uint8_t* d_bw,
                      const uint64_t* d_byte_off, uint64_t n_vec, fls_stream_t stream);
 int fls_gpu_ffor_u64(const uint64_t* d_in, uint64_t* d_out, const uint8_t* d_bw, const uint64_t* d_base,
                      const uint64_t* d_byte_off, uint64_t n_vec, fls_stream_t stream);
+/* Byte offsets of densely packed vectors (d_bw[v] * 128 bytes each, no reference counterpart): d_byte_off[v] for every
+ * vector; d_total[0] the bytes of all of them, d_total[1] nonzero when a width is above `width`.  Asynchronous. */
+int fls_gpu_pack_offsets(const uint8_t* d_bw, uint64_t n_vec, uint32_t width, uint64_t* d_byte_off, uint64_t* d_total,
+                         fls_stream_t stream);
 int fls_gpu_unrsum_u16(const uint16_t* d_in, uint16_t* d_out, uint64_t n_vec, fls_stream_t stream);
 int fls_gpu_unrsum_u32(const uint32_t* d_in, uint32_t* d_out, uint64_t n_vec, fls_stream_t stream);
 int fls_gpu_unrsum_u64(const uint64_t* d_in, uint64_t* d_out, uint64_t n_vec, fls_stream_t stream);

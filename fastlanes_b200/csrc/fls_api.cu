@@ -18,8 +18,8 @@ namespace flsgpu {
 #define FLS_NUM64 64, 0u, 8, 12, 2, KIND_PLAIN
 #define FLS_NUM32 32, 0u, 4, 15, 3, KIND_PLAIN
 #define FLS_NUMPATCH 64, 0u, 8, 12, 2, KIND_PATCH
-#define FLS_GATHER 32, 0u, 8, 10, 2, KIND_GATHER
-#define FLS_GATHER32 32, 0u, 4, 12, 2, KIND_GATHER
+#define FLS_GATHER 32, 0u, 8, 16, 2, KIND_GATHER
+#define FLS_GATHER32 32, 0u, 4, 16, 2, KIND_GATHER
 #define FLS_ANY 64, 8320u, 8, 6, 2, KIND_ALL
 
 template <int MAXWS, uint32_t GSTAGE, int EMAX, int WARPS, int STAGES, int KIND>
@@ -41,7 +41,7 @@ static cudaError_t launch_family(const DecodeArgs& a, cudaStream_t s, int sm_cou
 		per_sm          = per_sm < 1 ? 1 : per_sm;
 		occupancy[dev] = per_sm;
 	}
-	const uint64_t want = (a.n_items + WARPS - 1) / WARPS;
+	const uint64_t want = a.n_items; // at most a CTA an item
 	uint64_t       grid = static_cast<uint64_t>(sm_count) * per_sm;
 	if (grid_override > 0) { grid = static_cast<uint64_t>(grid_override); }
 	if (want < grid) { grid = want; }
@@ -86,18 +86,17 @@ static const Variant kNum32[]    = {FLS_VARIANT("num32 15x3", FLS_NUM32),
                                     FLS_VARIANT("num32 10x4", 32, 0u, 4, 10, 4, KIND_PLAIN)};
 static const Variant kNumPatch[] = {FLS_VARIANT("numpatch 12x2", FLS_NUMPATCH),
                                     FLS_VARIANT("numpatch 8x3", 64, 0u, 8, 8, 3, KIND_PATCH)};
-static const Variant kGather[]   = {FLS_VARIANT("gather 10x2", FLS_GATHER),
-                                    FLS_VARIANT("gather 8x3", 32, 0u, 8, 8, 3, KIND_GATHER),
-                                    FLS_VARIANT("gather 12x2", 32, 0u, 8, 12, 2, KIND_GATHER)};
-static const Variant kGather32[] = {FLS_VARIANT("gather32 12x2", FLS_GATHER32),
-                                    FLS_VARIANT("gather32 12x3", 32, 0u, 4, 12, 3, KIND_GATHER),
-                                    FLS_VARIANT("gather32 16x2", 32, 0u, 4, 16, 2, KIND_GATHER)};
+static const Variant kGather[]   = {FLS_VARIANT("gather 16x2", FLS_GATHER),
+                                    FLS_VARIANT("gather 20x2", 32, 0u, 8, 20, 2, KIND_GATHER)};
+static const Variant kGather32[] = {FLS_VARIANT("gather32 16x2", FLS_GATHER32),
+                                    FLS_VARIANT("gather32 20x2", 32, 0u, 4, 20, 2, KIND_GATHER)};
 static const Variant kAny[]      = {FLS_VARIANT("any 6x2", FLS_ANY)};
 // filter launches (predicate bitmaps instead of values): the same geometries in their KIND_FILTER form
-static const Variant kFNum64[]    = {FLS_VARIANT("filter num64 12x2", 64, 0u, 8, 12, 2, KIND_PLAIN | KIND_FILTER)};
+// (a vector's predicate is arithmetic on registers, so warps count for more than copies in flight: one slot each)
+static const Variant kFNum64[]    = {FLS_VARIANT("filter num64 20x1", 64, 0u, 8, 20, 1, KIND_PLAIN | KIND_FILTER)};
 static const Variant kFNum32[]    = {FLS_VARIANT("filter num32 15x3", 32, 0u, 4, 15, 3, KIND_PLAIN | KIND_FILTER)};
 static const Variant kFNumPatch[] = {FLS_VARIANT("filter numpatch 12x2", 64, 0u, 8, 12, 2, KIND_PATCH | KIND_FILTER)};
-static const Variant kFGather[]   = {FLS_VARIANT("filter gather 10x2", 32, 0u, 8, 10, 2, KIND_GATHER | KIND_FILTER)};
+static const Variant kFGather[]   = {FLS_VARIANT("filter gather 16x2", 32, 0u, 8, 16, 2, KIND_GATHER | KIND_FILTER)};
 static const Variant kFGather32[] = {FLS_VARIANT("filter gather32 16x2", 32, 0u, 4, 16, 2, KIND_GATHER | KIND_FILTER)};
 static const Variant kFAny[]      = {FLS_VARIANT("filter any 6x2", 64, 8320u, 8, 6, 2, KIND_ALL | KIND_FILTER)};
 

@@ -491,6 +491,18 @@ struct ElemT<8> {
 	using T = uint64_t;
 };
 
+// 16 decoded bytes to global memory.  The output's address comes out of a plan in shared memory, so that to the compiler
+// an ordinary store through it might change the staging buffer: every read of the buffer then waited for the store
+// before it.  Nothing in a launch reads an output.
+__device__ __forceinline__ void store_out16(uint8_t* out, const uint4& x) {
+#ifdef FLS_HOST_EMULATION
+	*reinterpret_cast<uint4*>(out) = x;
+#else
+	asm volatile("st.global.v4.u32 [%0], {%1, %2, %3, %4};" ::"l"(__cvta_generic_to_global(out)), "r"(x.x), "r"(x.y), "r"(x.z),
+	             "r"(x.w));
+#endif
+}
+
 template <int WS, int E>
 __device__ __forceinline__ void store_vector(const typename OutT<E>::T (&o)[32], uint8_t* out, uint8_t* ost,
                                              bool original, uint32_t t) {
@@ -536,9 +548,9 @@ __device__ __forceinline__ void store_vector(const typename OutT<E>::T (&o)[32],
 		__syncwarp();
 		if ((reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
 #pragma unroll
-			for (uint32_t c = t; c < 64u * E; c += 32) {
-				const uint4 x = *reinterpret_cast<const uint4*>(ost + stage_off(16 * c));
-				*reinterpret_cast<uint4*>(out + 16 * c) = x;
+			for (uint32_t j = 0; j < 2u * E; ++j) {
+				const uint32_t c = 32 * j + t;
+				store_out16(out + 16 * c, *reinterpret_cast<const uint4*>(ost + stage_off(16 * c)));
 			}
 		} else {
 			for (uint32_t b = t; b < 1024u * E; b += 32) { out[b] = ost[stage_off(b)]; }
@@ -727,6 +739,191 @@ __device__ __forceinline__ void filter_small_deltas(const Plan& p, const uint32_
 // vector's predicate bitmap is written instead of its values.
 enum : int { KIND_PLAIN = 0, KIND_GATHER = 1, KIND_PATCH = 2, KIND_ALL = 3, KIND_FILTER = 4 };
 
+// The value behind an index of a gathered stream: run value (RLE), dictionary entry (DICT), or the entry of a run's
+// code (RLE_DICT).  FAST (the usual case): the arrays lie at multiples of their element sizes and every index of the
+// vector is known to be in range, so that a run value or dictionary entry costs its address and its load; a run's code
+// is still checked.  The arrays are read-only for the launch, so the loads need not wait for the stores before them.
+// Otherwise every index is checked.  GSMEM: the run values / run codes are staged in shared memory with at least 8
+// readable bytes behind them.
+template <int E, int POST, bool FAST, bool GSMEM>
+struct Gathered {
+	using OT = typename OutT<E>::T;
+	using ET = typename ElemT<E>::T;
+	const uint8_t *runs, *dict;
+	uint32_t       n_runs, entry_c;
+	bool           bad = false;
+
+	__device__ __forceinline__ Gathered(const Plan& p, const uint8_t* gstage)
+	    : runs(GSMEM ? gstage + p.ghead : p.gsrc), dict(p.dict), n_runs(p.n_runs), entry_c(p.entry_c) {}
+	__device__ __forceinline__ OT operator()(uint32_t i) {
+		const uint8_t* table = POST == POST_RLE ? runs : dict;
+		if constexpr (FAST && POST != POST_RLE_DICT) {
+			return static_cast<OT>(__ldg(reinterpret_cast<const ET*>(table) + i));
+		} else if constexpr (FAST) {
+			i             = __ldg(reinterpret_cast<const uint32_t*>(runs) + i);
+			const bool in = i < entry_c;
+			bad |= !in;
+			return in ? static_cast<OT>(__ldg(reinterpret_cast<const ET*>(table) + i)) : OT(0);
+		} else {
+			if constexpr (POST == POST_RLE_DICT) {
+				const bool in = i < n_runs;
+				bad |= !in;
+				i = !in ? 0u : GSMEM ? sld4(runs + 4ull * i) : static_cast<uint32_t>(ld_le(runs + 4ull * i, 4));
+			}
+			const bool     in = i < (POST == POST_RLE ? n_runs : entry_c);
+			const uint8_t* a  = table + static_cast<uint64_t>(i) * E;
+			bad |= !in;
+			return !in ? OT(0) : GSMEM && POST == POST_RLE ? static_cast<OT>(sld<E>(a)) : static_cast<OT>(ld_le(a, E));
+		}
+	}
+};
+
+// Indices of a vector (32 a thread, run order) to values or bitmap.  Original order: the indices go through the
+// staging buffer, 2 or 4 bytes each, and are looked up where the values leave: 32 lanes then read 32 to 256
+// neighbouring positions, whose run indices are neighbours too (one or two sectors a load where lanes 64 positions
+// apart touched 32), the buffer holds indices instead of values, and no thread keeps 32 values, so that more warps
+// fit.  32,768 vectors of RLE int32: 51.2 us with the lookups in run order, 41.0 us so; 16,000 of DICT int32 47.9, 28.7 us.
+template <int WS, int E, int POST, bool FAST, bool GSMEM, int KIND>
+__device__ __forceinline__ bool gather_post(const Plan& p, const typename StreamT<WS>::T (&v)[32], const uint8_t* gstage,
+                                            uint8_t* ost, uint32_t t, const Pred& pr) {
+	using OT = typename OutT<E>::T;
+	using ET = typename ElemT<E>::T;
+	constexpr uint32_t              IW = WS / 8; // bytes of a staged index
+	Gathered<E, POST, FAST, GSMEM> get(p, gstage);
+	const bool filter = (KIND & KIND_FILTER) != 0 && p.cmp != OUT_VALUES;
+	if (!p.order) {
+		if constexpr ((KIND & KIND_FILTER) != 0) {
+			if (filter) {
+				OT o[32];
+#pragma unroll
+				for (int i = 0; i < 32; ++i) { o[i] = get(static_cast<uint32_t>(v[i])); }
+				filter_vector<WS, E>(o, p, ost, t, pr);
+				return get.bad;
+			}
+		}
+#pragma unroll
+		for (uint32_t r = 0; r < run_count<WS>(); ++r) {
+#pragma unroll
+			for (uint32_t q = 0; q < run_len<WS>(); ++q) {
+				reinterpret_cast<ET*>(p.out)[run_tpos<WS>(t, r, q)] = static_cast<ET>(get(static_cast<uint32_t>(v[r * run_len<WS>() + q])));
+			}
+		}
+		return get.bad;
+	}
+	__syncwarp(); // the staging buffer is the stage the packed words were just read from
+#pragma unroll
+	for (uint32_t r = 0; r < run_count<WS>(); ++r) {
+#pragma unroll
+		for (uint32_t c = 0; c < run_len<WS>() * IW / 16; ++c) {
+			uint32_t w[4];
+#pragma unroll
+			for (uint32_t k = 0; k < 4; ++k) {
+				if constexpr (WS == 16) {
+					const uint32_t i = r * 16 + c * 8 + 2 * k;
+					w[k]             = v[i] | (v[i + 1] << 16);
+				} else {
+					w[k] = static_cast<uint32_t>(v[c * 4 + k]);
+				}
+			}
+			*reinterpret_cast<uint4*>(ost + stage_off(run_start<WS>(t, r) * IW + 16 * c)) = make_uint4(w[0], w[1], w[2], w[3]);
+		}
+	}
+	__syncwarp();
+	auto index = [&](uint32_t pos) {
+		const uint8_t* a = ost + stage_off(pos * IW);
+		return WS == 16 ? static_cast<uint32_t>(*reinterpret_cast<const uint16_t*>(a)) : *reinterpret_cast<const uint32_t*>(a);
+	};
+	if constexpr ((KIND & KIND_FILTER) != 0) {
+		if (filter) {
+			const PredE<E> holds(pr, p.cmp == OUT_BITMAP_S);
+			uint32_t       mine = 0;
+#pragma unroll 8
+			for (uint32_t w = 0; w < 32; ++w) {
+				const uint32_t b = __ballot_sync(0xFFFFFFFFu, holds.in(get(index(32 * w + t))));
+				if (w == t) { mine = b; }
+			}
+			reinterpret_cast<uint32_t*>(p.out)[t] = mine ^ holds.flip;
+			__syncwarp();
+			return get.bad;
+		}
+	}
+	if ((reinterpret_cast<uintptr_t>(p.out) & 15u) == 0) {
+		constexpr uint32_t PER = 16 / E; // values a 16-byte store
+		constexpr uint32_t kUnroll = !FAST ? 1 : E == 8 ? 4 : 2 * E; // (8-byte values: more code in line costs small batches)
+#pragma unroll kUnroll
+		for (uint32_t j = 0; j < 2u * E; ++j) { // (a trip count known without t)
+			const uint32_t c = 32 * j + t;
+			// the PER indices lie in one 16-byte piece (two for 2-byte values of 4-byte indices)
+			uint32_t       idx[PER];
+			const uint8_t* a = ost + stage_off(c * PER * IW);
+			if constexpr (PER * IW == 4) {
+				const uint32_t x = *reinterpret_cast<const uint32_t*>(a);
+				idx[0] = x & 0xFFFFu, idx[1] = x >> 16;
+			} else if constexpr (PER * IW == 8 && IW == 2) {
+				const uint2 x = *reinterpret_cast<const uint2*>(a);
+				idx[0] = x.x & 0xFFFFu, idx[1] = x.x >> 16, idx[2] = x.y & 0xFFFFu, idx[3] = x.y >> 16;
+			} else if constexpr (PER * IW == 8) {
+				const uint2 x = *reinterpret_cast<const uint2*>(a);
+				idx[0] = x.x, idx[1] = x.y;
+			} else if constexpr (PER * IW == 16 && IW == 4) {
+				const uint4 x = *reinterpret_cast<const uint4*>(a);
+				idx[0] = x.x, idx[1] = x.y, idx[2] = x.z, idx[3] = x.w;
+			} else {
+#pragma unroll
+				for (uint32_t i = 0; i < PER; ++i) { idx[i] = index(c * PER + i); }
+			}
+			OT o[PER];
+#pragma unroll
+			for (uint32_t i = 0; i < PER; ++i) { o[i] = get(idx[i]); }
+			uint32_t w[4];
+#pragma unroll
+			for (uint32_t k = 0; k < 4; ++k) {
+				if constexpr (E == 8) {
+					w[k] = static_cast<uint32_t>(o[k / 2] >> (32 * (k & 1)));
+				} else if constexpr (E == 4) {
+					w[k] = static_cast<uint32_t>(o[k]);
+				} else {
+					w[k] = (static_cast<uint32_t>(o[2 * k]) & 0xFFFFu) | (static_cast<uint32_t>(o[2 * k + 1]) << 16);
+				}
+			}
+			store_out16(p.out + 16 * c, make_uint4(w[0], w[1], w[2], w[3]));
+		}
+	} else {
+		for (uint32_t i = t; i < kVec; i += 32) { reinterpret_cast<ET*>(p.out)[i] = static_cast<ET>(get(index(i))); }
+	}
+	__syncwarp();
+	return get.bad;
+}
+
+template <int WS, int E, bool GSMEM, int KIND>
+__device__ __forceinline__ void gather_vector(const Plan& p, const typename StreamT<WS>::T (&v)[32], const uint8_t* gstage,
+                                              uint8_t* ost, uint32_t t, int* status, const Pred& pr) {
+	// the largest index decides once for the vector whether its indices need checking
+	uint32_t top = 0;
+#pragma unroll
+	for (int i = 0; i < 32; ++i) { top = top < static_cast<uint32_t>(v[i]) ? static_cast<uint32_t>(v[i]) : top; }
+	const bool rle    = WS == 16;
+	bool       direct = top < (rle ? p.n_runs : p.entry_c);
+	direct            = !__any_sync(0xFFFFFFFFu, !direct);
+	const uintptr_t dict = reinterpret_cast<uintptr_t>(p.dict), runs = reinterpret_cast<uintptr_t>(p.gsrc);
+	bool            bad;
+	if constexpr (WS == 16) {
+		if (p.post == POST_RLE) {
+			bad = !GSMEM && direct && (runs & (E - 1)) == 0
+			          ? gather_post<WS, E, POST_RLE, true, false, KIND>(p, v, gstage, ost, t, pr)
+			          : gather_post<WS, E, POST_RLE, false, GSMEM, KIND>(p, v, gstage, ost, t, pr);
+		} else {
+			bad = !GSMEM && direct && (runs & 3u) == 0 && (dict & (E - 1)) == 0
+			          ? gather_post<WS, E, POST_RLE_DICT, true, false, KIND>(p, v, gstage, ost, t, pr)
+			          : gather_post<WS, E, POST_RLE_DICT, false, GSMEM, KIND>(p, v, gstage, ost, t, pr);
+		}
+	} else {
+		bad = direct && (dict & (E - 1)) == 0 ? gather_post<WS, E, POST_DICT, true, false, KIND>(p, v, gstage, ost, t, pr)
+		                                      : gather_post<WS, E, POST_DICT, false, false, KIND>(p, v, gstage, ost, t, pr);
+	}
+	if (__any_sync(0xFFFFFFFFu, bad) && t == 0) { atomicOr(status, STATUS_BAD_INDEX); }
+}
+
 template <int WS, int E, bool GSMEM = true, int KIND = KIND_ALL>
 __device__ __forceinline__ void decode_vector(const Plan& p, const uint8_t* stage, const uint8_t* gstage, uint8_t* ost,
                                               uint32_t t, int* status, const Pred& pr = Pred {}) {
@@ -743,56 +940,20 @@ __device__ __forceinline__ void decode_vector(const Plan& p, const uint8_t* stag
 	ST v[32];
 	decode_stream<WS, PATCH>(p, reinterpret_cast<const uint32_t*>(stage), t, v, ost, status);
 	if (!PATCH && post_is_patch(p.post) && t == 0) { atomicOr(status, STATUS_BAD_LAYOUT); }
-	OT o[32];
-	bool bad = false;
-	if (!GATHER || !post_is_gather(p.post)) {
-#pragma unroll
-		for (int i = 0; i < 32; ++i) { o[i] = static_cast<OT>(v[i]); }
-		if (!GATHER && post_is_gather(p.post) && t == 0) { atomicOr(status, STATUS_BAD_LAYOUT); }
-	} else if (p.post == POST_RLE) {
-		// run values keep the byte alignment they have inside the page
-		const uint8_t* vals = GSMEM ? gstage + p.ghead : p.gsrc;
-		if (!GSMEM && (reinterpret_cast<uintptr_t>(vals) & (E - 1)) == 0) {
-			// naturally aligned run values (the usual case): plain loads, no per-value alignment test
-			using VT        = typename ElemT<E>::T;
-			const VT* tvals = reinterpret_cast<const VT*>(vals);
-#pragma unroll
-			for (int i = 0; i < 32; ++i) {
-				const uint32_t idx = static_cast<uint32_t>(v[i]);
-				const bool     in  = idx < p.n_runs;
-				bad |= !in;
-				o[i] = in ? static_cast<OT>(tvals[idx]) : OT(0);
-			}
-		} else {
-#pragma unroll
-			for (int i = 0; i < 32; ++i) {
-				const uint32_t idx = static_cast<uint32_t>(v[i]);
-				const bool     in  = idx < p.n_runs;
-				bad |= !in;
-				const uint8_t* a = vals + static_cast<uint64_t>(idx) * E;
-				o[i] = !in ? OT(0) : GSMEM ? static_cast<OT>(sld<E>(a)) : static_cast<OT>(ld_le(a, E));
-			}
-		}
-	} else {
-		const uint8_t* codes        = GSMEM ? gstage + p.ghead : p.gsrc;
-		const bool     dict_aligned = (reinterpret_cast<uintptr_t>(p.dict) & (E - 1)) == 0;
-#pragma unroll
-		for (int i = 0; i < 32; ++i) {
-			uint32_t code = static_cast<uint32_t>(v[i]);
-			if (p.post == POST_RLE_DICT) {
-				const bool     in = code < p.n_runs;
-				const uint8_t* a  = codes + 4ull * code;
-				bad |= !in;
-				code = !in ? 0u : GSMEM ? sld4(a) : static_cast<uint32_t>(ld_le(a, 4));
-			}
-			const bool in = code < p.entry_c;
-			bad |= !in;
-			const uint8_t* a = p.dict + static_cast<uint64_t>(code) * E;
-			o[i] = !in ? OT(0) : dict_aligned ? static_cast<OT>(*reinterpret_cast<const typename ElemT<E>::T*>(a))
-			                                  : static_cast<OT>(ld_le(a, E));
+	if constexpr (GATHER && (WS == 16 || WS == 32)) {
+		if (post_is_gather(p.post)) {
+			gather_vector<WS, E, GSMEM, KIND>(p, v, gstage, ost, t, status, pr);
+			return;
 		}
 	}
-	if (__any_sync(0xFFFFFFFFu, bad) && t == 0) { atomicOr(status, STATUS_BAD_INDEX); }
+	// streams of other widths are never gathered from, and a kernel for gathers alone has no room to stage values
+	if (post_is_gather(p.post) || (KIND & KIND_ALL) == KIND_GATHER) {
+		if (t == 0) { atomicOr(status, STATUS_BAD_LAYOUT); }
+		return;
+	}
+	OT o[32];
+#pragma unroll
+	for (int i = 0; i < 32; ++i) { o[i] = static_cast<OT>(v[i]); }
 	if constexpr ((KIND & KIND_FILTER) != 0) {
 		bool values = false;
 		if constexpr ((KIND & KIND_PATCH) != 0) {
@@ -888,7 +1049,9 @@ template <int MAXWS, uint32_t GSTAGE, int EMAX, int WARPS, int STAGES, int KIND 
 struct Geometry {
 	static constexpr uint32_t kPB      = 16;
 	static constexpr uint32_t kStage   = MAXWS * 128u;
-	static constexpr uint32_t kOut     = EMAX * 1024u;
+	// what a vector is staged in on its way out: its values, or (gathers) its indices, at most 4 bytes each; a filter of
+	// plain streams keeps its values in registers
+	static constexpr uint32_t kOut     = (KIND & KIND_ALL) == KIND_GATHER ? 4096u : KIND == (KIND_PLAIN | KIND_FILTER) ? 1024u : EMAX * 1024u;
 	static constexpr uint32_t kMain    = kStage > kOut ? kStage : kOut;
 	static constexpr uint32_t kSlot    = kMain + kLaneWindow + GSTAGE;
 	static constexpr uint32_t kPlans   = 2 * kPB * sizeof(PlanS);
@@ -938,21 +1101,25 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_decode(const DecodeArgs a) {
 	PlanS*         plans  = reinterpret_cast<PlanS*>(wbase + 64);
 	uint8_t*       stages = wbase + 64 + G::kPlans;
 
+	// fewer items than warps: they go to the CTAs in turn, so that a small batch spreads over the SMs (100 vectors on
+	// 100 SMs instead of 7)
+	const uint64_t n  = a.n_items;
+	const uint64_t nw = static_cast<uint64_t>(gridDim.x) * WARPS;
+	const uint64_t gw = n < nw ? static_cast<uint64_t>(warp) * gridDim.x + blockIdx.x : static_cast<uint64_t>(blockIdx.x) * WARPS + warp;
+	if (gw >= n) { return; } // (warps never wait for one another)
+
 	if (lane == 0) {
 		for (int s = 0; s < STAGES; ++s) { mbar_init(&bars[s], 1); }
 		fence_mbar_init();
 	}
 
-	const uint64_t gw = static_cast<uint64_t>(blockIdx.x) * WARPS + warp;
-	const uint64_t nw = static_cast<uint64_t>(gridDim.x) * WARPS;
-	const uint64_t n  = a.n_items;
-
 	auto stage_ptr  = [&](uint32_t s) { return stages + s * G::kSlot; };
 	auto lb_ptr     = [&](uint32_t s) { return stages + s * G::kSlot + G::kMain; };
 	auto gstage_ptr = [&](uint32_t s) { return stages + s * G::kSlot + G::kMain + kLaneWindow; };
-	// Lane-parallel metadata fetch: lane j resolves the plan of the warp's item blk*PB + j.
-	auto fill = [&](uint32_t blk) {
-		if (lane < PB) {
+	// Lane-parallel metadata fetch: lane j resolves the plan of the warp's item blk*PB + j (count of them).
+	static_assert(PB == 16, "the first fill takes both halves of the ring");
+	auto fill = [&](uint32_t blk, uint32_t count) {
+		if (lane < count) {
 			const uint64_t k    = static_cast<uint64_t>(blk) * PB + lane;
 			const uint64_t item = gw + k * nw;
 			Plan           p {};
@@ -970,8 +1137,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_decode(const DecodeArgs a) {
 	};
 	const uint32_t limit = a.spin_limit ? a.spin_limit : kMbarSpinLimit;
 
-	fill(0);
-	fill(1);
+	fill(0, 32); // both halves of the ring at once
 	__syncwarp();
 	for (uint32_t s = 0; s < STAGES; ++s) { issue_k(s, s); }
 
@@ -979,7 +1145,7 @@ __global__ void __launch_bounds__(WARPS * 32, 1) k_decode(const DecodeArgs a) {
 	bool     aborted = false;
 	for (uint64_t item = gw; item < n; item += nw, ++k) {
 		if (k % PB == 0 && k > 0) {
-			fill(k / PB + 1);
+			fill(k / PB + 1, PB);
 			__syncwarp();
 		}
 		const uint32_t s      = k % STAGES;

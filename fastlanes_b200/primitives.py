@@ -17,11 +17,23 @@ _DTYPE = {8: torch.uint8, 16: torch.uint16, 32: torch.uint32, 64: torch.uint64}
 
 
 def _stream():
-    return ctypes_stream(torch.cuda.current_stream())
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def ctypes_stream(s):
     return s.cuda_stream
+
+
+class _ByWidth(dict):
+    def __missing__(self, w):
+        raise AttributeError(f"no such primitive for width {w}")
+
+
+# the library's functions by width, looked up once (a call's own time is what a small batch costs)
+_FN = {op: _ByWidth({w: getattr(lib, f"fls_gpu_{op}_u{w}") for w in ws}) for op, ws in
+       {"unpack": (8, 16, 32, 64), "unffor": (8, 16, 32, 64), "rsum": (8, 16, 32, 64), "unffor_rsum": (16, 32, 64),
+        "untranspose_i": (8, 16, 32, 64), "transpose_i": (8, 16, 32, 64), "ffor": (8, 16, 32, 64),
+        "unrsum": (16, 32, 64), "analyze": (16, 32, 64)}.items()}
 
 
 def _ptr(t):
@@ -45,7 +57,7 @@ def unpack(packed, bw, byte_off=None, order=TRANSPOSED, width=None):
     w = width or width_of(packed)
     n = bw.numel()
     out = torch.empty(n * 1024, dtype=_DTYPE[w], device=packed.device)
-    check(getattr(lib, f"fls_gpu_unpack_u{w}")(_ptr(packed), _ptr(out), _ptr(bw), _ptr(byte_off), n, order,
+    check(_FN["unpack"][w](_ptr(packed), _ptr(out), _ptr(bw), _ptr(byte_off), n, order,
                                                _stream()), "unpack")
     return out
 
@@ -55,7 +67,7 @@ def unffor(packed, bw, base, byte_off=None, order=TRANSPOSED):
     w = width_of(base)
     n = bw.numel()
     out = torch.empty(n * 1024, dtype=_DTYPE[w], device=base.device)
-    check(getattr(lib, f"fls_gpu_unffor_u{w}")(_ptr(packed), _ptr(out), _ptr(bw), _ptr(base), _ptr(byte_off), n,
+    check(_FN["unffor"][w](_ptr(packed), _ptr(out), _ptr(bw), _ptr(base), _ptr(byte_off), n,
                                                order, _stream()), "unffor")
     return out
 
@@ -65,7 +77,7 @@ def rsum(deltas, lane_base, order=TRANSPOSED):
     w = width_of(deltas)
     n = deltas.numel() // 1024
     out = torch.empty_like(deltas)
-    check(getattr(lib, f"fls_gpu_rsum_u{w}")(_ptr(deltas), _ptr(out), _ptr(lane_base), n, order, _stream()), "rsum")
+    check(_FN["rsum"][w](_ptr(deltas), _ptr(out), _ptr(lane_base), n, order, _stream()), "rsum")
     return out
 
 
@@ -74,7 +86,7 @@ def unffor_rsum(packed, bw, base, lane_base, byte_off=None, order=TRANSPOSED):
     w = width_of(base)
     n = bw.numel()
     out = torch.empty(n * 1024, dtype=_DTYPE[w], device=base.device)
-    check(getattr(lib, f"fls_gpu_unffor_rsum_u{w}")(_ptr(packed), _ptr(out), _ptr(bw), _ptr(base), _ptr(lane_base),
+    check(_FN["unffor_rsum"][w](_ptr(packed), _ptr(out), _ptr(bw), _ptr(base), _ptr(lane_base),
                                                     _ptr(byte_off), n, order, _stream()), "unffor_rsum")
     return out
 
@@ -83,7 +95,7 @@ def untranspose_i(x):
     """generated::untranspose::untranspose_i (untranspose_o is the same permutation)."""
     w = width_of(x)
     out = torch.empty_like(x)
-    check(getattr(lib, f"fls_gpu_untranspose_i_u{w}")(_ptr(x), _ptr(out), x.numel() // 1024, _stream()),
+    check(_FN["untranspose_i"][w](_ptr(x), _ptr(out), x.numel() // 1024, _stream()),
           "untranspose_i")
     return out
 
@@ -95,7 +107,7 @@ def transpose_i(x):
     """generated::transpose::transpose_i (transpose_o is the same permutation)."""
     w = width_of(x)
     out = torch.empty_like(x)
-    check(getattr(lib, f"fls_gpu_transpose_i_u{w}")(_ptr(x), _ptr(out), x.numel() // 1024, _stream()), "transpose_i")
+    check(_FN["transpose_i"][w](_ptr(x), _ptr(out), x.numel() // 1024, _stream()), "transpose_i")
     return out
 
 
@@ -113,7 +125,7 @@ def ffor(x, bw, base=None):
     # every byte is written by the packing, except for vectors of an impossible width
     alloc = torch.zeros if bad or size < 16 else torch.empty
     out = alloc(max(size, 16), dtype=torch.uint8, device=x.device)
-    check(getattr(lib, f"fls_gpu_ffor_u{w}")(_ptr(x), _ptr(out), _ptr(bw), _ptr(base), _ptr(off), n, _stream()),
+    check(_FN["ffor"][w](_ptr(x), _ptr(out), _ptr(bw), _ptr(base), _ptr(off), n, _stream()),
           "ffor")
     return out, off
 
@@ -126,7 +138,7 @@ def unrsum(x):
     """generated::unrsum: deltas along each lane (first element of a lane becomes 0)."""
     w = width_of(x)
     out = torch.empty_like(x)
-    check(getattr(lib, f"fls_gpu_unrsum_u{w}")(_ptr(x), _ptr(out), x.numel() // 1024, _stream()), "unrsum")
+    check(_FN["unrsum"][w](_ptr(x), _ptr(out), x.numel() // 1024, _stream()), "unrsum")
     return out
 
 
@@ -136,7 +148,7 @@ def analyze(x, signed=False):
     n = x.numel() // 1024
     bw = torch.empty(n, dtype=torch.uint8, device=x.device)
     base = torch.empty(n, dtype=x.dtype, device=x.device)
-    check(getattr(lib, f"fls_gpu_analyze_u{w}")(_ptr(x), _ptr(bw), _ptr(base), n, int(signed), _stream()), "analyze")
+    check(_FN["analyze"][w](_ptr(x), _ptr(bw), _ptr(base), n, int(signed), _stream()), "analyze")
     return bw, base
 
 

@@ -30,7 +30,6 @@ namespace sel {
 constexpr int      K        = FLS_SEL_K;
 constexpr int      NF       = FLS_SEL_FEATURES;
 constexpr int      H        = FLS_SEL_HIDDEN;
-constexpr uint64_t kEmpty   = ~0ull;      // empty key of the hash tables; the value ~0 itself has a slot of its own
 constexpr uint32_t kMaxVecPerChunk = 64;
 constexpr int      kWarps   = 8;
 
@@ -178,55 +177,77 @@ __device__ __forceinline__ uint32_t pack_parts(const Parts& p) {
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Statistics of the learned selector (one warp, one vector).  hkeys / hcnt: this warp's 2048-slot table.
+// Statistics of the learned selector (one warp, one vector).  slots: this warp's table, 2048 entries of 11 hash bits,
+// the 10-bit position of the key's first value put in (the key itself: vals holds the vector) and an 11-bit count.
+// 4 bytes an entry instead of 12 let 16 warps run on an SM instead of 8, and the loop over the vector's rows, instead
+// of 32 inserts in line, fits the instruction cache: the kernel waited on latency and on instruction fetch.
+// 3,660 vectors: 105 us, 79 us so.
 // ---------------------------------------------------------------------------------------------------------
 constexpr uint32_t kHSlots = 2048;
 
-__device__ __forceinline__ uint32_t hash_slot(uint64_t x, uint32_t bits) {
-	return static_cast<uint32_t>((x * 0x9E3779B97F4A7C15ull) >> (64 - bits));
+template <class T>
+__device__ __forceinline__ uint32_t feat_hash(T x) {
+	uint32_t a = static_cast<uint32_t>(x) * 0x9E3779B1u;
+	if constexpr (sizeof(T) == 8) { a += static_cast<uint32_t>(x >> 32) * 0x85EBCA77u; }
+	a ^= a >> 15;
+	a *= 0x2C1B3C6Du;
+	return a ^ (a >> 13);
+}
+
+// Counts of the vector's values into the (empty) table: a row of 32 neighbouring values a step, one insert a run.
+template <class T>
+__device__ __forceinline__ void count_values(const T* vals, uint32_t lane, uint32_t* slots) {
+#pragma unroll 2
+	for (uint32_t r = 0; r < 32; ++r) {
+		const T        x     = __ldg(vals + 32 * r + lane);
+		const T        prev  = __shfl_up_sync(0xFFFFFFFFu, x, 1);
+		const bool     start = lane == 0 || x != prev;
+		const uint32_t after = (__ballot_sync(0xFFFFFFFFu, start) >> lane) >> 1; // the starts past this lane
+		if (start) {
+			const uint32_t weight = after ? __ffs(after) : 32 - lane;
+			const uint32_t h      = feat_hash(x);
+			const uint32_t tag = h << 21, mine = tag | ((32 * r + lane) << 11) | weight;
+			uint32_t       s   = h >> 21;
+			for (uint32_t probe = 0; probe < kHSlots; ++probe) {
+				uint32_t e = *reinterpret_cast<volatile uint32_t*>(slots + s);
+				if (e == 0) {
+					e = atomicCAS(slots + s, 0u, mine);
+					if (e == 0) { break; }
+				}
+				if ((e ^ tag) < (1u << 21) && __ldg(vals + ((e >> 11) & 1023u)) == x) {
+					atomicAdd(slots + s, weight);
+					break;
+				}
+				s = (s + 1) & (kHSlots - 1);
+			}
+		}
+	}
+	__syncwarp();
 }
 
 template <int W>
 __device__ void vector_features(const typename UT<W>::T (&x)[32], uint32_t lane, bool sgn, const Parts& P,
-                                uint64_t* hkeys, uint32_t* hcnt, float* out) {
+                                const typename UT<W>::T* vals, uint32_t* slots, float* out) {
 	using T             = typename UT<W>::T;
 	const T        flip = sgn ? (T(1) << (W - 1)) : T(0);
 	const uint32_t sm   = P.start_mask;
-	// distinct values and the top multiplicity (exact: 1024 values in 2048 slots; the key ~0 counts aside)
-	uint32_t sentinel = 0;
-#pragma unroll
-	for (int i = 0; i < 32; ++i) {
-		const uint64_t key = static_cast<uint64_t>(x[i]);
-		if (key == kEmpty) {
-			++sentinel;
-			continue;
-		}
-		uint32_t h = hash_slot(key, 11);
-		for (uint32_t probe = 0; probe < kHSlots; ++probe) {
-			const uint64_t old = atomicCAS(reinterpret_cast<unsigned long long*>(hkeys + h), kEmpty, key);
-			if (old == kEmpty || old == key) {
-				atomicAdd(hcnt + h, 1u);
-				break;
-			}
-			h = (h + 1) & (kHSlots - 1);
-		}
-	}
-	__syncwarp();
+	// distinct values and the top multiplicity (exact: 1024 values in 2048 slots)
+	count_values(vals, lane, slots);
 	uint32_t dv = 0, top = 0;
-	for (uint32_t s = lane; s < kHSlots; s += 32) {
-		const uint32_t c = hcnt[s];
-		dv += c ? 1u : 0u;
-		top = c > top ? c : top;
-		hkeys[s] = kEmpty;
-		hcnt[s]  = 0;
+	for (uint32_t s = lane; s < kHSlots / 4; s += 32) {
+		const uint4    e    = reinterpret_cast<const uint4*>(slots)[s];
+		const uint32_t w[4] = {e.x, e.y, e.z, e.w};
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			const uint32_t c = w[i] & 0x7FFu;
+			dv += c ? 1u : 0u;
+			top = c > top ? c : top;
+		}
+		reinterpret_cast<uint4*>(slots)[s] = make_uint4(0, 0, 0, 0);
 	}
-	dv       = warp_sum(dv);
-	top      = warp_max(top);
-	sentinel = warp_sum(sentinel);
-	if (sentinel) {
-		++dv;
-		top = sentinel > top ? sentinel : top;
-	}
+	dv  = warp_sum(dv);
+	top = warp_max(top);
+	__syncwarp();
 	// adjacency in original order: increases, decreases, largest |difference|
 	const T  prev = __shfl_sync(0xFFFFFFFFu, x[31], prev_run_lane(lane));
 	uint32_t inc = 0, dec = 0, bw_a = 0;
@@ -404,17 +425,13 @@ __global__ void __launch_bounds__(kWarps * 32) k_parts(ItemArgs a, uint32_t* par
 	}
 }
 
-constexpr uint32_t kFeatSmem = kWarps * kHSlots * (8 + 4);
+constexpr uint32_t kFeatSmem = kWarps * kHSlots * 4;
 
-__global__ void __launch_bounds__(kWarps * 32) k_features(ItemArgs a, float* feat) {
+__global__ void __launch_bounds__(kWarps * 32, 2) k_features(ItemArgs a, float* feat) {
 	extern __shared__ __align__(16) uint8_t fsm[];
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-	uint64_t*      hk   = reinterpret_cast<uint64_t*>(fsm) + warp * kHSlots;
-	uint32_t*      hc   = reinterpret_cast<uint32_t*>(fsm + kWarps * kHSlots * 8) + warp * kHSlots;
-	for (uint32_t s = lane; s < kHSlots; s += 32) {
-		hk[s] = kEmpty;
-		hc[s] = 0;
-	}
+	uint32_t*      hs   = reinterpret_cast<uint32_t*>(fsm) + warp * kHSlots;
+	for (uint32_t s = lane; s < kHSlots; s += 32) { hs[s] = 0; }
 	__syncwarp();
 	for (uint64_t it = blockIdx.x * static_cast<uint64_t>(kWarps) + warp; it < a.n_items;
 	     it += static_cast<uint64_t>(gridDim.x) * kWarps) {
@@ -424,12 +441,12 @@ __global__ void __launch_bounds__(kWarps * 32) k_features(ItemArgs a, float* fea
 			uint64_t x[32];
 			load_run<64>(c, m.vec, lane, x);
 			const Parts P = vector_parts<64>(x, lane, c.sgn != 0);
-			vector_features<64>(x, lane, c.sgn != 0, P, hk, hc, feat + it * NF);
+			vector_features<64>(x, lane, c.sgn != 0, P, reinterpret_cast<const uint64_t*>(c.values) + m.vec * 1024ull, hs, feat + it * NF);
 		} else {
 			uint32_t x[32];
 			load_run<32>(c, m.vec, lane, x);
 			const Parts P = vector_parts<32>(x, lane, c.sgn != 0);
-			vector_features<32>(x, lane, c.sgn != 0, P, hk, hc, feat + it * NF);
+			vector_features<32>(x, lane, c.sgn != 0, P, reinterpret_cast<const uint32_t*>(c.values) + m.vec * 1024ull, hs, feat + it * NF);
 		}
 		__syncwarp();
 	}
@@ -1520,9 +1537,94 @@ __global__ void __launch_bounds__(256) k_gemm(int M, int N, int Kd, const float*
 	}
 }
 
-// Softmax of every row of Z (n x K) into P; with labels: dZ = (P - onehot) / n and the mean loss added to
-// *loss (and to loss_hist[*step] when given).
-__global__ void k_softmax(const float* Z, uint64_t n, float* P, const int32_t* y, float* dZ, float* loss,
+// Class probabilities of n feature rows: the whole forward pass of the MLP, 32 rows a CTA, every layer's activations
+// and all weights in shared memory.  Each sum runs over k in order, as k_gemm's do, and the softmax is k_softmax's, so
+// the results are theirs bit for bit.  The three products, the softmax and their round trips through global memory
+// were four launches of 3 to 30 us (each of 116 CTAs of 64-row tiles, a quarter of the SMs idle); this one takes 23 us from cold
+// caches for 3,660 rows.
+constexpr uint32_t kMlpRows = 32;
+struct MlpSmem {
+	float w2[H][H], w1[NF][H], w3[H][K + 2];
+	float b1[H], b2[H], b3[K + 2];
+	float x[kMlpRows][NF + 1], h1[kMlpRows][H + 4], h2[kMlpRows][H + 4];
+};
+
+// out[rows][H] = relu(in[rows][KD] * w + b): thread (tx, ty) takes columns 4 tx .. + 3 of rows ty, ty + 8, + 16, + 24
+template <int KD, int LDA>
+__device__ __forceinline__ void mlp_layer(const float (*in)[LDA], const float (*w)[H], const float* b, float (*out)[H + 4],
+                                          uint32_t tx, uint32_t ty) {
+	float acc[4][4] = {};
+#pragma unroll 8
+	for (int k = 0; k < KD; ++k) {
+		const float4 wv = *reinterpret_cast<const float4*>(&w[k][4 * tx]);
+#pragma unroll
+		for (int i = 0; i < 4; ++i) {
+			const float a = in[ty + 8 * i][k];
+			acc[i][0] = fmaf(a, wv.x, acc[i][0]), acc[i][1] = fmaf(a, wv.y, acc[i][1]);
+			acc[i][2] = fmaf(a, wv.z, acc[i][2]), acc[i][3] = fmaf(a, wv.w, acc[i][3]);
+		}
+	}
+#pragma unroll
+	for (int i = 0; i < 4; ++i) {
+#pragma unroll
+		for (int j = 0; j < 4; ++j) { out[ty + 8 * i][4 * tx + j] = fmaxf(acc[i][j] + b[4 * tx + j], 0.0f); }
+	}
+}
+
+__global__ void __launch_bounds__(256) k_mlp(const float* __restrict__ params, const float* __restrict__ X, uint64_t n,
+                                             float* __restrict__ P) {
+	extern __shared__ __align__(16) uint8_t smem[];
+	MlpSmem&       S   = *reinterpret_cast<MlpSmem*>(smem);
+	const uint32_t tid = threadIdx.x, tx = tid % 32, ty = tid / 32;
+	const float*   w1 = params;
+	const float *  b1 = w1 + NF * H, *w2 = b1 + H, *b2 = w2 + H * H, *w3 = b2 + H, *b3 = w3 + H * K;
+	for (uint32_t e = tid; e < NF * H; e += 256) { S.w1[e / H][e % H] = __ldg(w1 + e); }
+	for (uint32_t e = tid; e < H * H; e += 256) { S.w2[e / H][e % H] = __ldg(w2 + e); }
+	for (uint32_t e = tid; e < H * K; e += 256) { S.w3[e / K][e % K] = __ldg(w3 + e); }
+	if (tid < H) {
+		S.b1[tid] = b1[tid];
+		S.b2[tid] = b2[tid];
+	}
+	if (tid < K) { S.b3[tid] = b3[tid]; }
+	for (uint64_t r0 = static_cast<uint64_t>(blockIdx.x) * kMlpRows; r0 < n; r0 += static_cast<uint64_t>(gridDim.x) * kMlpRows) {
+		for (uint32_t e = tid; e < kMlpRows * NF; e += 256) {
+			S.x[e / NF][e % NF] = r0 + e / NF < n ? __ldg(X + r0 * NF + e) : 0.0f;
+		}
+		__syncthreads();
+		mlp_layer<NF, NF + 1>(S.x, S.w1, S.b1, S.h1, tx, ty);
+		__syncthreads();
+		mlp_layer<H, H + 4>(S.h1, S.w2, S.b2, S.h2, tx, ty);
+		__syncthreads();
+		if (tid < kMlpRows * K) { // a logit a thread, into x
+			const uint32_t r = tid / K, c = tid % K;
+			float          acc = 0.0f;
+#pragma unroll 8
+			for (int k = 0; k < H; ++k) { acc = fmaf(S.h2[r][k], S.w3[k][c], acc); }
+			S.x[r][c] = acc + S.b3[c];
+		}
+		__syncthreads();
+		if (tid < kMlpRows && r0 + tid < n) {
+			float z[K], mx = -INFINITY, s = 0.0f;
+#pragma unroll
+			for (int k = 0; k < K; ++k) {
+				z[k] = S.x[tid][k];
+				mx   = fmaxf(mx, z[k]);
+			}
+#pragma unroll
+			for (int k = 0; k < K; ++k) {
+				z[k] = expf(z[k] - mx);
+				s += z[k];
+			}
+#pragma unroll
+			for (int k = 0; k < K; ++k) { P[(r0 + tid) * K + k] = z[k] / s; }
+		}
+		__syncthreads(); // x is read to the end before the next rows
+	}
+}
+
+// Softmax of every labelled row of Z (n x K): dZ = (P - onehot) / n and the mean loss added to *loss (and to
+// loss_hist[*step] when given).
+__global__ void k_softmax(const float* Z, uint64_t n, const int32_t* y, float* dZ, float* loss,
                           float* loss_hist, const uint32_t* step) {
 	float l = 0.0f;
 	for (uint64_t r = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; r < n;
@@ -1541,21 +1643,16 @@ __global__ void k_softmax(const float* Z, uint64_t n, float* P, const int32_t* y
 #pragma unroll
 		for (int k = 0; k < K; ++k) {
 			z[k] /= s;
-			if (P) { P[r * K + k] = z[k]; }
 		}
-		if (y) {
-			const int32_t t = y[r];
-			l -= logf(fmaxf(z[t], 1e-30f));
+		const int32_t t = y[r];
+		l -= logf(fmaxf(z[t], 1e-30f));
 #pragma unroll
-			for (int k = 0; k < K; ++k) { dZ[r * K + k] = (z[k] - (k == t ? 1.0f : 0.0f)) / static_cast<float>(n); }
-		}
+		for (int k = 0; k < K; ++k) { dZ[r * K + k] = (z[k] - (k == t ? 1.0f : 0.0f)) / static_cast<float>(n); }
 	}
-	if (y) {
-		l = warp_sum(l);
-		if ((threadIdx.x & 31u) == 0) {
-			if (loss) { atomicAdd(loss, l / static_cast<float>(n)); }
-			if (loss_hist) { atomicAdd(loss_hist + *step, l / static_cast<float>(n)); }
-		}
+	l = warp_sum(l);
+	if ((threadIdx.x & 31u) == 0) {
+		if (loss) { atomicAdd(loss, l / static_cast<float>(n)); }
+		if (loss_hist) { atomicAdd(loss_hist + *step, l / static_cast<float>(n)); }
 	}
 }
 
@@ -1701,6 +1798,22 @@ cudaError_t forward(cudaStream_t s, const float* params, const float* X, uint64_
 	if ((e = gemm(s, (int)n, H, NF, X, NF, 0, p.w1, H, 0, H1, H, p.b1, nullptr, EPI_BIAS | EPI_RELU)) != cudaSuccess) { return e; }
 	if ((e = gemm(s, (int)n, H, H, H1, H, 0, p.w2, H, 0, H2, H, p.b2, nullptr, EPI_BIAS | EPI_RELU)) != cudaSuccess) { return e; }
 	return gemm(s, (int)n, K, H, H2, H, 0, p.w3, K, 0, Z, K, p.b3, nullptr, EPI_BIAS);
+}
+
+// class probabilities of n rows
+cudaError_t probabilities(cudaStream_t s, const float* params, const float* X, uint64_t n, float* P) {
+	Device* d = current_device();
+	if (!d || d->ordinal < 0 || d->ordinal >= 64) { return cudaErrorInvalidDevice; }
+	static bool set[64] = {};
+	if (!set[d->ordinal]) {
+		const cudaError_t e = cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(MlpSmem));
+		if (e != cudaSuccess) { return e; }
+		set[d->ordinal] = true;
+	}
+	const uint64_t tiles = (n + kMlpRows - 1) / kMlpRows;
+	k_mlp<<<static_cast<unsigned>(std::min<uint64_t>(tiles, d->sm_count)), 256, sizeof(MlpSmem), s>>>(params, X, n, P);
+	++launch_counter();
+	return cudaGetLastError();
 }
 
 // backward from dZ (n x K): gradients into G (parameter layout); dH2 / dH1: n x H scratch
@@ -2198,22 +2311,17 @@ int fls_sel_learned(fls_sel_plan* p, const float* d_params, uint32_t stride, flo
 	int          rc  = sample_set(p, stride, &set);
 	if (rc != FLS_OK) { return rc; }
 	const uint64_t n = set->n;
-	if (!p->l_work.need(n * (NF + 2 * H + 2 * K) * 4) || !p->l_conf.need(p->n_chunks * 4)) { return FLS_ERR_CUDA; }
+	if (!p->l_work.need(n * (NF + K) * 4) || !p->l_conf.need(p->n_chunks * 4)) { return FLS_ERR_CUDA; }
 	Scratch& conf = p->l_conf;
 	float*   feat = p->l_work.as<float>();
-	float*   h1   = feat + n * NF;
-	float*   h2   = h1 + n * H;
-	float*   z    = h2 + n * H;
-	float*   prob = z + n * K;
+	float*   prob = feat + n * NF;
 	ItemArgs a {p->cols_d.as<Col>(), set->items.as<Item>(), n};
 	if (sample_features(p, a, feat, s) != cudaSuccess) { return FLS_ERR_CUDA; }
-	if (forward(s, d_params, feat, n, h1, h2, z) != cudaSuccess) { return FLS_ERR_CUDA; }
-	k_softmax<<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(z, n, prob, nullptr, nullptr,
-	                                                                                            nullptr, nullptr, nullptr);
+	if (probabilities(s, d_params, feat, n, prob) != cudaSuccess) { return FLS_ERR_CUDA; }
 	k_vote<<<static_cast<unsigned>((p->n_chunks + 7) / 8), 256, 0, s>>>(prob, set->chunk_items.as<uint32_t>(),
 	                                                                     static_cast<uint32_t>(p->n_chunks), d_choice,
 	                                                                     conf.as<float>(), p->str ? kStrK : K);
-	launch_counter() += 2;
+	++launch_counter();
 	if (cudaGetLastError() != cudaSuccess) { return FLS_ERR_CUDA; }
 	if (d_conf && cudaMemcpyAsync(d_conf, conf.m.p, p->n_chunks * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
 		return FLS_ERR_CUDA;
@@ -2254,15 +2362,7 @@ int fls_sel_mlp_forward(const float* d_params, const float* d_x, uint64_t n, flo
 	if (!d_params || ((!d_x || !d_prob) && n) || n >= (1ull << 31)) { return FLS_ERR_ARG; }
 	if (n == 0) { return FLS_OK; }
 	cudaStream_t s = static_cast<cudaStream_t>(stream);
-	DevMem       w;
-	if (!w.alloc(n * (2 * H + K) * 4)) { return FLS_ERR_CUDA; }
-	float* h1 = w.as<float>();
-	float* h2 = h1 + n * H;
-	float* z  = h2 + n * H;
-	if (forward(s, d_params, d_x, n, h1, h2, z) != cudaSuccess) { return FLS_ERR_CUDA; }
-	k_softmax<<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(z, n, d_prob, nullptr, nullptr,
-	                                                                                            nullptr, nullptr, nullptr);
-	++launch_counter();
+	if (probabilities(s, d_params, d_x, n, d_prob) != cudaSuccess) { return FLS_ERR_CUDA; }
 	return cudaStreamSynchronize(s) == cudaSuccess ? FLS_OK : FLS_ERR_CUDA;
 }
 
@@ -2280,7 +2380,7 @@ int fls_sel_mlp_grad(const float* d_params, const float* d_x, const int32_t* d_y
 	float* dh1 = dh2 + n * H;
 	if (cudaMemsetAsync(d_loss, 0, 4, s) != cudaSuccess) { return FLS_ERR_CUDA; }
 	if (forward(s, d_params, d_x, n, h1, h2, z) != cudaSuccess) { return FLS_ERR_CUDA; }
-	k_softmax<<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(z, n, nullptr, d_y, dz, d_loss,
+	k_softmax<<<static_cast<unsigned>(std::min<uint64_t>((n + 255) / 256, 4096)), 256, 0, s>>>(z, n, d_y, dz, d_loss,
 	                                                                                            nullptr, nullptr);
 	++launch_counter();
 	if (backward(s, d_params, d_x, n, h1, h2, dz, dh2, dh1, d_grad) != cudaSuccess) { return FLS_ERR_CUDA; }
@@ -2344,7 +2444,7 @@ int fls_sel_train(float* d_params, const float* d_x, const int32_t* d_y, const u
 	if (cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal) != cudaSuccess) { return FLS_ERR_CUDA; }
 	k_gather<<<64, 256, 0, s>>>(d_x, d_y, d_perm, st, batch, xb, yb);
 	forward(s, d_params, xb, B, h1, h2, z);
-	k_softmax<<<static_cast<unsigned>((B + 255) / 256), 256, 0, s>>>(z, B, nullptr, yb, dz, nullptr, d_loss_hist, st);
+	k_softmax<<<static_cast<unsigned>((B + 255) / 256), 256, 0, s>>>(z, B, yb, dz, nullptr, d_loss_hist, st);
 	backward(s, d_params, xb, B, h1, h2, dz, dh2, dh1, g);
 	k_adam<<<64, 256, 0, s>>>(d_params, g, m, v, P, lr, 0.9f, 0.999f, 1e-8f, 0, st);
 	k_step_inc<<<1, 1, 0, s>>>(st);

@@ -397,8 +397,8 @@ static int single_pass_decode(const fls_string_plan* p, uint32_t* d_offsets, uin
 	if (cudaMemsetAsync(p->lb.p, 0, 8ull * (1 + n_vec), s) != cudaSuccess) { return FLS_ERR_CUDA; }
 	StrSetArgs x {};
 	x.cols        = p->dargs.p;
-	x.chunk_w     = static_cast<uint32_t>(p->sp_warps);
-	x.n_chunks    = (n_vec + x.chunk_w - 1) / x.chunk_w;
+	x.n_cols      = 1;
+	x.n_items     = n_vec;
 	x.flags       = p->lb.p;
 	x.status      = p->args.status;
 	x.out_offsets = d_offsets;
@@ -458,10 +458,8 @@ int fls_string_plan_destroy(fls_string_plan* p) {
 struct fls_string_set {
 	std::vector<StrArgs> args;     // every column's arguments: item_base, and the outputs once bound
 	DevArr<StrArgs>      cols;     // the same in device memory
-	DevArr<uint32_t>     chunk_col, chunk_v0;
-	DevArr<uint64_t>     lb;       // ticket + one look-back word per vector of every column
+	DevArr<uint64_t>     lb;       // a ticket per column + one look-back word per vector of every column
 	uint64_t             n_items  = 0;
-	uint32_t             n_chunks = 0;
 	int                  warps    = 0;
 	uint32_t             smem = 0, dict_cap = 0, tab_cap = 0;
 	bool                 rows16 = true, bound = false;
@@ -498,23 +496,7 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 	}
 	set->warps = static_cast<int>(w < kStrMaxWarps ? w : kStrMaxWarps);
 	set->smem  = static_cast<uint32_t>(set->warps * pw + (set->dict_cap ? dict_max + tab : 0u));
-	// chunks of `warps` vectors that never cross a column, in column order
-	std::vector<uint32_t> cc, cv;
-	for (uint32_t i = 0; i < n; ++i) {
-		for (uint32_t v = 0; v < set->args[i].col.n_vec; v += static_cast<uint32_t>(set->warps)) {
-			cc.push_back(i);
-			cv.push_back(v);
-		}
-	}
-	set->n_chunks = static_cast<uint32_t>(cc.size());
-	if (!set->cols.alloc(n) || !set->lb.alloc(1 + set->n_items) || !set->chunk_col.alloc(cc.size()) ||
-	    !set->chunk_v0.alloc(cv.size())) {
-		return FLS_ERR_CUDA;
-	}
-	if (!cc.empty() && (cudaMemcpy(set->chunk_col.p, cc.data(), 4 * cc.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-	                    cudaMemcpy(set->chunk_v0.p, cv.data(), 4 * cv.size(), cudaMemcpyHostToDevice) != cudaSuccess)) {
-		return FLS_ERR_CUDA;
-	}
+	if (!set->cols.alloc(n) || !set->lb.alloc(n + set->n_items)) { return FLS_ERR_CUDA; }
 	*out = set.release();
 	return FLS_OK;
 }
@@ -542,13 +524,11 @@ int fls_string_set_bind(fls_string_set* set, uint32_t* const* d_offsets, uint8_t
 int fls_string_set_decode(const fls_string_set* set, fls_stream_t stream) {
 	if (!set || !set->bound) { return FLS_ERR_ARG; }
 	cudaStream_t s = static_cast<cudaStream_t>(stream);
-	if (cudaMemsetAsync(set->lb.p, 0, 8ull * (1 + set->n_items), s) != cudaSuccess) { return FLS_ERR_CUDA; }
+	if (cudaMemsetAsync(set->lb.p, 0, 8ull * (set->args.size() + set->n_items), s) != cudaSuccess) { return FLS_ERR_CUDA; }
 	StrSetArgs x {};
 	x.cols      = set->cols.p;
-	x.chunk_col = set->chunk_col.p;
-	x.chunk_v0  = set->chunk_v0.p;
-	x.n_chunks  = set->n_chunks;
-	x.chunk_w   = static_cast<uint32_t>(set->warps);
+	x.n_cols    = static_cast<uint32_t>(set->args.size());
+	x.n_items   = set->n_items;
 	x.flags     = set->lb.p;
 	x.status    = set->status;
 	x.dict_cap  = set->dict_cap;

@@ -806,8 +806,8 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 
 // Single-pass FSST / BYTE_ARR decode (no lengths pass, no scan).  A warp takes vectors by ticket (lb[0]), in
 // vector order, so every vector it waits for was taken by a running warp that publishes without waiting.  Per
-// vector: its rows; its decoded total -- the sum of its codes' symbol lengths when no escape is among its bytes,
-// else the escape-aware walk of stream_vector (a BYTE_ARR vector's total is its compressed length) -- published
+// vector: its rows; its decoded total -- the sum of its codes' symbol lengths when its escapes, if any, stand alone,
+// else the general walk of stream_vector (a BYTE_ARR vector's total is its compressed length) -- published
 // in its look-back word lb[1 + v]; its first output byte from the earlier vectors' words (lookback); then its
 // offsets and bytes (stream_vector), whose total must match.
 template <int KIND>
@@ -848,12 +848,14 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_stream_single(const StrAr
 		const bool ok  = p.ok;
 		bool       bad = false;
 		if (!ok && lane == 0) { atomicOr(a.status, p.bw > p.ws ? STATUS_BAD_BW : STATUS_BAD_LAYOUT); }
-		uint32_t T = 0;
+		uint32_t T    = 0;
+		bool     lone = false; // its escapes stand alone
 		if (ok) {
 			load_rows<false>(p, buf, lane, a.status);
 			const uint32_t L = stream_rows_length(rows32, vn, lane, &bad);
 			T                = L;
-			if (kFsst && !fsst_plain_total(vb, L, flen, lane, &T)) {
+			lone             = kFsst && fsst_total<true>(rows32, vb, L, flen, lane, &T);
+			if (kFsst && !lone) {
 				StreamOut o {};
 				T = stream_vector<false, true, kStrWindow>(rows32, vb, vn, fsym, flen, lane, o, &bad);
 			}
@@ -869,7 +871,7 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_stream_single(const StrAr
 			for (uint32_t r = lane; r < kVec; r += 32) { offs[r] = static_cast<uint32_t>(P); }
 		} else {
 			StreamOut o {offs, a.bytes, P, win};
-			const uint32_t got = stream_vector<true, kFsst, kStrWindow>(rows32, vb, vn, fsym, flen, lane, o, &bad);
+			const uint32_t got = stream_vector<true, kFsst, kStrWindow>(rows32, vb, vn, fsym, flen, lane, o, &bad, lone);
 			if (got != T) { bad = true; }
 		}
 		if (lane == 0 && v + 1 == n) { a.offsets[n * kVec] = static_cast<uint32_t>(P + T); }

@@ -224,8 +224,8 @@ __device__ __forceinline__ T warp_sum(T x) {
 //     function of its 4 bytes (state 1 = "the next byte is a literal"), a warp scan of the functions gives every
 //     lane its entry state.  Chunks without a 255 (nearly all of them) skip this: every byte starts a code.
 //   * decoded lengths (symbol length; 1 for an escape; 0 for its literal) are prefix-summed across the warp;
-//   * every lane writes its symbols at its offset into the warp's output window as whole words
-//     (put_syms: the put_row protocol), and rows starting in the chunk take their offsets from the sums.
+//   * every lane ORs its symbols at its offset into the warp's zeroed output window (or_symbol), and rows starting in
+//     the chunk take their offsets from the sums.
 // An escape as a row's last byte decodes as one zero byte (as the oracle's row decoder does).
 // ---------------------------------------------------------------------------------------------------------
 constexpr uint32_t kStreamChunk = 128; // stream bytes per warp step
@@ -280,65 +280,17 @@ __device__ __forceinline__ void stream_row_mask(const uint32_t* rows32, uint32_t
 	*rc = r;
 }
 
-// A lane's decoded bytes -- up to 4 symbols (value, length; length 0 = nothing, its value then 0) in order --
-// into the word window at byte d, whole words: every word is stored by the lane owning its first byte, bytes
-// past the lane's end zero; a lane starting inside a word returns its bytes of that word (*hk, *head) for an
-// atomic OR after a warp sync (the protocol of put_row).  Returns whether such a head is left.
-// The bytes gather in a 128-bit accumulator a0..a3 (word k at a0) holding nb < 64 bits before every symbol, so
-// a symbol (at most 64 bits) leaves at most one pair of whole words behind it: one predicated two-word emit
-// per symbol, and no branch on where a word goes.
-__device__ __forceinline__ bool put_syms(uint32_t* win, uint32_t d, const uint64_t (&sv)[4], const uint32_t (&sl)[4],
-                                         uint32_t* hk, uint32_t* head) {
-	const uint32_t k0  = d >> 2;
-	const bool     mid = (d & 3u) != 0;
-	uint32_t       k   = k0;
-	uint32_t       nb  = 8u * (d & 3u);
-	uint32_t       a0 = 0, a1 = 0, a2 = 0, a3 = 0;
-	uint32_t       hv   = 0;
-	bool           held = false;
-	// words k, k + 1 leave: the first word of a lane that starts inside it is its head instead
-	auto emit2 = [&]() {
-		const bool h = mid && k == k0;
-		if (!h) { win[k] = a0; }
-		win[k + 1] = a1;
-		hv         = h ? a0 : hv;
-		held       = held || h;
-	};
-#pragma unroll
-	for (int j = 0; j < 4; ++j) {
-		const uint32_t lo = static_cast<uint32_t>(sv[j]), hi = static_cast<uint32_t>(sv[j] >> 32);
-		const uint32_t sh = nb & 31u;
-		const uint32_t t0 = lo << sh;
-		const uint32_t t1 = __funnelshift_l(lo, hi, sh);
-		const uint32_t t2 = __funnelshift_l(hi, 0u, sh); // hi >> (32 - sh), 0 for sh = 0
-		const bool     lw = nb < 32u;
-		a0 |= lw ? t0 : 0u;
-		a1 |= lw ? t1 : t0;
-		a2 |= lw ? t2 : t1;
-		a3 |= lw ? 0u : t2;
-		nb += 8u * sl[j];
-		if (nb >= 64u) {
-			emit2();
-			a0 = a2;
-			a1 = a3;
-			a2 = 0;
-			a3 = 0;
-			k += 2;
-			nb -= 64u;
-		}
-	}
-	// what is left: bits [0, nb) of a0, a1 (nb > 8 * (d & 3) when the lane wrote nothing yet and has bytes)
-	const bool any = (sl[0] | sl[1] | sl[2] | sl[3]) != 0;
-	if (any && nb > 0u) {
-		const bool h = mid && k == k0;
-		if (!h) { win[k] = a0; }
-		hv   = h ? a0 : hv;
-		held = held || h;
-		if (nb > 32u) { win[k + 1] = a1; }
-	}
-	*hk   = k0;
-	*head = hv;
-	return held;
+// A symbol's l bytes (0: none; value zero past them) into the word window at byte d: its up to three words are OR-ed in,
+// the window being zero past what is written, so that neither the lane nor its neighbours have to know whose bytes
+// share a word.  (Gathering a lane's symbols into whole words first took 28 instructions a symbol, this takes 13.)
+__device__ __forceinline__ void or_symbol(uint32_t* win, uint32_t d, uint64_t value, uint32_t l) {
+	if (l == 0) { return; }
+	const uint32_t lo = static_cast<uint32_t>(value), hi = static_cast<uint32_t>(value >> 32);
+	const uint32_t at = d & 3u, s = 8u * at;
+	uint32_t*      w  = win + (d >> 2);
+	atomicOr(w, lo << s);
+	if (at + l > 4) { atomicOr(w + 1, __funnelshift_l(lo, hi, s)); }
+	if (at + l > 8) { atomicOr(w + 2, __funnelshift_l(hi, 0u, s)); }
 }
 
 // Compressed length of a vector's rows (rows32: its 1024 cumulative row end offsets, row r at word r + r / 32;
@@ -358,12 +310,16 @@ __device__ __forceinline__ uint32_t stream_rows_length(const uint32_t* rows32, u
 	return *bad ? 0u : rows32[kVec - 1 + (kVec - 1) / 32];
 }
 
-// Decoded byte total of an FSST vector's compressed bytes [0, L) when none of them is an escape (255): every
-// byte is then a code and the total is the sum of their symbol lengths (len: the symbol lengths, code 255's 0).
-// Returns false when a byte 255 may be among them -- the escape-aware walk (stream_vector) decides then; the
+// Decoded byte total of an FSST vector's compressed bytes [0, L): the sum of its bytes' symbol lengths (len: code 255's
+// 0), when no byte is an escape.  ROWS: escapes are allowed where no row (rows32, non-decreasing) ends inside a run of
+// bytes 255 or between the run and the literal of its last escape.  Such a run starts with an escape whatever came
+// before it, its bytes are escapes and literals in turn, every escape decodes to one byte, and after a run of odd length
+// the next byte is a literal and no code.
+// Returns false when the bytes are not of that kind -- the general walk (stream_vector) decides then; without ROWS the
 // zero-byte test can also fire on a byte 254 just above a 255 outside the range, which costs only that walk.
-__device__ __forceinline__ bool fsst_plain_total(const uint8_t* vb, uint32_t L, const uint8_t* len, uint32_t lane,
-                                                 uint32_t* total) {
+template <bool ROWS>
+__device__ __forceinline__ bool fsst_total(const uint32_t* rows32, const uint8_t* vb, uint32_t L, const uint8_t* len,
+                                           uint32_t lane, uint32_t* total) {
 	const uintptr_t va   = reinterpret_cast<uintptr_t>(vb);
 	const uint32_t  off  = static_cast<uint32_t>(va & 3u);
 	const uint32_t* base = reinterpret_cast<const uint32_t*>(va - off);
@@ -372,7 +328,7 @@ __device__ __forceinline__ bool fsst_plain_total(const uint8_t* vb, uint32_t L, 
 	// 8 words per lane in flight per round: the walk is one read of the bytes, bound by load latency otherwise
 	constexpr uint32_t kU = 8;
 	for (uint32_t q0 = lane; q0 < nw; q0 += 32 * kU) {
-		uint32_t w[kU];
+		uint32_t w[kU], some = 0; // words with an escape
 #pragma unroll
 		for (uint32_t u = 0; u < kU; ++u) { w[u] = q0 + 32 * u < nw ? __ldg(base + q0 + 32 * u) : 0u; }
 #pragma unroll
@@ -394,11 +350,53 @@ __device__ __forceinline__ bool fsst_plain_total(const uint8_t* vb, uint32_t L, 
 				}
 			}
 			const uint32_t x = ~w[u]; // escape bytes turn into zero bytes
-			esc |= (x - 0x01010101u) & ~x & vm;
+			const uint32_t f = (x - 0x01010101u) & ~x & vm;
+			if constexpr (ROWS) {
+				some |= f ? 1u << u : 0u;
+			} else {
+				esc |= f;
+			}
+		}
+		if constexpr (ROWS) {
+			while (some) {
+				const uint32_t u = static_cast<uint32_t>(__ffsll(static_cast<long long>(some))) - 1;
+				some &= some - 1;
+				for (uint32_t j = 0; j < 4; ++j) {
+					const int64_t p = 4ll * (q0 + 32 * u) - off + j; // a run's first byte
+					if (p < 0 || p >= static_cast<int64_t>(L) || __ldg(vb + p) != 255u || (p > 0 && __ldg(vb + p - 1) == 255u)) { continue; }
+					const uint32_t at = static_cast<uint32_t>(p);
+					uint32_t       k  = 1;
+					while (k < 64 && at + k < L && __ldg(vb + at + k) == 255u) { ++k; }
+					const uint32_t past = at + k + (k & 1u); // the byte after the run and its last literal
+					if (k == 64 || past > L) {
+						esc = 1;
+						continue;
+					}
+					sum += (k + 1) / 2;
+					if (k & 1u) { sum -= len[__ldg(vb + at + k)]; }
+					uint32_t lo = 0, n = kVec; // the first row end past the run's first byte
+					while (n > 0) {
+						const uint32_t h = n / 2, r = lo + h;
+						if (rows32[r + (r >> 5)] <= at) {
+							lo = r + 1;
+							n -= h + 1;
+						} else {
+							n = h;
+						}
+					}
+					esc |= lo < kVec && rows32[lo + (lo >> 5)] < past ? 1u : 0u;
+				}
+			}
 		}
 	}
 	*total = warp_sum(sum);
 	return !__any_sync(0xFFFFFFFFu, esc != 0);
+}
+
+// The total of a vector without escapes.
+__device__ __forceinline__ bool fsst_plain_total(const uint8_t* vb, uint32_t L, const uint8_t* len, uint32_t lane,
+                                                 uint32_t* total) {
+	return fsst_total<false>(nullptr, vb, L, len, lane, total);
 }
 
 // Per-vector output of the materialising pass.
@@ -412,11 +410,13 @@ struct StreamOut {
 // One vector of an FSST (KIND_FSST = true) or BYTE_ARR column: rows32 its 1024 cumulative row end offsets in
 // original order (row r at word r + r / 32), vb / vn its compressed bytes (vn 0 and rows all zero for none).
 // Returns the decoded byte total; MAT also writes the offsets and bytes (o).  *bad: the rows are not
-// non-decreasing within vn (the vector then decodes as 1024 empty rows).
+// non-decreasing within vn (the vector then decodes as 1024 empty rows).  lone: no row ends inside
+// the vector's escapes (fsst_total<true> said so), so that a byte's part follows from the bytes 255 right before it and
+// the state entering a lane from the lane before, without row starts and a scan.
 template <bool MAT, bool KIND_FSST, uint32_t kWindow>
 __device__ __forceinline__ uint32_t stream_vector(const uint32_t* rows32, const uint8_t* vb, uint32_t vn,
                                                   const uint64_t* sym, const uint8_t* len, uint32_t lane,
-                                                  const StreamOut& o, bool* bad) {
+                                                  const StreamOut& o, bool* bad, bool lone = false) {
 	const uint32_t  L     = stream_rows_length(rows32, vn, lane, bad);
 	if constexpr (!KIND_FSST && !MAT) { return L; } // a plain-bytes vector decodes to its own bytes
 	const uintptr_t va    = reinterpret_cast<uintptr_t>(vb);
@@ -434,8 +434,8 @@ __device__ __forceinline__ uint32_t stream_vector(const uint32_t* rows32, const 
 	uint32_t fill = static_cast<uint32_t>(o.vbase & 15u);
 	uint64_t lo   = o.vbase;
 	if constexpr (MAT) {
-		// the first lane may start inside this word: it ORs its bytes in
-		if (lane == 0) { win32[fill >> 2] = 0; }
+#pragma unroll
+		for (uint32_t c = 16 * lane; c < kWindow; c += 512) { *reinterpret_cast<uint4*>(o.win + c) = make_uint4(0, 0, 0, 0); }
 		__syncwarp();
 	}
 	auto flush = [&](bool all) {
@@ -443,20 +443,22 @@ __device__ __forceinline__ uint32_t stream_vector(const uint32_t* rows32, const 
 		const uint32_t upto = all ? fill : full;
 		for (uint32_t c = 16 * lane; c < upto; c += 512) {
 			const uint64_t g = W + c;
+			const uint4    x = *reinterpret_cast<const uint4*>(o.win + c);
 			if (g >= lo && c + 16 <= upto) {
-				*reinterpret_cast<uint4*>(o.bytes + g) = *reinterpret_cast<const uint4*>(o.win + c);
+				*reinterpret_cast<uint4*>(o.bytes + g) = x;
 			} else {
 				for (uint32_t i = 0; i < 16 && c + i < upto; ++i) {
 					if (g + i >= lo) { o.bytes[g + i] = o.win[c + i]; }
 				}
 			}
+			*reinterpret_cast<uint4*>(o.win + c) = make_uint4(0, 0, 0, 0);
 		}
 		__syncwarp();
 		if (!all) {
-			// the partial chunk [full, fill) moves to the window start (its bytes past `fill` are zero: every word
-			// was stored whole, zeros past its writer's end)
+			// the partial chunk [full, fill) moves to the window start
 			if (lane == 0 && full != 0 && (fill & 15u) != 0) {
-				*reinterpret_cast<uint4*>(o.win) = *reinterpret_cast<const uint4*>(o.win + full);
+				*reinterpret_cast<uint4*>(o.win)        = *reinterpret_cast<const uint4*>(o.win + full);
+				*reinterpret_cast<uint4*>(o.win + full) = make_uint4(0, 0, 0, 0);
 			}
 			__syncwarp();
 			W += full;
@@ -480,32 +482,53 @@ __device__ __forceinline__ uint32_t stream_vector(const uint32_t* rows32, const 
 		q1 = q2;
 		q2 = q3;
 		q3 = ldw(ck + 4);
-		const uint32_t b4    = off ? __funnelshift_r(w0, w1, 8u * off) : w0; // stream bytes cb+4l .. +3
-		const uint32_t bnext = (w1 >> (8u * off)) & 0xFFu;                   // stream byte cb+4l+4
-		const uint32_t pos0  = cb + 4 * lane;
-		const uint32_t nv    = pos0 >= L ? 0u : (L - pos0 < 4u ? L - pos0 : 4u);
+		uint32_t       b4   = __funnelshift_r(w0, w1, 8u * off); // stream bytes cb+4l .. +3
+		const uint32_t pos0 = cb + 4 * lane;
+		uint32_t       nv   = 4;
+		uint32_t       vm   = 0x80808080u; // the top bit of every byte inside the stream
+		if (cb + kStreamChunk > L) { // the last chunk
+			nv = pos0 >= L ? 0u : (L - pos0 < 4u ? L - pos0 : 4u);
+			vm = nv == 0 ? 0u : vm >> (8 * (4 - nv));
+			b4 |= nv >= 4 ? 0u : 0xFFFFFFFFu << (8 * nv); // bytes past the end read as code 255, whose entry is empty
+		}
 		uint64_t       sv[4];
 		uint32_t       sl[4];
 		if constexpr (!KIND_FSST) {
+			// plain bytes: a lane's are one symbol
+			sv[0] = nv >= 4 ? b4 : b4 & ~(0xFFFFFFFFu << (8 * nv));
+			sl[0] = nv;
 #pragma unroll
-			for (uint32_t j = 0; j < 4; ++j) {
-				sv[j] = j < nv ? (b4 >> (8 * j)) & 0xFFu : 0u;
-				sl[j] = j < nv ? 1u : 0u;
-			}
+			for (uint32_t j = 1; j < 4; ++j) { sv[j] = sl[j] = 0; }
 		} else {
-			uint32_t esc = 0;
-#pragma unroll
-			for (uint32_t j = 0; j < 4; ++j) { esc |= (j < nv && ((b4 >> (8 * j)) & 0xFFu) == 255u) ? 1u << j : 0u; }
-			if (!__any_sync(0xFFFFFFFFu, esc != 0 || carry != 0)) {
+			const uint32_t inv = ~b4; // a byte 255 turns into a zero byte
+			if (!__any_sync(0xFFFFFFFFu, ((inv - 0x01010101u) & ~inv & vm) != 0 || carry != 0)) {
 				// no escape anywhere in the chunk: every byte starts a code
 #pragma unroll
 				for (uint32_t j = 0; j < 4; ++j) {
-					// a byte past the stream's end reads as code 255, whose table entry is empty (symbol 0, length 0)
-					const uint32_t c = j < nv ? (b4 >> (8 * j)) & 0xFFu : 255u;
+					const uint32_t c = (b4 >> (8 * j)) & 0xFFu;
 					sv[j]            = sym[c];
 					sl[j]            = len[c];
 				}
+			} else if (lone && !__any_sync(0xFFFFFFFFu, inv == 0 && nv == 4)) { // (a lane of nothing but 255s: the general way)
+				const uint32_t bnext = (w1 >> (8u * off)) & 0xFFu; // stream byte cb+4l+4
+				// 255s at the lane's end, after a byte that is none: an odd number leaves a literal to the next lane
+				const uint32_t odd = (static_cast<uint32_t>(__clzll(static_cast<long long>(inv)) - 32) >> 3) & 1u;
+				uint32_t       st  = __shfl_up_sync(0xFFFFFFFFu, odd, 1);
+				if (lane == 0) { st = carry; }
+				carry = __shfl_sync(0xFFFFFFFFu, odd, 31); // (past the stream's end it does not matter)
+#pragma unroll
+				for (uint32_t j = 0; j < 4; ++j) {
+					const uint32_t c    = (b4 >> (8 * j)) & 0xFFu;
+					const bool     mark = !st && c == 255u && j < nv;
+					sv[j]               = mark ? (j < 3 ? (b4 >> (8 * (j + 1))) & 0xFFu : bnext) : st ? 0u : sym[c];
+					sl[j]               = mark ? 1u : st ? 0u : len[c];
+					st                  = mark ? 1u : 0u;
+				}
 			} else {
+				uint32_t esc = 0;
+#pragma unroll
+				for (uint32_t j = 0; j < 4; ++j) { esc |= (j < nv && ((b4 >> (8 * j)) & 0xFFu) == 255u) ? 1u << j : 0u; }
+				const uint32_t bnext = (w1 >> (8u * off)) & 0xFFu; // stream byte cb+4l+4
 				uint32_t m[4];
 				bool     at_end;
 				uint32_t r = rc;
@@ -564,26 +587,35 @@ __device__ __forceinline__ uint32_t stream_vector(const uint32_t* rows32, const 
 		const uint32_t X   = inc - e;
 		const uint32_t T   = __shfl_sync(0xFFFFFFFFu, inc, 31);
 		if constexpr (MAT) {
-			// offsets of the rows starting in this chunk (before cb + 128): from the owner lane of their first byte
-			const uint32_t part = sl[0] | ((sl[0] + sl[1]) << 8) | ((sl[0] + sl[1] + sl[2]) << 16);
+			// offsets of the rows starting in this chunk (before cb + 128): from the owner lane of their first byte, whose
+			// bytes j = 0..3 decode from X + byte j of part on
+			uint32_t part;
+			if constexpr (KIND_FSST) {
+				part = (sl[0] << 8) | ((sl[0] + sl[1]) << 16) | ((sl[0] + sl[1] + sl[2]) << 24);
+			} else {
+				part = 0x03020100u;
+			}
+			const uint32_t at = static_cast<uint32_t>(o.vbase) + vdec;
 			while (rc < kVec) {
 				const uint32_t rr  = rc + lane;
 				const uint32_t s   = rr < kVec ? stream_row_start(rows32, rr) : 0xFFFFFFFFu;
 				const bool     in  = s < cb + kStreamChunk;
 				const uint32_t rel = s - cb;
-				const uint32_t own = (rel >> 2) & 31u, sub = rel & 3u;
+				const uint32_t own = (rel >> 2) & 31u;
 				const uint32_t xo  = __shfl_sync(0xFFFFFFFFu, X, own);
 				const uint32_t po  = __shfl_sync(0xFFFFFFFFu, part, own);
-				if (in) { o.offsets[rr] = static_cast<uint32_t>(o.vbase + vdec + xo + (sub ? (po >> (8 * (sub - 1))) & 0xFFu : 0u)); }
+				if (in) { o.offsets[rr] = at + xo + ((po >> (8 * (rel & 3u))) & 0xFFu); }
 				const uint32_t n = __popc(__ballot_sync(0xFFFFFFFFu, in));
 				rc += n;
 				if (n < 32) { break; }
 			}
 			if (fill + T > kWindow) { flush(false); }
-			uint32_t hk = 0, head = 0;
-			const bool mid = put_syms(win32, fill + X, sv, sl, &hk, &head);
-			__syncwarp(); // every word's whole store lands before the lanes that start inside it OR in
-			if (mid) { atomicOr(win32 + hk, head); }
+			uint32_t d = fill + X;
+#pragma unroll
+			for (uint32_t j = 0; j < (KIND_FSST ? 4 : 1); ++j) {
+				or_symbol(win32, d, sv[j], sl[j]);
+				d += sl[j];
+			}
 			__syncwarp();
 			fill += T;
 		}

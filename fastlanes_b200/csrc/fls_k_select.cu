@@ -1246,10 +1246,13 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 						} else if (idle == 0xFFFFFFFFu) {
 							break;
 						}
-						if (have && left) {
-							const uint32_t step = str_next_code(S, load8(p, inside), left, &cl);
-							p += step;
-							left -= step;
+						// four codes between two looks at who is idle
+						for (uint32_t k = 0; k < 4; ++k) {
+							if (have && left) {
+								const uint32_t step = str_next_code(S, load8(p, inside), left, &cl);
+								p += step;
+								left -= step;
+							}
 						}
 						if (have && left == 0) {
 							c.clen[r0 + j] = cl;

@@ -148,6 +148,8 @@ struct fls_string_plan {
 	DevArr<uint32_t>         dict_ends;
 	DevArr<uint32_t>         dict_rows; // packed start | length << 24 of every entry, when they fit
 	DevArr<uint8_t>          dict_bytes;
+	DevArr<uint8_t>          dict8; // single-pass DICT decode: the dictionary's entries on 8-byte boundaries
+	DevArr<uint32_t>         rows8;
 	DevArr<uint64_t>         vec_total;
 	DevArr<uint64_t>         vec_base;
 	DevArr<uint32_t>         codes; // patched DICT pages: their decoded code stream
@@ -299,6 +301,24 @@ int fls_string_plan_create(const uint8_t* d_page, uint64_t page_size, const uint
 						return FLS_ERR_CUDA;
 					}
 					a.dict_rows = p->dict_rows.p;
+					// the same entries on 8-byte boundaries, for the single-pass decode
+					std::vector<uint32_t> rows8(entry_c);
+					uint64_t              at = 0;
+					for (uint32_t c = 0; c < entry_c; ++c) {
+						const uint32_t n = ends[c] >> 24;
+						rows8[c]         = static_cast<uint32_t>(at / 8) | (n << 24);
+						at += (n + 7) & ~7u;
+					}
+					a.dict8_n = (at + 15) & ~15ull;
+					if (!p->rows8.alloc(entry_c) || !p->dict8.alloc(a.dict8_n + 16) ||
+					    cudaMemcpy(p->rows8.p, rows8.data(), 4ull * entry_c, cudaMemcpyHostToDevice) != cudaSuccess ||
+					    cudaMemset(p->dict8.p, 0, a.dict8_n + 16) != cudaSuccess ||
+					    launch_dict_align(p->dict_bytes.p, p->dict_rows.p, p->rows8.p, entry_c, p->dict8.p, nullptr) != cudaSuccess ||
+					    cudaStreamSynchronize(nullptr) != cudaSuccess) { // decodes may run on any stream
+						return FLS_ERR_CUDA;
+					}
+					a.rows8 = p->rows8.p;
+					a.dict8 = p->dict8.p;
 				}
 			}
 			a.entry_c      = entry_c;
@@ -339,15 +359,15 @@ int fls_string_plan_create(const uint8_t* d_page, uint64_t page_size, const uint
 		p->single            = true;
 		const uint32_t   pw  = dict_pass_smem_per_warp(a.rows16);
 		const uint64_t   tab = (4ull * a.entry_c + 15) & ~15ull;
-		const uint64_t   all = 224 * 1024;
+		const uint64_t   all = 224 * 1024, d8 = a.dict8_n;
 		uint64_t         sw  = all / pw;
-		if (dict_sm + tab < all && (all - dict_sm - tab) / pw >= 8) {
-			p->sp_dict_cap = static_cast<uint32_t>(dict_sm);
+		if (d8 + tab < all && (all - d8 - tab) / pw >= 8) {
+			p->sp_dict_cap = static_cast<uint32_t>(d8);
 			p->sp_tab_cap  = a.entry_c;
-			sw             = (all - dict_sm - tab) / pw;
+			sw             = (all - d8 - tab) / pw;
 		}
 		p->sp_warps = static_cast<int>(sw < kStrMaxWarps ? sw : kStrMaxWarps);
-		p->sp_smem  = static_cast<uint32_t>(p->sp_warps * pw + (p->sp_dict_cap ? dict_sm + tab : 0u));
+		p->sp_smem  = static_cast<uint32_t>(p->sp_warps * pw + (p->sp_dict_cap ? d8 + tab : 0u));
 		if (!p->dargs.alloc(1) || !p->lb.alloc(1ull + pi.vec_c) ||
 		    cudaMemcpy(p->dargs.p, &a, sizeof(StrArgs), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return FLS_ERR_CUDA;
@@ -481,7 +501,7 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 		set->args.push_back(a);
 		set->n_items += a.col.n_vec;
 		set->rows16 = set->rows16 && a.rows16;
-		dict_max    = std::max<uint64_t>(dict_max, (a.dict_bytes_n + 15) & ~15ull);
+		dict_max    = std::max<uint64_t>(dict_max, a.dict8_n);
 		tab_max     = std::max<uint64_t>(tab_max, a.entry_c);
 		set->status = a.status;
 	}

@@ -84,6 +84,18 @@ __global__ void __launch_bounds__(1024) k_fsst_dict(const uint8_t* lens, const u
 // ---------------------------------------------------------------------------------------------------------
 // Per-vector building blocks
 // ---------------------------------------------------------------------------------------------------------
+// A thread an 8-byte piece of an entry (at most 32).
+__global__ void k_dict_align(const uint8_t* bytes, const uint32_t* rows, const uint32_t* rows8, uint32_t entry_c,
+                             uint8_t* bytes8) {
+	const uint32_t c = blockIdx.x * (blockDim.x / 32) + threadIdx.x / 32, i = 8 * (threadIdx.x & 31u);
+	if (c >= entry_c) { return; }
+	const uint32_t start = rows[c] & 0xFFFFFFu, n = rows[c] >> 24;
+	if (i >= n) { return; }
+	uint64_t x = 0;
+	for (uint32_t b = 0; b < 8 && i + b < n; ++b) { x |= static_cast<uint64_t>(bytes[start + i + b]) << (8 * b); }
+	*reinterpret_cast<uint64_t*>(bytes8 + 8ull * (rows8[c] & 0xFFFFFFu) + i) = x;
+}
+
 __device__ __forceinline__ uint32_t dict_start(const uint32_t* ends, uint32_t code) {
 	return code == 0 ? 0u : ends[code - 1];
 }
@@ -612,11 +624,11 @@ __device__ __forceinline__ uint64_t lookback(const uint64_t* words, uint32_t v, 
 
 // Rows of one DICT vector into Arrow offsets and bytes from the first output byte vbase: 32 rows at a time (a
 // row per lane, positions by a warp scan) into the warp's output window (put_row), which leaves in 16-byte
-// stores.  tab: the packed row table (start | length << 24) of the dictionary's entry_c entries.  Returns the
+// stores.  tab: the row table ((start / 8) | length << 24) of the dictionary's entry_c entries.  Returns the
 // bytes written; *bad for codes outside the dictionary (such rows are empty).
 template <bool R16>
 __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const uint32_t* tab, uint32_t entry_c,
-                                                    const uint8_t* dict, uint8_t* win, uint32_t* offs, uint8_t* bytes,
+                                                    const uint2* dict, uint8_t* win, uint32_t* offs, uint8_t* bytes,
                                                     uint64_t vbase, uint32_t lane, bool* bad) {
 	uint32_t* win32 = reinterpret_cast<uint32_t*>(win);
 	uint64_t  W     = vbase & ~15ull; // output position of win[0]
@@ -672,7 +684,7 @@ __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const u
 		if (fill + T > kStrWindow) { flush(false); }
 		if (fill + T <= kStrWindow) {
 			uint32_t   hk = 0, head = 0;
-			const bool mid = put_row(win32, fill + (o - vpos), reinterpret_cast<const uint32_t*>(dict), fs, fl, &hk, &head);
+			const bool mid = put_row8(win32, fill + (o - vpos), dict + fs, fl, &hk, &head);
 			__syncwarp(); // every word's whole store lands before the rows that start inside it OR in
 			if (mid) { atomicOr(win32 + hk, head); }
 			fill += T;
@@ -680,7 +692,7 @@ __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const u
 			// a batch larger than the window: straight to global memory after the window's pending bytes
 			flush(true);
 			uint8_t* dst = bytes + vbase + o;
-			for (uint32_t i = 0; i < fl; ++i) { dst[i] = dict[fs + i]; }
+			for (uint32_t i = 0; i < fl; ++i) { dst[i] = reinterpret_cast<const uint8_t*>(dict + fs)[i]; }
 			const uint64_t pos = vbase + vpos + T;
 			W                  = pos & ~15ull;
 			fill               = static_cast<uint32_t>(pos & 15u);
@@ -745,11 +757,11 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 		const StrArgs& A     = s.cols[col];
 		const uint32_t n_vec = A.col.n_vec;
 		if constexpr (SMDICT) {
-			// the column's decoded dictionary (cudaMalloc'd, 16 bytes of slack) and row table
-			const uint32_t nb16 = static_cast<uint32_t>((A.dict_bytes_n + 15) / 16);
-			const uint4*   src  = reinterpret_cast<const uint4*>(A.dict_bytes);
+			// the column's aligned dictionary (cudaMalloc'd, a multiple of 16 bytes) and row table
+			const uint32_t nb16 = static_cast<uint32_t>((A.dict8_n + 15) / 16);
+			const uint4*   src  = reinterpret_cast<const uint4*>(A.dict8);
 			for (uint32_t i = threadIdx.x; i < nb16; i += blockDim.x) { reinterpret_cast<uint4*>(sdict)[i] = __ldg(src + i); }
-			for (uint32_t i = threadIdx.x; i < A.entry_c; i += blockDim.x) { stab[i] = __ldg(A.dict_rows + i); }
+			for (uint32_t i = threadIdx.x; i < A.entry_c; i += blockDim.x) { stab[i] = __ldg(A.rows8 + i); }
 			__syncthreads();
 		}
 		while (warp < s.active) {
@@ -758,8 +770,8 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 			ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
 			if (ticket >= n_vec) { break; }
 			const uint32_t  v       = static_cast<uint32_t>(ticket);
-			const uint8_t*  dict    = SMDICT ? sdict : A.dict_bytes;
-			const uint32_t* tab     = SMDICT ? stab : A.dict_rows;
+			const uint2*    dict    = reinterpret_cast<const uint2*>(SMDICT ? sdict : A.dict8);
+			const uint32_t* tab     = SMDICT ? stab : A.rows8;
 			const uint32_t  entry_c = A.entry_c;
 			uint64_t*       words   = s.flags + s.n_cols + A.item_base;
 			const Plan      p       = make_plan(A.col, v);
@@ -904,6 +916,14 @@ cudaError_t launch_fsst_dict(const uint8_t* lens, const uint8_t* comp, uint64_t 
                              cudaStream_t s) {
 	if (entry_c == 0) { return cudaSuccess; }
 	k_fsst_dict<<<1, 1024, 0, s>>>(lens, comp, comp_size, entry_c, tab, ends, bytes, cap, status);
+	++launch_counter();
+	return cudaGetLastError();
+}
+
+cudaError_t launch_dict_align(const uint8_t* bytes, const uint32_t* rows, const uint32_t* rows8, uint32_t entry_c,
+                              uint8_t* bytes8, cudaStream_t s) {
+	if (entry_c == 0) { return cudaSuccess; }
+	k_dict_align<<<(entry_c + 7) / 8, 256, 0, s>>>(bytes, rows, rows8, entry_c, bytes8);
 	++launch_counter();
 	return cudaGetLastError();
 }

@@ -58,6 +58,11 @@ struct StrArgs {
 	uint64_t         bytes_cap;
 	int*             status;
 	uint64_t         item_base; // single-pass DICT decode: index of the column's vector 0 among the look-back words
+	// single-pass DICT decode: the dictionary with every entry on an 8-byte boundary, zero between them, and entry c as
+	// (start / 8) | length << 24
+	const uint8_t*   dict8;
+	const uint32_t*  rows8;
+	uint64_t         dict8_n;
 };
 
 // One launch of the single-pass DICT decode (k_dict_pass) over the vectors of one or more DICT string columns.
@@ -66,7 +71,7 @@ struct StrArgs {
 // its predecessors' totals are known, its inclusive prefix (a decoupled look-back within its column), so each vector
 // learns its first output byte without a separate lengths pass.
 struct StrSetArgs {
-	const StrArgs*  cols;      // per-column arguments in device memory (each with dict_rows: start | length << 24)
+	const StrArgs*  cols;      // per-column arguments in device memory (each with dict8 and rows8)
 	uint32_t        n_cols;
 	uint32_t        active;    // warps of a CTA that take vectors (fewer for sets of fewer vectors than warps)
 	uint64_t        n_items;   // vectors of all columns
@@ -85,6 +90,10 @@ struct StrSetArgs {
 uint32_t dict_pass_smem_per_warp(bool rows16);
 cudaError_t launch_dict_pass(const StrSetArgs& a, bool rows16, int warps, uint32_t dyn_smem, cudaStream_t s,
                              int sm_count = 0);
+
+// The dictionary's entries (rows: start | length << 24) from bytes to their places in bytes8 (rows8), zero behind them.
+cudaError_t launch_dict_align(const uint8_t* bytes, const uint32_t* rows, const uint32_t* rows8, uint32_t entry_c,
+                              uint8_t* bytes8, cudaStream_t s);
 
 cudaError_t launch_fsst_dict(const uint8_t* lens, const uint8_t* comp, uint64_t comp_size, uint32_t entry_c,
                              const FsstTable* tab, uint32_t* ends, uint8_t* bytes, uint64_t cap, int* status,

@@ -359,7 +359,7 @@ int fls_string_plan_create(const uint8_t* d_page, uint64_t page_size, const uint
 		p->single            = true;
 		const uint32_t   pw  = dict_pass_smem_per_warp(a.rows16);
 		const uint64_t   tab = (4ull * a.entry_c + 15) & ~15ull;
-		const uint64_t   all = 224 * 1024, d8 = a.dict8_n;
+		const uint64_t   all = kDictPassSmem, d8 = a.dict8_n;
 		uint64_t         sw  = all / pw;
 		if (d8 + tab < all && (all - d8 - tab) / pw >= 8) {
 			p->sp_dict_cap = static_cast<uint32_t>(d8);
@@ -507,7 +507,7 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 	}
 	const uint32_t pw  = dict_pass_smem_per_warp(set->rows16);
 	const uint64_t tab = (4 * tab_max + 15) & ~15ull;
-	const uint64_t all = 224 * 1024;
+	const uint64_t all = kDictPassSmem;
 	uint64_t       w   = all / pw;
 	if (dict_max + tab < all && (all - dict_max - tab) / pw >= 8) {
 		set->dict_cap = static_cast<uint32_t>(dict_max);

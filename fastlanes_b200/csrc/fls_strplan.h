@@ -86,6 +86,8 @@ struct StrSetArgs {
 	uint32_t        tab_cap;  // entries held for the packed row table (with dict_cap)
 };
 
+// dynamic shared memory of a k_dict_pass CTA (227 KB less its static words)
+constexpr uint32_t kDictPassSmem = 226 * 1024;
 // per-warp shared memory of k_dict_pass: the vector's rows and the output window
 uint32_t dict_pass_smem_per_warp(bool rows16);
 cudaError_t launch_dict_pass(const StrSetArgs& a, bool rows16, int warps, uint32_t dyn_smem, cudaStream_t s,

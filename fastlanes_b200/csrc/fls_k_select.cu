@@ -1581,7 +1581,10 @@ __global__ void __launch_bounds__(256) k_mlp(const float* __restrict__ params, c
 	const uint32_t tid = threadIdx.x, tx = tid % 32, ty = tid / 32;
 	const float*   w1 = params;
 	const float *  b1 = w1 + NF * H, *w2 = b1 + H, *b2 = w2 + H * H, *w3 = b2 + H, *b3 = w3 + H * K;
+	// unrolled so that the weights' loads are in flight together: every CTA waits for them once, before its first row
+#pragma unroll 8
 	for (uint32_t e = tid; e < NF * H; e += 256) { S.w1[e / H][e % H] = __ldg(w1 + e); }
+#pragma unroll 16
 	for (uint32_t e = tid; e < H * H; e += 256) { S.w2[e / H][e % H] = __ldg(w2 + e); }
 	for (uint32_t e = tid; e < H * K; e += 256) { S.w3[e / K][e % K] = __ldg(w3 + e); }
 	if (tid < H) {
@@ -1883,7 +1886,7 @@ struct fls_sel_plan {
 	uint32_t              chunk_vectors = 64;
 	// wizard scratch (gtab: the chunk dictionary's slot scratch, one region per CTA; the subset lists of a
 	// wizard run over some chunks) and the learned selector's; all grow-only
-	Scratch bw_code, parts, info, dict_n, gtab, sub_items, sub_ranges, sub_ccol, sub_ids, sub_sizes, sub_best, vlen, vclen,
+	Scratch bw_code, parts, info, dict_n, gtab, sub_lists, sub_sizes, sub_best, vlen, vclen,
 	    dict_w, l_work, l_conf;
 	// string columns (fls_sel_plan_create_strings): the plan's columns are the row hashes; these are the strings
 	bool                str = false;
@@ -1944,6 +1947,7 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 	const Item*     items_d  = p->items_d.as<Item>();
 	const uint32_t* ranges_d = p->chunk_items_d.as<uint32_t>();
 	const uint32_t* ccol_d   = p->chunk_col_d.as<uint32_t>();
+	const uint32_t* ids_d    = nullptr;
 	uint64_t        n_items  = p->items.size();
 	if (!all) {
 		std::vector<Item>     it;
@@ -1961,18 +1965,21 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 		ranges[chunks.size()] = static_cast<uint32_t>(it.size());
 		n_items               = it.size();
 		if (it.empty()) { return FLS_OK; }
-		if (!p->sub_items.need(it.size() * sizeof(Item)) || !p->sub_ranges.need(ranges.size() * 4) ||
-		    !p->sub_ccol.need(ccol.size() * 4) || !p->sub_ids.need(chunks.size() * 4) ||
-		    cudaMemcpyAsync(p->sub_items.m.p, it.data(), it.size() * sizeof(Item), cudaMemcpyHostToDevice, s) != cudaSuccess ||
-		    cudaMemcpyAsync(p->sub_ranges.m.p, ranges.data(), ranges.size() * 4, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-		    cudaMemcpyAsync(p->sub_ccol.m.p, ccol.data(), ccol.size() * 4, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-		    cudaMemcpyAsync(p->sub_ids.m.p, chunks.data(), chunks.size() * 4, cudaMemcpyHostToDevice, s) != cudaSuccess ||
-		    cudaStreamSynchronize(s) != cudaSuccess) { // the host lists go out of scope
+		// one copy for the four lists, and no wait (a copy from pageable memory is staged before the call returns)
+		const size_t         o1 = it.size() * sizeof(Item), o2 = o1 + ranges.size() * 4, o3 = o2 + ccol.size() * 4;
+		std::vector<uint8_t> lists(o3 + chunks.size() * 4);
+		std::memcpy(lists.data(), it.data(), o1);
+		std::memcpy(lists.data() + o1, ranges.data(), ranges.size() * 4);
+		std::memcpy(lists.data() + o2, ccol.data(), ccol.size() * 4);
+		std::memcpy(lists.data() + o3, chunks.data(), chunks.size() * 4);
+		if (!p->sub_lists.need(lists.size()) ||
+		    cudaMemcpyAsync(p->sub_lists.m.p, lists.data(), lists.size(), cudaMemcpyHostToDevice, s) != cudaSuccess) {
 			return FLS_ERR_CUDA;
 		}
-		items_d  = p->sub_items.as<Item>();
-		ranges_d = p->sub_ranges.as<uint32_t>();
-		ccol_d   = p->sub_ccol.as<uint32_t>();
+		items_d  = p->sub_lists.as<Item>();
+		ranges_d = reinterpret_cast<const uint32_t*>(p->sub_lists.as<uint8_t>() + o1);
+		ccol_d   = reinterpret_cast<const uint32_t*>(p->sub_lists.as<uint8_t>() + o2);
+		ids_d    = reinterpret_cast<const uint32_t*>(p->sub_lists.as<uint8_t>() + o3);
 	}
 	if (n_items == 0) { return FLS_OK; }
 	if (!p->parts.need(n_items * 4) || !p->bw_code.need(n_items * 4) || !p->info.need(n_items * sizeof(VecInfo)) || !p->dict_n.need(chunks.size() * 4)) {
@@ -2041,7 +2048,7 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 	if (!all) {
 		// the subset's choices go to their chunks (sizes of a subset are not reported)
 		if (d_best) {
-			k_scatter_best<<<64, 256, 0, s>>>(best, p->sub_ids.as<uint32_t>(), static_cast<uint32_t>(chunks.size()), d_best);
+			k_scatter_best<<<64, 256, 0, s>>>(best, ids_d, static_cast<uint32_t>(chunks.size()), d_best);
 			++launch_counter();
 		}
 	} else if (d_dict_n) {
@@ -2315,7 +2322,7 @@ int fls_sel_learned(fls_sel_plan* p, const float* d_params, uint32_t stride, flo
 	if (rc != FLS_OK) { return rc; }
 	const uint64_t n = set->n;
 	if (!p->l_work.need(n * (NF + K) * 4) || !p->l_conf.need(p->n_chunks * 4)) { return FLS_ERR_CUDA; }
-	Scratch& conf = p->l_conf;
+	float*   conf = d_conf ? d_conf : p->l_conf.as<float>();
 	float*   feat = p->l_work.as<float>();
 	float*   prob = feat + n * NF;
 	ItemArgs a {p->cols_d.as<Col>(), set->items.as<Item>(), n};
@@ -2323,15 +2330,12 @@ int fls_sel_learned(fls_sel_plan* p, const float* d_params, uint32_t stride, flo
 	if (probabilities(s, d_params, feat, n, prob) != cudaSuccess) { return FLS_ERR_CUDA; }
 	k_vote<<<static_cast<unsigned>((p->n_chunks + 7) / 8), 256, 0, s>>>(prob, set->chunk_items.as<uint32_t>(),
 	                                                                     static_cast<uint32_t>(p->n_chunks), d_choice,
-	                                                                     conf.as<float>(), p->str ? kStrK : K);
+	                                                                     conf, p->str ? kStrK : K);
 	++launch_counter();
 	if (cudaGetLastError() != cudaSuccess) { return FLS_ERR_CUDA; }
-	if (d_conf && cudaMemcpyAsync(d_conf, conf.m.p, p->n_chunks * 4, cudaMemcpyDeviceToDevice, s) != cudaSuccess) {
-		return FLS_ERR_CUDA;
-	}
 	if (threshold > 0.0f) {
 		std::vector<float> hc(p->n_chunks);
-		if (cudaMemcpyAsync(hc.data(), conf.m.p, hc.size() * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
+		if (cudaMemcpyAsync(hc.data(), conf, hc.size() * 4, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
 		    cudaStreamSynchronize(s) != cudaSuccess) {
 			return FLS_ERR_CUDA;
 		}

@@ -1036,46 +1036,55 @@ __device__ __forceinline__ uint64_t str_load8_inside(const StrCol& c, uint64_t p
 // compressed lengths are written as 0 and the vector's sum is scaled by rs).  The CTAs go through the columns one
 // after the other, a warp taking units of kStrUnit rows.
 //   memo     rows whose hash another row of the column had before (dictionary-like columns: nearly all) take its
-//            compressed length from a table in global memory, 64-bit entries of the hash and the length, cleared for
-//            every call; rows are told apart by hash and length.  A first launch over
-//            every `stride`-th vector fills it: all units start at once, so that without it nothing would be found;
+//            compressed length from the column's part of a table in global memory, 64-bit entries of the hash and
+//            the length, cleared for every call; rows are told apart by hash and length.  A first launch over every
+//            `stride`-th vector fills it: all units start at once, so that without it nothing would be found.  With
+//            one table for all columns, those whose rows all differ would push the others' entries out;
 //   match    greedy matching looks at the next two bytes in a 64 KB table in shared memory (what they start: nothing,
 //            a one- or two-byte symbol, or a group of longer ones), so that only the few symbols of one group are
 //            compared, where the symbols sharing a first byte were walked one after the other;
-//   lanes    draw rows from the warp's list as they finish (8 at a time), one code a step: rows of 1 to 20 codes
-//            would otherwise leave most lanes idle.
-// 5.7 M rows (a third of them all different, 17 codes each): 1,677 us by rows and first-byte lists, 128 + 481 us for the
-// two launches, of which the matching is 410 and the hashes 66; instruction-bound.
+//   lanes    draw rows from the warp's list as they finish (8 at a time), four codes between two looks: rows of 1 to 20
+//            codes would otherwise leave most lanes idle.
+// 5.7 M rows of 6 columns (a third of the rows all different, 17 codes each): 1,677 us by rows and first-byte lists; for
+// the two launches 128 + 481 us with one memo for all columns, 123 + 255 us with one each and eight bytes loaded for
+// four codes, 57 + 298 us with units of 32 rows in the first launch.  Bound by instructions and the latency of the rows'
+// loads (issue slots half used, registers full).
 constexpr int      kStrWarps = 16;
-constexpr uint32_t kStrUnit  = 128;          // rows a warp takes at a time
-constexpr uint32_t kStrMemo  = 1u << 17;     // entries (1 MB, in L2)
+constexpr uint32_t kStrPer = 3, kStrUnit = 1024 >> kStrPer; // rows a warp takes at a time (log2 of a vector's units)
+constexpr uint32_t kStrFillPer = 5, kStrFillUnit = 1024 >> kStrFillPer; // one a lane in the launch that fills the memo
+// log2 of a column's memo entries: as many as the largest column has rows, at most 1 MB, and (down to the least) all
+// columns' at most 8 MB, which is cleared in a few microseconds and stays in L2
+constexpr uint32_t kStrMemoMin = 12, kStrMemoMax = 17, kStrMemoAll = 20;
 constexpr uint32_t kStrMemoLen = 4094;       // longest compressed length an entry holds
 struct StrRowsSmem {
-	uint8_t  pair[65536]; // by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g
+	// by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g; behind them, by a row's last byte
+	uint8_t  pair[65536 + 256];
 	StrTab   t;
 	uint32_t off[kStrWarps][kStrUnit + 1]; // a unit's row offsets from its first row's
 	uint16_t list[kStrWarps][kStrUnit];    // rows to match
 };
 
-// Codes and their cost (1, or 2 for an escaped byte) of the string bytes in x, `left` of them still in the row: the
-// length of the next code's bytes; *cost grows by its compressed size.
-__device__ __forceinline__ uint32_t str_next_code(const StrRowsSmem& S, uint64_t x, uint64_t left, uint32_t* cost) {
-	uint32_t what = S.pair[x & 0xFFFFu], step = 0;
-	if (left == 1) { what = (S.t.one[(x & 0xFFu) >> 5] >> (x & 31u)) & 1u; }
+// What the string bytes in x, `left` of them still in the row, start (an entry of pair; its first two bytes are read).
+__device__ __forceinline__ uint32_t str_look(const StrRowsSmem& S, uint32_t x, uint32_t left) {
+	return S.pair[left == 1 ? 65536u + (x & 0xFFu) : x & 0xFFFFu];
+}
+
+// The next code's bytes and (*cost grows by) its compressed size: 1, or 2 for an escaped byte.  x: the next 8 bytes.
+__device__ __forceinline__ uint32_t str_next_code(const StrRowsSmem& S, uint64_t x, uint32_t left, uint32_t* cost) {
+	uint32_t what = str_look(S, static_cast<uint32_t>(x), left);
 	if (what >= kStrGroup) {
 		const uint32_t g = what - kStrGroup;
 		for (uint32_t k = S.t.start[g]; k < S.t.start[g + 1]; ++k) {
 			const ulonglong2 m = S.t.sym[k];
 			if ((x & m.y) == m.x && S.t.len[k] <= left) {
-				step = S.t.len[k];
-				break;
+				*cost += 1;
+				return S.t.len[k];
 			}
 		}
-		what = step ? 1u : S.t.g_short[g];
+		what = S.t.g_short[g];
 	}
-	if (step == 0) { step = what == 2 ? 2u : 1u; }
 	*cost += what ? 1u : 2u;
-	return step;
+	return what == 2 ? 2u : 1u;
 }
 
 __device__ __forceinline__ uint64_t str_hash_step(uint64_t h, uint64_t x, uint64_t left) {
@@ -1085,15 +1094,18 @@ __device__ __forceinline__ uint64_t str_hash_step(uint64_t h, uint64_t x, uint64
 constexpr uint64_t kStrHashSeed = 0x243F6A8885A308D3ull;
 
 // A unit whose offsets do not fit 31 bits from its first one (rows of gigabytes, or corrupt offsets), row by row.
-__device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c, uint64_t r0, uint32_t rs, uint32_t lane,
-                                           uint64_t* sl, uint64_t* sc) {
-	for (uint32_t j = lane; j < kStrUnit; j += 32) {
+__device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c, uint64_t r0, uint32_t unit, uint32_t rs,
+                                           uint32_t lane, uint64_t* sl, uint64_t* sc) {
+	for (uint32_t j = lane; j < unit; j += 32) {
 		const uint64_t r = r0 + j, b = __ldg(c.offsets + r), e = __ldg(c.offsets + r + 1), m = e >= b ? e - b : 0;
 		uint64_t       h = kStrHashSeed ^ m;
 		for (uint64_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_load8(c, b + p), m - p); }
 		uint32_t cl = 0;
 		if ((r & 1023u) % rs == 0) {
-			for (uint64_t p = 0; p < m;) { p += str_next_code(S, str_load8(c, b + p), m - p, &cl); }
+			for (uint64_t p = 0; p < m;) {
+				const uint64_t left = m - p;
+				p += str_next_code(S, str_load8(c, b + p), left < 8 ? static_cast<uint32_t>(left) : 8u, &cl);
+			}
 		}
 		c.hash[r] = h;
 		c.len[r]  = static_cast<uint32_t>(m);
@@ -1103,13 +1115,13 @@ __device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c
 	}
 }
 
-// A row's memo entry: its place, and the entry without the length (the low 12 bits hold length + 1); place and entry
-// together hold all 64 bits of the hash, mixed with the column (its lengths are by its own table) and the row's own
-// length (short rows of different lengths can share a hash: "a" and "b\0" do).
-__device__ __forceinline__ uint64_t str_memo_key(uint64_t h, uint32_t col, uint32_t m, uint32_t* at) {
-	h ^= (static_cast<uint64_t>(col) << 32 | m) * 0x9E3779B97F4A7C15ull;
-	*at = static_cast<uint32_t>(h) & (kStrMemo - 1);
-	return ((h >> 5) ^ (h << 47)) & ~0xFFFull; // bits 17-63 of the hash in bits 12-58
+// A row's memo entry: its place (`bits`, at least 12, of the hash), and the entry without the length (the low 12 bits
+// hold length + 1); place and entry together hold all 64 bits of the hash, mixed with the row's own length (short rows
+// of different lengths can share a hash: "a" and "b\0" do).
+__device__ __forceinline__ uint64_t str_memo_key(uint64_t h, uint32_t m, uint32_t bits, uint32_t* at) {
+	h ^= m * 0x9E3779B97F4A7C15ull;
+	*at = static_cast<uint32_t>(h) & ((1u << bits) - 1u);
+	return h & ~0xFFFull;
 }
 
 struct StrRowsArgs {
@@ -1117,7 +1129,8 @@ struct StrRowsArgs {
 	const Item*   items; // by column
 	uint64_t      n_items;
 	uint64_t *    vlen, *vclen; // optional: sums of every item, zero before the first launch
-	uint64_t*     memo;
+	uint64_t*     memo; // 1 << memo_bits entries for every column
+	uint32_t      memo_bits;
 	uint32_t      rs;
 	uint32_t      stride; // every stride-th item in the launch that fills the memo, the others in the next one
 	uint32_t      fill;
@@ -1126,9 +1139,9 @@ struct StrRowsArgs {
 __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArgs a) {
 	extern __shared__ __align__(16) uint8_t smem[];
 	StrRowsSmem&       S  = *reinterpret_cast<StrRowsSmem*>(smem);
-	constexpr uint32_t nt = kStrWarps * 32, kPer = 1024 / kStrUnit; // units of a vector
+	constexpr uint32_t nt = kStrWarps * 32;
+	const uint32_t     unit = a.fill ? kStrFillUnit : kStrUnit, per = a.fill ? kStrFillPer : kStrPer; // rows; log2 of units
 	const uint32_t     tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, rs = a.rs;
-	uint64_t* const    memo = a.memo;
 	// this launch's items: i * stride (fill), or the others in order; number i of them
 	const uint64_t n_fill = (a.n_items + a.stride - 1) / a.stride;
 	const uint64_t n      = a.fill ? n_fill : a.n_items - n_fill;
@@ -1146,12 +1159,13 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 				hi = mid;
 			}
 		}
-		const uint64_t u0 = first * kPer, u1 = lo * kPer;
+		const uint64_t u0 = first << per, u1 = lo << per;
 		first             = lo;
 		// the CTA's first unit of the column at or after u0: one of warp gw .. gw + kStrWarps - 1 (mod nw)
 		const uint64_t mine = u0 + (gw + kStrWarps - 1 + nw - u0 % nw) % nw; // of the CTA's last warp
 		if (mine >= u1 + kStrWarps - 1) { continue; }
-		const StrCol c = a.cols[col];
+		const StrCol    c    = a.cols[col];
+		uint64_t* const memo = a.memo + (static_cast<uint64_t>(col) << a.memo_bits);
 		__syncthreads(); // the previous column's table is read to the end
 		for (uint32_t k = tid; k < sizeof(StrTab) / 4; k += nt) {
 			reinterpret_cast<uint32_t*>(&S.t)[k] = __ldg(reinterpret_cast<const uint32_t*>(c.tab) + k);
@@ -1160,6 +1174,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 		for (uint32_t k = tid; k < 65536 / 4; k += nt) { // bytes 4k .. 4k + 3: the low byte of the pair
 			const uint32_t m                       = S.t.one[(k & 63u) >> 3] >> (4 * (k & 7u));
 			reinterpret_cast<uint32_t*>(S.pair)[k] = (m & 1u) | ((m & 2u) << 7) | ((m & 4u) << 14) | ((m & 8u) << 21);
+			if (k < 64) { reinterpret_cast<uint32_t*>(S.pair)[65536 / 4 + k] = reinterpret_cast<uint32_t*>(S.pair)[k]; }
 		}
 		__syncthreads();
 		for (uint32_t k = tid; k < S.t.n_two; k += nt) { S.pair[S.t.two[k]] = 2; }
@@ -1167,23 +1182,23 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 		for (uint32_t k = tid; k < S.t.n_pair; k += nt) { S.pair[S.t.pair[k]] = static_cast<uint8_t>(kStrGroup + S.t.pair_group[k]); }
 		__syncthreads();
 		for (uint64_t u = u0 + (gw + warp + nw - u0 % nw) % nw; u < u1; u += nw) {
-			const uint64_t it = item(u / kPer);
+			const uint64_t it = item(u >> per);
 			uint64_t       sl = 0, sc = 0;
 			{
-				const uint64_t r0   = static_cast<uint64_t>(a.items[it].vec) * 1024 + (u % kPer) * kStrUnit;
+				const uint64_t r0   = static_cast<uint64_t>(a.items[it].vec) * 1024 + (u & ((1u << per) - 1u)) * unit;
 				const uint64_t o0   = __ldg(c.offsets + r0);
 				uint32_t*      off  = S.off[warp];
 				uint16_t*      list = S.list[warp];
 				bool           wide = false;
 				__syncwarp(); // the warp's previous unit is read to the end
-				for (uint32_t j = lane; j <= kStrUnit; j += 32) {
+				for (uint32_t j = lane; j <= unit; j += 32) {
 					const uint64_t o = __ldg(c.offsets + r0 + j) - o0;
 					wide |= o >= (1ull << 31);
 					off[j] = static_cast<uint32_t>(o);
 				}
 				__syncwarp();
 				if (__any_sync(0xFFFFFFFFu, wide)) {
-					str_unit_wide(S, c, r0, rs, lane, &sl, &sc);
+					str_unit_wide(S, c, r0, unit, rs, lane, &sl, &sc);
 				} else {
 					// offsets from o0 below this lie at least 12 bytes before the column's end
 					const uint64_t room  = c.n_bytes > o0 ? c.n_bytes - o0 : 0;
@@ -1192,10 +1207,10 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 					uint32_t todo = 0;
 					uint32_t at = 0, row = 0, ask = 0; // the look into the memo of the row before
 					uint64_t key = 0, seen = 0;
-					for (uint32_t j = lane; j < kStrUnit + 32; j += 32) {
+					for (uint32_t j = lane; j < unit + 32; j += 32) {
 						uint32_t row_next = j, ask_next = 0, at_next = 0;
 						uint64_t key_next = 0, seen_next = 0;
-						if (j < kStrUnit) {
+						if (j < unit) {
 							const uint32_t b = off[j], e = off[j + 1], m = e >= b ? e - b : 0;
 							const bool     inside = e < limit;
 							uint64_t       h = kStrHashSeed ^ m;
@@ -1205,7 +1220,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 							c.len[r]         = m;
 							sl += m;
 							if ((r & 1023u) % rs == 0) {
-								key_next  = str_memo_key(h, col, m, &at_next);
+								key_next  = str_memo_key(h, m, a.memo_bits, &at_next);
 								seen_next = __ldcg(memo + at_next);
 								ask_next  = 1;
 							} else {
@@ -1246,13 +1261,34 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 						} else if (idle == 0xFFFFFFFFu) {
 							break;
 						}
-						// four codes between two looks at who is idle
+						// four codes between two looks at who is idle, from one load of eight bytes while they are of one
+						// and two bytes: straight through, as no more is asked of them than the table's entry
+						uint64_t x   = left ? load8(p, inside) : 0;
+						uint32_t got = 8;
+#pragma unroll
 						for (uint32_t k = 0; k < 4; ++k) {
-							if (have && left) {
-								const uint32_t step = str_next_code(S, load8(p, inside), left, &cl);
-								p += step;
-								left -= step;
+							const uint32_t what = str_look(S, static_cast<uint32_t>(x), left);
+							const bool     on   = left != 0;
+							uint32_t       step = on ? 1u + (what >> 1) : 0u;
+							if (on && what >= kStrGroup) {
+								if (got < 8) {
+									x   = load8(p, inside);
+									got = 8;
+								}
+								step = str_next_code(S, x, left, &cl);
+								if (got < step + 2 * (3 - k)) { // the codes to come may need two bytes each
+									x   = left > step ? load8(p + step, inside) : 0;
+									got = 8 + step;
+								} else {
+									x = step < 8 ? x >> (8 * step) : 0;
+								}
+							} else {
+								cl += on ? 1u + (what == 0) : 0u;
+								x >>= 8 * step;
 							}
+							p += step;
+							left -= step;
+							got -= step;
 						}
 						if (have && left == 0) {
 							c.clen[r0 + j] = cl;
@@ -1265,7 +1301,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 						const uint64_t r = r0 + list[k];
 						const uint32_t l = c.clen[r];
 						const uint32_t b = off[list[k]], e = off[list[k] + 1];
-						key              = str_memo_key(c.hash[r], col, e >= b ? e - b : 0, &at);
+						key              = str_memo_key(c.hash[r], e >= b ? e - b : 0, a.memo_bits, &at);
 						if (l <= kStrMemoLen) { __stcg(memo + at, key | (l + 1)); }
 					}
 				}
@@ -1283,7 +1319,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 // k_str_rows over n_items vectors, two CTAs a SM: the launch that fills the memo over as many vectors as give every
 // warp a unit, then the rest.
 cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_items, uint64_t* vlen, uint64_t* vclen,
-                            uint32_t rs, uint64_t* memo, cudaStream_t s) {
+                            uint32_t rs, uint64_t* memo, uint32_t memo_bits, uint64_t n_cols, cudaStream_t s) {
 	Device* d = current_device();
 	if (!d || d->ordinal < 0 || d->ordinal >= 64) { return cudaErrorInvalidDevice; }
 	static bool set[64] = {};
@@ -1292,16 +1328,16 @@ cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_it
 		if (e != cudaSuccess) { return e; }
 		set[d->ordinal] = true;
 	}
-	cudaError_t e = cudaMemsetAsync(memo, 0, kStrMemo * 8, s);
+	cudaError_t e = cudaMemsetAsync(memo, 0, (n_cols << memo_bits) * 8, s);
 	if (e == cudaSuccess && vlen) { e = cudaMemsetAsync(vlen, 0, n_items * 8, s); }
 	if (e == cudaSuccess && vclen) { e = cudaMemsetAsync(vclen, 0, n_items * 8, s); }
 	if (e != cudaSuccess) { return e; }
-	const uint64_t warps = static_cast<uint64_t>(d->sm_count) * 2 * kStrWarps, per = 1024 / kStrUnit;
-	const uint64_t step  = (n_items * per + warps - 1) / warps;
-	StrRowsArgs    a {cols, items, n_items, vlen, vclen, memo, rs, static_cast<uint32_t>(std::max<uint64_t>(1, step)), 1};
+	const uint64_t warps = static_cast<uint64_t>(d->sm_count) * 2 * kStrWarps, step = ((n_items << kStrFillPer) + warps - 1) / warps;
+	StrRowsArgs    a {cols, items, n_items, vlen, vclen, memo, memo_bits, rs, static_cast<uint32_t>(std::max<uint64_t>(1, step)), 1};
 	for (const uint32_t fill : {1u, 0u}) {
 		const uint64_t n_fill = (n_items + a.stride - 1) / a.stride, n = fill ? n_fill : n_items - n_fill;
-		const uint64_t ctas   = std::min((n * per + kStrWarps - 1) / kStrWarps, static_cast<uint64_t>(d->sm_count) * 2);
+		const uint64_t units  = n << (fill ? kStrFillPer : kStrPer);
+		const uint64_t ctas   = std::min((units + kStrWarps - 1) / kStrWarps, static_cast<uint64_t>(d->sm_count) * 2);
 		a.fill                = fill;
 		if (ctas) {
 			k_str_rows<<<static_cast<unsigned>(ctas), kStrWarps * 32, sizeof(StrRowsSmem), s>>>(a);
@@ -1892,6 +1928,7 @@ struct fls_sel_plan {
 	bool                str = false;
 	std::vector<StrCol> scols;
 	DevMem              scols_d, tabs_d, hash_d, len_d, clen_d, wptr_d, str_memo;
+	uint32_t            memo_bits = 0;
 	std::map<uint32_t, ItemSet> samples; // stride -> sampled items
 };
 
@@ -1991,7 +2028,7 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 			return FLS_ERR_CUDA;
 		}
 		if (launch_str_rows(p->scols_d.as<StrCol>(), items_d, n_items, p->vlen.as<uint64_t>(), p->vclen.as<uint64_t>(), 1u,
-		                    p->str_memo.as<uint64_t>(), s) != cudaSuccess) {
+		                    p->str_memo.as<uint64_t>(), p->memo_bits, p->scols.size(), s) != cudaSuccess) {
 			return FLS_ERR_CUDA;
 		}
 	}
@@ -2221,7 +2258,14 @@ int fls_sel_plan_create_strings(const fls_sel_str_column* cols, uint32_t n_cols,
 	               (rc = upload(own->wptr_d, wp.data(), sizeof(void*) * wp.size())) != FLS_OK)) {
 		return rc != FLS_OK ? rc : FLS_ERR_CUDA;
 	}
-	if (!own->str_memo.alloc(kStrMemo * 8)) { return FLS_ERR_CUDA; }
+	uint64_t most = 1; // rows of a column
+	for (uint32_t c = 0; c < n_cols; ++c) { most = std::max<uint64_t>(most, cols[c].n_rows); }
+	own->memo_bits = kStrMemoMax;
+	while (own->memo_bits > kStrMemoMin && ((1ull << (own->memo_bits - 1)) >= most ||
+	                                        (static_cast<uint64_t>(n_cols) << own->memo_bits) > (1ull << kStrMemoAll))) {
+		--own->memo_bits;
+	}
+	if (!own->str_memo.alloc((static_cast<uint64_t>(n_cols ? n_cols : 1) << own->memo_bits) * 8)) { return FLS_ERR_CUDA; }
 	own->str   = true;
 	own->scols = sc;
 	own->hash_d.p = hash.p, hash.p = nullptr;
@@ -2280,7 +2324,7 @@ cudaError_t        sample_features(fls_sel_plan* p, const ItemArgs& a, float* fe
 	if (p->str) {
 		const cudaError_t e =
 		    launch_str_rows(p->scols_d.as<StrCol>(), a.items, a.n_items, nullptr, nullptr, kStrFeatRowStride,
-		                    p->str_memo.as<uint64_t>(), s);
+		                    p->str_memo.as<uint64_t>(), p->memo_bits, p->scols.size(), s);
 		if (e != cudaSuccess) { return e; }
 	}
 	cudaError_t e = launch_features(a, feat, s);

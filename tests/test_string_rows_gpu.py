@@ -63,3 +63,34 @@ def test_string_rows_edges(cuda, n_vec):
         assert int(sizes[c, 0]) == frame + sum(map(len, rows)) + 4096 * n_vec
     assert P.device_status() == 0
     plan.close()
+
+
+@pytest.mark.parametrize("n_cols", [40, 300])
+def test_string_rows_many_columns(cuda, n_cols):
+    """Columns of the same strings under different tables, more vectors than the launch that fills the memo takes, and
+    (300 columns) the smallest part of the memo for each."""
+    import torch
+
+    from fastlanes_b200 import primitives as P
+    from fastlanes_b200 import select as SL
+
+    rng = np.random.default_rng(n_cols)
+    names = [n for n in TABLES if n != "pairs"]
+    pool = [bytes(rng.choice(np.frombuffer(b"abcdefghx\0\xff", np.uint8), int(n))) for n in rng.integers(0, 30, 200)]
+    cost = {name: np.array([_compressed(r, TABLES[name]) for r in pool]) for name in names}
+    lens = np.array([len(r) for r in pool])
+    n_vec = -(-600 // n_cols)
+    cols, want, keep = [], [], {name: _table(TABLES[name]) for name in names}
+    for c in range(n_cols):
+        pick = rng.integers(0, len(pool), 1024 * n_vec)
+        offs = np.concatenate([[0], np.cumsum(lens[pick])]).astype(np.int64)
+        data = torch.from_numpy(np.frombuffer(b"".join(pool[i] for i in pick), np.uint8).copy()).to(cuda)
+        name = names[c % len(names)]
+        cols.append((data, torch.from_numpy(offs).to(cuda), keep[name]))
+        frame = 8 + 4 * 2 + 4 * 2 * (n_vec - 1)
+        want.append(frame + int(cost[name][pick].sum()) + 4096 * n_vec + 8 + keep[name].size)
+    plan = SL.StrSelectionPlan(cols)
+    sizes = plan.wizard()[0].cpu().numpy()
+    assert [int(x) for x in sizes[:, 2]] == want
+    assert P.device_status() == 0
+    plan.close()

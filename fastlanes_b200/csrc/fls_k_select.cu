@@ -1054,14 +1054,14 @@ constexpr uint32_t kStrPer = 3, kStrUnit = 1024 >> kStrPer; // rows a warp takes
 constexpr uint32_t kStrFillPer = 5, kStrFillUnit = 1024 >> kStrFillPer; // one a lane in the launch that fills the memo
 // log2 of a column's memo entries: as many as the largest column has rows, at most 1 MB, and (down to the least) all
 // columns' at most 8 MB, which is cleared in a few microseconds and stays in L2
-constexpr uint32_t kStrMemoMin = 12, kStrMemoMax = 17, kStrMemoAll = 20;
+constexpr uint32_t kStrMemoMin = 13, kStrMemoMax = 17, kStrMemoAll = 20;
 constexpr uint32_t kStrMemoLen = 4094;       // longest compressed length an entry holds
 struct StrRowsSmem {
 	// by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g; behind them, by a row's last byte
 	uint8_t  pair[65536 + 256];
 	StrTab   t;
 	uint32_t off[kStrWarps][kStrUnit + 1]; // a unit's row offsets from its first row's
-	uint16_t list[kStrWarps][kStrUnit];    // rows to match
+	uint16_t list[kStrWarps][kStrUnit];    // rows to match; bit 15: which of its pair's memo entries a row takes
 };
 
 // What the string bytes in x, `left` of them still in the row, start (an entry of pair; its first two bytes are read).
@@ -1115,12 +1115,14 @@ __device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c
 	}
 }
 
-// A row's memo entry: its place (`bits`, at least 12, of the hash), and the entry without the length (the low 12 bits
-// hold length + 1); place and entry together hold all 64 bits of the hash, mixed with the row's own length (short rows
-// of different lengths can share a hash: "a" and "b\0" do).
+// A row's memo entry: its place (a pair of entries, told by bits - 1, at least 12, of the hash), and the entry without the
+// length (the low 12 bits hold length + 1); place and entry together hold all 64 bits of the hash, mixed with the
+// row's own length (short rows of different lengths can share a hash: "a" and "b\0" do).  In pairs, because strings
+// that share a place push each other out for good, and a warp waits for its few rows that miss: 4,096 strings in 64 Ki
+// single entries, of which 6 % share one, 83 + 667 us for 7.4 M rows of 12 columns, 81 + 541 us so.
 __device__ __forceinline__ uint64_t str_memo_key(uint64_t h, uint32_t m, uint32_t bits, uint32_t* at) {
 	h ^= m * 0x9E3779B97F4A7C15ull;
-	*at = static_cast<uint32_t>(h) & ((1u << bits) - 1u);
+	*at = static_cast<uint32_t>(h) & ((1u << (bits - 1)) - 1u);
 	return h & ~0xFFFull;
 }
 
@@ -1164,8 +1166,8 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 		// the CTA's first unit of the column at or after u0: one of warp gw .. gw + kStrWarps - 1 (mod nw)
 		const uint64_t mine = u0 + (gw + kStrWarps - 1 + nw - u0 % nw) % nw; // of the CTA's last warp
 		if (mine >= u1 + kStrWarps - 1) { continue; }
-		const StrCol    c    = a.cols[col];
-		uint64_t* const memo = a.memo + (static_cast<uint64_t>(col) << a.memo_bits);
+		const StrCol      c    = a.cols[col];
+		ulonglong2* const memo = reinterpret_cast<ulonglong2*>(a.memo + (static_cast<uint64_t>(col) << a.memo_bits));
 		__syncthreads(); // the previous column's table is read to the end
 		for (uint32_t k = tid; k < sizeof(StrTab) / 4; k += nt) {
 			reinterpret_cast<uint32_t*>(&S.t)[k] = __ldg(reinterpret_cast<const uint32_t*>(c.tab) + k);
@@ -1206,10 +1208,12 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 					auto load8 = [&](uint32_t p, bool inside) { return inside ? str_load8_inside(c, o0 + p) : str_load8(c, o0 + p); };
 					uint32_t todo = 0;
 					uint32_t at = 0, row = 0, ask = 0; // the look into the memo of the row before
-					uint64_t key = 0, seen = 0;
+					uint64_t key = 0;
+					ulonglong2 seen = make_ulonglong2(0, 0);
 					for (uint32_t j = lane; j < unit + 32; j += 32) {
 						uint32_t row_next = j, ask_next = 0, at_next = 0;
-						uint64_t key_next = 0, seen_next = 0;
+						uint64_t key_next = 0;
+						ulonglong2 seen_next = make_ulonglong2(0, 0);
 						if (j < unit) {
 							const uint32_t b = off[j], e = off[j + 1], m = e >= b ? e - b : 0;
 							const bool     inside = e < limit;
@@ -1227,15 +1231,17 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 								c.clen[r] = 0;
 							}
 						}
-						const bool hit = ask && (seen & ~0xFFFull) == key && (seen & 0xFFFu) != 0;
+						const uint64_t found = (seen.x & ~0xFFFull) == key ? seen.x : seen.y;
+						const bool     hit   = ask && (found & ~0xFFFull) == key && (found & 0xFFFu) != 0;
 						if (hit) {
-							const uint32_t cl = static_cast<uint32_t>(seen & 0xFFFu) - 1;
+							const uint32_t cl = static_cast<uint32_t>(found & 0xFFFu) - 1;
 							c.clen[r0 + row]  = cl;
 							sc += cl;
 						}
 						const bool     miss = ask && !hit;
+						const uint32_t slot = seen.x == 0 ? 0u : seen.y == 0 ? 1u : static_cast<uint32_t>(key >> 40) & 1u;
 						const uint32_t m    = __ballot_sync(0xFFFFFFFFu, miss);
-						if (miss) { list[todo + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(row); }
+						if (miss) { list[todo + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(row | slot << 15); }
 						todo += __popc(m);
 						row = row_next, ask = ask_next, at = at_next, key = key_next, seen = seen_next;
 					}
@@ -1249,7 +1255,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 								const uint32_t k = next + __popc(idle & ((1u << lane) - 1u));
 								have             = k < todo;
 								if (have) {
-									j                = list[k];
+									j                = list[k] & 0x7FFFu;
 									p                = off[j];
 									const uint32_t e = off[j + 1];
 									left             = e >= p ? e - p : 0;
@@ -1298,11 +1304,14 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 					}
 					__syncwarp();
 					for (uint32_t k = lane; k < todo; k += 32) { // what was matched, for the rows to come
-						const uint64_t r = r0 + list[k];
+						const uint32_t i = list[k] & 0x7FFFu;
+						const uint64_t r = r0 + i;
 						const uint32_t l = c.clen[r];
-						const uint32_t b = off[list[k]], e = off[list[k] + 1];
+						const uint32_t b = off[i], e = off[i + 1];
 						key              = str_memo_key(c.hash[r], e >= b ? e - b : 0, a.memo_bits, &at);
-						if (l <= kStrMemoLen) { __stcg(memo + at, key | (l + 1)); }
+						if (l <= kStrMemoLen) { // into the entry of the pair that was free, or over one of the two
+							__stcg(reinterpret_cast<uint64_t*>(memo + at) + (list[k] >> 15), key | (l + 1));
+						}
 					}
 				}
 			}

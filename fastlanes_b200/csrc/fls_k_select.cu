@@ -12,6 +12,7 @@
 #include "fls_device.cuh"
 #include "fls_runtime.h"
 #include "fls_b200.h"
+#include "fls_cd_queue.cuh"
 #include "fls_select.h"
 #include "fls_strings.cuh"
 #include "fls_strplan.h"
@@ -470,9 +471,11 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_features(ItemArgs a, float* 
 //             in shared memory; keys that have to look further go back on it.  So runs, other parts' keys and long
 //             probes cost no idle lanes (a loop of its own for every warp of keys went round for its unluckiest
 //             lane, 200 to 300 instructions a step);
-//   parts     a chunk of more distinct values goes through the table in parts of the hash space (2, then 4, ...);
-//             the count beside the rows done says early whether it will.
-// Exact for every chunk.  Instruction-bound.  28 integer columns (30 M values, 462
+//   parts     a chunk of more distinct values goes through the table in parts of the hash space (2, then 4); the count
+//             beside the rows done says early whether it will;
+//   sort      keys that crowd, whatever the reason (every hash has such keys), spend a warp's looks or overflow four
+//             parts: their chunk's positions are sorted by value instead.
+// Exact for every chunk: the hash only decides how long it takes.  Instruction-bound.  28 integer columns (30 M values, 462
 // chunks): 1,855 us with 16 Ki slots of keys and positions and a bucket pass through global memory, 284 us so; 5.7 M
 // string hashes (90 chunks): 710 us, 138 us.
 // ---------------------------------------------------------------------------------------------------------
@@ -480,10 +483,11 @@ constexpr uint32_t kCdThreads = 1024;
 constexpr uint32_t kCdWarps   = kCdThreads / 32;
 constexpr uint32_t kCdSlots   = 47 * 1024;
 constexpr uint32_t kCdCap     = 43 * 1024; // keys the table takes (eleven twelfths), and those in flight
-constexpr uint32_t kCdMaxParts = 256;
-constexpr uint32_t kCdMaxSteps = 1u << 20; // a warp's steps in a part; never reached: the table has free slots
+constexpr uint32_t kCdMaxParts = 4; // two hold every chunk whose keys spread
+// looks a warp may spend on the keys of one filling of the table.  Keys that spread leave it far away (a table filled to
+// kCdCap takes some 300 a warp, a warp whose 2,048 keys all come last some 5,000); keys that crowd are sorted instead.
+constexpr uint32_t kCdLooks    = 1u << 14;
 constexpr uint32_t kCdWords   = kMaxVecPerChunk * 1024 / 32;
-constexpr uint32_t kCdFree    = 0xFFFFFFFFu;
 constexpr uint64_t kCdGBytes  = kMaxVecPerChunk * 1024 * 2; // per CTA: the slots of every vector's keys
 // unique: the filter (2^20 bits) lies where the table of the marked values then goes; behind it the marks (2^18 bits)
 constexpr uint32_t kCdUniqueSlots = 32 * 1024;
@@ -496,11 +500,11 @@ static_assert(kCdCap + 2 * kCdThreads < kCdSlots && kCdSlots < 0xFFFFu, "free sl
 struct ChunkDictSmem {
 	uint32_t table[kCdSlots]; // at the end: the exclusive prefix of the bitmap words' popcounts
 	uint32_t bits[kCdWords];  // first positions
-	uint64_t qkey[kCdWarps][64];
-	uint16_t qpos[kCdWarps][64], qslot[kCdWarps][64], qtag[kCdWarps][64];
+	uint64_t qkey[kCdWarps][kCdQueue];
+	uint16_t qpos[kCdWarps][kCdQueue], qslot[kCdWarps][kCdQueue], qtag[kCdWarps][kCdQueue];
 	uint32_t vrange[kMaxVecPerChunk][2]; // smallest and largest first position of a vector's values
 	uint32_t wsum[33];
-	uint32_t chunk, over, count, mode, distinct;
+	uint32_t chunk, over, spent, count, mode, distinct;
 	uint64_t lo;    // direct: the lowest value
 	uint64_t dw[2]; // weights of the first positions
 };
@@ -524,94 +528,6 @@ struct ChunkDictArgs {
 	uint64_t*       dict_w;
 	uint16_t*       gslots; // gridDim.x regions of kCdGBytes
 	uint32_t*       ticket; // zero: the next chunk to take
-};
-
-// A key's hash: *place places it (its top bits choose the part), *tag is what its slot keeps in the upper half (never
-// all ones, so that no slot reads as free).  32-bit keys: the 32-bit finaliser of MurmurHash3 (Appleby), a bijection.
-__device__ __forceinline__ void cd_hash(uint32_t x, uint32_t* place, uint32_t* tag) {
-	x ^= x >> 16;
-	x *= 0x85ebca6bu;
-	x ^= x >> 13;
-	x *= 0xc2b2ae35u;
-	x ^= x >> 16;
-	*place           = x;
-	const uint32_t t = x << 16;
-	*tag             = t == 0xFFFF0000u ? 0u : t;
-}
-// 64-bit keys: two linear combinations of the halves by odd constants, the one that places mixed as above.
-__device__ __forceinline__ void cd_hash(uint64_t x, uint32_t* place, uint32_t* tag) {
-	const uint32_t lo = static_cast<uint32_t>(x), hi = static_cast<uint32_t>(x >> 32);
-	uint32_t       a  = lo * 0x9E3779B1u + hi * 0x85EBCA77u;
-	const uint32_t t  = (lo * 0xC2B2AE3Du + hi * 0x27D4EB2Fu) & 0xFFFF0000u;
-	a ^= a >> 15;
-	a *= 0x2C1B3C6Du;
-	a ^= a >> 13;
-	*place = a;
-	*tag   = t == 0xFFFF0000u ? 0u : t;
-}
-
-// One look at slot *s for value x at position pos: done (it is the key's slot now) or not (*s is the next one).
-template <class T>
-__device__ __forceinline__ bool cd_step(uint32_t* table, uint32_t n_slots, const T* vals, T x, uint32_t pos, uint32_t tag,
-                                        uint32_t* s, bool* fresh) {
-	uint32_t e = *reinterpret_cast<volatile uint32_t*>(table + *s);
-	if (e == kCdFree) {
-		e = atomicCAS(table + *s, kCdFree, tag | pos);
-		if (e == kCdFree) {
-			*fresh = true;
-			return true;
-		}
-	}
-	if ((e ^ tag) < 0x10000u && __ldg(vals + (e & 0xFFFFu)) == x) {
-		if (pos < (e & 0xFFFFu)) { atomicMin(table + *s, tag | pos); }
-		return true;
-	}
-	*s = *s + 1 == n_slots ? 0 : *s + 1;
-	return false;
-}
-
-// A warp's queue of keys on their way into the table, and the list of the slots they ended in (the current vector's).
-template <class T>
-struct CdQueue {
-	T*         key;
-	uint16_t * pos, *slot, *tag;
-	uint16_t*  list;
-	uint32_t   q, n; // keys queued, slots listed
-
-	__device__ __forceinline__ void push(bool take, T x, uint32_t at_pos, uint32_t s, uint32_t t, uint32_t lane) {
-		const uint32_t m = __ballot_sync(0xFFFFFFFFu, take);
-		if (take) {
-			const uint32_t at = q + __popc(m & ((1u << lane) - 1u));
-			key[at]           = x;
-			pos[at]           = static_cast<uint16_t>(at_pos);
-			slot[at]          = static_cast<uint16_t>(s);
-			tag[at]           = static_cast<uint16_t>(t >> 16);
-		}
-		q += __popc(m);
-		__syncwarp();
-	}
-	// One look for every lane's key (those of `have`); the unfinished ones go on the queue.  Returns the new keys.
-	__device__ __forceinline__ uint32_t look(uint32_t* table, uint32_t n_slots, const T* vals, bool have, T x,
-	                                         uint32_t at_pos, uint32_t s, uint32_t t, uint32_t lane) {
-		bool fresh = false, done = false;
-		if (have) { done = cd_step<T>(table, n_slots, vals, x, at_pos, t, &s, &fresh); }
-		const uint32_t m = __ballot_sync(0xFFFFFFFFu, done);
-		if (done) { list[n + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(s); }
-		n += __popc(m);
-		push(have && !done, x, at_pos, s, t, lane);
-		return __popc(__ballot_sync(0xFFFFFFFFu, fresh));
-	}
-	// The last up to 32 queued keys take a look each.
-	__device__ __forceinline__ uint32_t pop(uint32_t* table, uint32_t n_slots, const T* vals, uint32_t lane) {
-		const uint32_t take = q < 32 ? q : 32;
-		q -= take;
-		const bool     have = lane < take;
-		const uint32_t at   = q + (have ? lane : 0u);
-		const T        x    = key[at];
-		const uint32_t p = pos[at], s = slot[at], t = static_cast<uint32_t>(tag[at]) << 16;
-		__syncwarp(); // read before the unfinished ones are written back
-		return look(table, n_slots, vals, have, x, p, s, t, lane);
-	}
 };
 
 // How the chunk of items [i0, i0 + nv) is done (warp 0; CD_*), from its vectors' notes.
@@ -638,10 +554,80 @@ __device__ __forceinline__ void cd_choose(const ChunkDictArgs& a, uint32_t i0, u
 	unsorted = __any_sync(0xFFFFFFFFu, unsorted != 0);
 	if (lane == 0) {
 		S.lo       = lo;
+		S.spent    = 0;
 		S.distinct = runs - borders; // of a sorted chunk
 		// fewer runs than the table takes in one part with room to spare go straight to it
 		S.mode = !unsorted && !a.w0 ? CD_SORTED : hi - lo < kCdSlots ? CD_DIRECT : runs > kCdCap / 2 ? CD_UNIQUE : CD_TABLE;
 	}
+}
+
+// First positions and vector ranges of a chunk without a hash: its positions (order: space for them in global memory)
+// sorted by value and then position with Batcher's merge exchange (Knuth, The Art of Computer Programming 3, algorithm
+// 5.2.2M), so that the positions of a value stand side by side, the first one in front.  136 passes over 65,536
+// positions: some milliseconds a chunk, however its keys are made.
+template <class T>
+__device__ __noinline__ void cd_sort(const T* vals, uint32_t nv, uint16_t* order, const uint32_t* w0, const uint32_t* w1,
+                                     ChunkDictSmem& S) {
+	const uint32_t tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, n = nv * 1024;
+	for (uint32_t i = tid; i < n; i += kCdThreads) { order[i] = static_cast<uint16_t>(i); }
+	__syncthreads();
+	const uint32_t top = 1u << (31 - __clz(n - 1)); // the largest power of two below n
+	for (uint32_t p = top; p > 0; p >>= 1) {
+		uint32_t r = 0, d = p;
+		for (uint32_t q = top;; q >>= 1) {
+			for (uint32_t i = tid; i + d < n; i += kCdThreads) {
+				if ((i & p) != r) { continue; }
+				const uint32_t a = order[i], b = order[i + d];
+				const T        x = __ldg(vals + a), y = __ldg(vals + b);
+				if (x > y || (x == y && a > b)) {
+					order[i]     = static_cast<uint16_t>(b);
+					order[i + d] = static_cast<uint16_t>(a);
+				}
+			}
+			__syncthreads();
+			if (q == p) { break; }
+			d = q - p;
+			r = p;
+		}
+	}
+	// nv neighbouring positions a thread; each takes its value's first position from the last head (the first position
+	// of a value) up to it, which may lie in an earlier thread's stretch: a scan hands it on
+	const uint32_t i0 = tid * nv;
+	auto           is_head = [&](uint32_t i) { return i == 0 || __ldg(vals + order[i]) != __ldg(vals + order[i - 1]); };
+	uint32_t       head = 0; // the stretch's last one, plus one
+	uint64_t       s0 = 0, s1 = 0;
+	for (uint32_t i = i0; i < i0 + nv; ++i) {
+		if (!is_head(i)) { continue; }
+		const uint32_t f = order[i];
+		head             = i + 1;
+		atomicOr(S.bits + (f >> 5), 1u << (f & 31u));
+		if (w0) {
+			s0 += __ldg(w0 + f);
+			s1 += __ldg(w1 + f);
+		}
+	}
+	if (w0) {
+		atomicAdd(reinterpret_cast<unsigned long long*>(S.dw), static_cast<unsigned long long>(s0));
+		atomicAdd(reinterpret_cast<unsigned long long*>(S.dw + 1), static_cast<unsigned long long>(s1));
+	}
+	uint32_t upto = head; // the last head of the warp's lanes up to this one
+	for (uint32_t d = 1; d < 32; d <<= 1) {
+		const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, upto, d);
+		if (lane >= d) { upto = max(upto, y); }
+	}
+	uint32_t before = __shfl_up_sync(0xFFFFFFFFu, upto, 1);
+	if (lane == 0) { before = 0; }
+	if (lane == 31) { S.wsum[warp] = upto; }
+	__syncthreads();
+	for (uint32_t w = 0; w < warp; ++w) { before = max(before, S.wsum[w]); }
+	uint32_t f = before ? order[before - 1] : 0u;
+	for (uint32_t i = i0; i < i0 + nv; ++i) {
+		const uint32_t pos = order[i];
+		if (is_head(i)) { f = pos; }
+		atomicMin(&S.vrange[pos >> 10][0], f);
+		atomicMax(&S.vrange[pos >> 10][1], f);
+	}
+	__syncthreads();
 }
 
 template <int W>
@@ -668,7 +654,7 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 	const uint32_t*    w1   = a.w0 ? a.w1[m0.col] + row0 : nullptr;
 	volatile uint32_t* over = &S.over;
 	uint64_t           sw0 = 0, sw1 = 0; // weights of the first positions this thread finds
-	CdQueue<T>         Q {reinterpret_cast<T*>(S.qkey[warp]), S.qpos[warp], S.qslot[warp], S.qtag[warp], nullptr, 0, 0};
+	CdQueue<T>         Q {reinterpret_cast<T*>(S.qkey[warp]), S.qpos[warp], S.qslot[warp], S.qtag[warp], nullptr, 0, 0, 0};
 	constexpr uint32_t kPer = kMaxVecPerChunk / kCdWarps; // vectors of a warp: warp, warp + kCdWarps
 	uint32_t           listed[kPer];
 	auto clear = [&](uint32_t words) { // of the table
@@ -779,8 +765,8 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 				for (uint32_t i = 0; i < 4; ++i) {
 					T          x;
 					const bool start = row(v, r0 + i, &x);
-					uint32_t   place, tag;
-					cd_hash(x, &place, &tag);
+					uint32_t   place, other;
+					cd_hash(x, &place, &other);
 					const uint32_t b = place >> 12;
 					if (start && ((atomicOr(filter + (b >> 5), 1u << (b & 31u)) >> (b & 31u)) & 1u)) {
 						atomicOr(marks + (b >> 7), 1u << ((b >> 2) & 31u));
@@ -803,19 +789,20 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 		if (found) {
 			clear(kCdUniqueSlots);
 			if (tid == 0) { S.count = 0; }
+			Q.left = kCdLooks;
 			__syncthreads();
 #pragma unroll
 			for (uint32_t j = 0; j < kPer; ++j) {
 				const uint32_t v = warp + j * kCdWarps;
-				uint32_t       lo = ~0u, hi = 0u, steps = 0;
+				uint32_t       lo = ~0u, hi = 0u;
 				Q.list = slots + v * 1024;
 				Q.q = Q.n = 0;
 				for (uint32_t r = 0; r < 32 && v < nv; ++r) {
 					if (__any_sync(0xFFFFFFFFu, *over != 0)) { break; } // one answer for the whole warp
 					T          x;
 					const bool start = row(v, r, &x);
-					uint32_t   place, tag;
-					cd_hash(x, &place, &tag);
+					uint32_t   place, other;
+					cd_hash(x, &place, &other);
 					const uint32_t pos  = v * 1024 + r * 32 + lane;
 					const bool     mark = start && ((marks[place >> 19] >> ((place >> 14) & 31u)) & 1u);
 					const uint32_t only = __ballot_sync(0xFFFFFFFFu, start && !mark);
@@ -828,9 +815,12 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 						sw0 += __ldg(w0 + pos);
 						sw1 += __ldg(w1 + pos);
 					}
-					Q.push(mark, x, pos, __umulhi(place, kCdUniqueSlots), tag, lane);
+					Q.push(mark, x, pos, __umulhi(place, kCdUniqueSlots), cd_tag(other), lane);
 					uint32_t fresh = 0;
-					while ((Q.q >= 32 || (r == 31 && Q.q > 0)) && ++steps < kCdMaxSteps) { fresh += Q.pop(S.table, kCdUniqueSlots, vals, lane); }
+					if (!Q.drain(S.table, kCdUniqueSlots, vals, r == 31, lane, &fresh)) {
+						if (lane == 0) { S.spent = *over = 1; }
+						break;
+					}
 					if (lane == 0 && fresh && atomicAdd(&S.count, fresh) + fresh > kCdUniqueCap) { *over = 1; }
 				}
 				listed[j] = Q.n;
@@ -838,7 +828,6 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 					S.vrange[v][0] = lo;
 					S.vrange[v][1] = hi;
 				}
-				if (steps >= kCdMaxSteps && lane == 0) { atomicOr(a.status, STATUS_BAD_INDEX); }
 			}
 			__syncthreads();
 			found = S.over == 0;
@@ -846,13 +835,13 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 			if (found) { collect(kCdUniqueSlots); }
 		}
 	}
-	for (uint32_t parts_log = 0; !found; ++parts_log) {
+	for (uint32_t parts_log = 0; !found && (1u << parts_log) <= kCdMaxParts && S.spent == 0; ++parts_log) {
 		reset();
 		for (uint32_t part = 0; part < (1u << parts_log); ++part) {
 			clear(kCdSlots);
 			if (tid == 0) { S.count = S.over = 0; }
+			Q.left = kCdLooks;
 			__syncthreads();
-			uint32_t steps = 0;
 #pragma unroll
 			for (uint32_t j = 0; j < kPer; ++j) {
 				const uint32_t v    = warp + j * kCdWarps;
@@ -863,20 +852,22 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 					if (__any_sync(0xFFFFFFFFu, *over != 0)) { break; } // one answer for the whole warp
 					T        x;
 					bool     need = row(v, r, &x);
-					uint32_t place, tag;
-					cd_hash(x, &place, &tag);
-					if (parts_log) { need = need && (place >> (32 - parts_log)) == part; }
-					const uint32_t pos = v * 1024 + r * 32 + lane, s = __umulhi(place << parts_log, kCdSlots);
+					uint32_t place, other;
+					cd_hash(x, &place, &other);
+					need = need && cd_part(other, parts_log) == part;
+					const uint32_t pos = v * 1024 + r * 32 + lane, s = __umulhi(place, kCdSlots), tag = cd_tag(other);
 					uint32_t       fresh = 0;
 					bool           looked = true;
 					if (Q.q == 0 && __all_sync(0xFFFFFFFFu, need)) { // a full warp as it is
 						fresh = Q.look(S.table, kCdSlots, vals, true, x, pos, s, tag, lane);
-						++steps;
 					} else {
 						Q.push(need, x, pos, s, tag, lane);
 						looked = Q.q >= 32;
 					}
-					while ((Q.q >= 32 || (r == 31 && Q.q > 0)) && ++steps < kCdMaxSteps) { fresh += Q.pop(S.table, kCdSlots, vals, lane); }
+					if (!Q.drain(S.table, kCdSlots, vals, r == 31, lane, &fresh)) {
+						if (lane == 0) { S.spent = *over = 1; }
+						break;
+					}
 					++rows;
 					if (lane == 0 && (looked || r == 31)) {
 						// room left, and room for the chunk if the keys go on coming at this rate?
@@ -888,7 +879,6 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 				}
 				listed[j] = Q.n;
 			}
-			if (steps >= kCdMaxSteps && lane == 0) { atomicOr(a.status, STATUS_BAD_INDEX); }
 			__syncthreads();
 			const bool full = S.over != 0;
 			__syncthreads(); // S.over is read before it is cleared
@@ -896,10 +886,11 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 			collect(kCdSlots);
 			found = part + 1 == (1u << parts_log);
 		}
-		if (!found && (2u << parts_log) > kCdMaxParts) {
-			if (tid == 0) { atomicOr(a.status, STATUS_BAD_INDEX); } // never: 256 parts of 65,536 values
-			break;
-		}
+	}
+	if (!found) {
+		reset();
+		__syncthreads();
+		cd_sort<T>(vals, nv, slots, w0, w1, S);
 	}
 	if (w0) {
 		sw0 = warp_sum(sw0);

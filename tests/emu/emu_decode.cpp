@@ -3,6 +3,7 @@
 // harness fills the way the kernel's bulk copies would.  Used by tests/test_device_logic_emulated.py.
 #define FLS_HOST_EMULATION 1
 #include "fls_decode.cu"
+#include "fls_cd_queue.cuh"
 #include "fls_page.h"
 #include "fls_strings.cuh"
 #include "fls_b200.h"
@@ -275,4 +276,66 @@ extern "C" int emu_fsst_plain_total(const uint8_t* len, const uint8_t* vb, uint3
 	for (auto& x : th) { x.join(); }
 	*total = tot;
 	return plain;
+}
+
+// Hashes of the chunk dictionary (fls_cd_queue.cuh) of n keys of 32 or 64 bits.
+extern "C" void emu_cd_hash(int width, const uint8_t* keys, uint64_t n, uint32_t* place, uint32_t* other) {
+	for (uint64_t i = 0; i < n; ++i) {
+		if (width == 64) {
+			uint64_t x;
+			std::memcpy(&x, keys + 8 * i, 8);
+			sel::cd_hash(x, place + i, other + i);
+		} else {
+			uint32_t x;
+			std::memcpy(&x, keys + 4 * i, 4);
+			sel::cd_hash(x, place + i, other + i);
+		}
+	}
+}
+
+// One warp's queue over n_rows rows of 32 keys (need: which of them go in) and a table of n_slots slots, with `looks`
+// looks to spend, as k_chunk_dict fills it.  *n_keys: the new keys.  Returns
+// the most keys that were queued after a row, or -1 when the looks were spent, -2 when anything was written outside
+// the queue.
+extern "C" int emu_cd_queue(const uint64_t* keys, const uint8_t* need, uint32_t n_rows, uint32_t n_slots, uint32_t looks,
+                            uint32_t* n_keys) {
+	constexpr uint32_t    kQ = sel::kCdQueue, kPad = 64;
+	std::vector<uint32_t> table(n_slots, sel::kCdFree);
+	std::vector<uint64_t> key(kQ + 2 * kPad, 0xA5A5A5A5A5A5A5A5ull);
+	std::vector<uint16_t> pos(kQ + 2 * kPad, 0xA5A5), slot = pos, tag = pos, list(n_rows * 32 + kPad, 0);
+	std::barrier<>        bar(32);
+	EmuWarp               w {&bar, {}, {}};
+	std::vector<std::thread> th;
+	int                   most = 0;
+	bool                  spent = false;
+	uint32_t              total = 0;
+	for (uint32_t t = 0; t < 32; ++t) {
+		th.emplace_back([&, t] {
+			g_emu_warp = &w;
+			g_emu_lane = static_cast<int>(t);
+			sel::CdQueue<uint64_t> Q {key.data() + kPad, pos.data() + kPad, slot.data() + kPad, tag.data() + kPad, list.data(), 0, 0, looks};
+			uint32_t               fresh = 0;
+			for (uint32_t r = 0; r < n_rows; ++r) {
+				const uint32_t at = r * 32 + t;
+				uint32_t       place, other;
+				sel::cd_hash(keys[at], &place, &other);
+				const uint32_t s = static_cast<uint32_t>((static_cast<uint64_t>(place) * n_slots) >> 32);
+				Q.push(need[at] != 0, keys[at], at, s, sel::cd_tag(other), t);
+				if (t == 0 && static_cast<int>(Q.q) > most) { most = static_cast<int>(Q.q); }
+				if (!Q.drain(table.data(), n_slots, keys, r + 1 == n_rows, t, &fresh)) {
+					if (t == 0) { spent = true; }
+					break;
+				}
+			}
+			if (t == 0) { total = fresh; }
+		});
+	}
+	for (auto& x : th) { x.join(); }
+	*n_keys = total;
+	for (uint32_t i = 0; i < kPad; ++i) {
+		for (const uint32_t at : {i, kPad + kQ + i}) {
+			if (key[at] != 0xA5A5A5A5A5A5A5A5ull || pos[at] != 0xA5A5 || slot[at] != 0xA5A5 || tag[at] != 0xA5A5) { return -2; }
+		}
+	}
+	return spent ? -1 : most;
 }

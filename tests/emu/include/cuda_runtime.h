@@ -113,6 +113,15 @@ inline unsigned __ballot_sync(unsigned, bool p) {
 	return r;
 }
 inline int atomicOr(int* a, int v) { return __atomic_fetch_or(a, v, __ATOMIC_SEQ_CST); }
+inline unsigned atomicCAS(unsigned* a, unsigned c, unsigned v) {
+	__atomic_compare_exchange_n(a, &c, v, false, __ATOMIC_SEQ_CST, __ATOMIC_SEQ_CST);
+	return c;
+}
+inline unsigned atomicMin(unsigned* a, unsigned v) {
+	unsigned o = __atomic_load_n(a, __ATOMIC_SEQ_CST);
+	while (v < o && !__atomic_compare_exchange_n(a, &o, v, false, __ATOMIC_SEQ_CST, __ATOMIC_SEQ_CST)) {}
+	return o;
+}
 inline unsigned atomicOr(unsigned* a, unsigned v) { return __atomic_fetch_or(a, v, __ATOMIC_SEQ_CST); }
 template <class T>
 T __ldg(const T* p) {

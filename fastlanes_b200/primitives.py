@@ -122,8 +122,8 @@ def ffor(x, bw, base=None):
     total = torch.empty(2, dtype=torch.int64, device=x.device)
     check(lib.fls_gpu_pack_offsets(_ptr(bw), bw.numel(), w, _ptr(off), _ptr(total), _stream()), "pack_offsets")
     size, bad = total.tolist()
-    # every byte is written by the packing, except for vectors of an impossible width
-    alloc = torch.zeros if bad or size < 16 else torch.empty
+    # every byte is written by the packing, except for vectors of an impossible width and widths without a vector
+    alloc = torch.zeros if bad or size < 16 or bw.numel() != n else torch.empty
     out = alloc(max(size, 16), dtype=torch.uint8, device=x.device)
     check(_FN["ffor"][w](_ptr(x), _ptr(out), _ptr(bw), _ptr(base), _ptr(off), n, _stream()),
           "ffor")

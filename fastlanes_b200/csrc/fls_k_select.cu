@@ -1026,11 +1026,11 @@ __device__ __forceinline__ uint64_t str_load8_inside(const StrCol& c, uint64_t p
 // row, the exact figure the wizard's sizes need; rs > 1, the learned selector's features: the other rows'
 // compressed lengths are written as 0 and the vector's sum is scaled by rs).  The CTAs go through the columns one
 // after the other, a warp taking units of kStrUnit rows.
-//   memo     rows whose hash another row of the column had before (dictionary-like columns: nearly all) take its
-//            compressed length from the column's part of a table in global memory, 64-bit entries of the hash and
-//            the length, cleared for every call; rows are told apart by hash and length.  A first launch over every
-//            `stride`-th vector fills it: all units start at once, so that without it nothing would be found.  With
-//            one table for all columns, those whose rows all differ would push the others' entries out;
+//   memo     rows that another row of the column equals (dictionary-like columns: nearly all) take its compressed
+//            length from the column's part of a table in global memory, cleared for every call: an entry says where
+//            a row's bytes are, and both rows' bytes are compared.  A first launch over every `stride`-th vector fills
+//            it: all units start at once, so that without it nothing would be found.  With one table for all columns,
+//            those whose rows all differ would push the others' entries out;
 //   match    greedy matching looks at the next two bytes in a 64 KB table in shared memory (what they start: nothing,
 //            a one- or two-byte symbol, or a group of longer ones), so that only the few symbols of one group are
 //            compared, where the symbols sharing a first byte were walked one after the other;
@@ -1046,7 +1046,6 @@ constexpr uint32_t kStrFillPer = 5, kStrFillUnit = 1024 >> kStrFillPer; // one a
 // log2 of a column's memo entries: as many as the largest column has rows, at most 1 MB, and (down to the least) all
 // columns' at most 8 MB, which is cleared in a few microseconds and stays in L2
 constexpr uint32_t kStrMemoMin = 13, kStrMemoMax = 17, kStrMemoAll = 20;
-constexpr uint32_t kStrMemoLen = 4094;       // longest compressed length an entry holds
 struct StrRowsSmem {
 	// by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g; behind them, by a row's last byte
 	uint8_t  pair[65536 + 256];
@@ -1078,10 +1077,11 @@ __device__ __forceinline__ uint32_t str_next_code(const StrRowsSmem& S, uint64_t
 	return what == 2 ? 2u : 1u;
 }
 
-__device__ __forceinline__ uint64_t str_hash_step(uint64_t h, uint64_t x, uint64_t left) {
-	const uint64_t k = left >= 8 ? x : (x & ((1ull << (8 * left)) - 1));
-	return str_mix(h ^ k) + 0x9E3779B97F4A7C15ull;
+// the string bytes in x, `left` of them (at least one) still in the row, zero past them
+__device__ __forceinline__ uint64_t str_row_bytes(uint64_t x, uint64_t left) {
+	return left >= 8 ? x : (x & ((1ull << (8 * left)) - 1));
 }
+__device__ __forceinline__ uint64_t str_hash_step(uint64_t h, uint64_t x) { return str_mix(h ^ x) + 0x9E3779B97F4A7C15ull; }
 constexpr uint64_t kStrHashSeed = 0x243F6A8885A308D3ull;
 
 // A unit whose offsets do not fit 31 bits from its first one (rows of gigabytes, or corrupt offsets), row by row.
@@ -1090,7 +1090,7 @@ __device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c
 	for (uint32_t j = lane; j < unit; j += 32) {
 		const uint64_t r = r0 + j, b = __ldg(c.offsets + r), e = __ldg(c.offsets + r + 1), m = e >= b ? e - b : 0;
 		uint64_t       h = kStrHashSeed ^ m;
-		for (uint64_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_load8(c, b + p), m - p); }
+		for (uint64_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_row_bytes(str_load8(c, b + p), m - p)); }
 		uint32_t cl = 0;
 		if ((r & 1023u) % rs == 0) {
 			for (uint64_t p = 0; p < m;) {
@@ -1106,16 +1106,22 @@ __device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c
 	}
 }
 
-// A row's memo entry: its place (a pair of entries, told by bits - 1, at least 12, of the hash), and the entry without the
-// length (the low 12 bits hold length + 1); place and entry together hold all 64 bits of the hash, mixed with the
-// row's own length (short rows of different lengths can share a hash: "a" and "b\0" do).  In pairs, because strings
-// that share a place push each other out for good, and a warp waits for its few rows that miss: 4,096 strings in 64 Ki
-// single entries, of which 6 % share one, 83 + 667 us for 7.4 M rows of 12 columns, 81 + 541 us so.
-__device__ __forceinline__ uint64_t str_memo_key(uint64_t h, uint32_t m, uint32_t bits, uint32_t* at) {
-	h ^= m * 0x9E3779B97F4A7C15ull;
-	*at = static_cast<uint32_t>(h) & ((1u << (bits - 1)) - 1u);
-	return h & ~0xFFFull;
+// A memo entry: a row's compressed length + 1 (0: no entry), its length, where it starts in the column's bytes, and 8 bits
+// of its hash, so that few other rows' bytes are looked at.  Rows of more bytes, or further in, have none.  The place is
+// a pair of entries, told by the low bits - 1 bits of the hash: strings that share a place push each other out for good,
+// and a warp waits for its few rows that miss: 4,096 strings in 64 Ki single entries, of which 6 % share one, 83 + 667 us
+// for 7.4 M rows of 12 columns, 81 + 541 us so.
+constexpr uint32_t kStrMemoClenBits = 11, kStrMemoLenBits = 11, kStrMemoAtBits = 34;
+constexpr uint32_t kStrMemoClen = (1u << kStrMemoClenBits) - 2, kStrMemoLen = (1u << kStrMemoLenBits) - 1; // at most
+constexpr uint32_t kStrMemoAtPos = kStrMemoClenBits + kStrMemoLenBits, kStrMemoTagPos = kStrMemoAtPos + kStrMemoAtBits;
+constexpr uint64_t kStrMemoAtEnd = 1ull << kStrMemoAtBits;
+static_assert(kStrMemoTagPos == 56, "8 bits of the hash");
+
+// what an entry of a row of hash h and length m has beside the row's place and compressed length
+__device__ __forceinline__ uint64_t str_memo_key(uint64_t h, uint32_t m) {
+	return (h & ~((1ull << kStrMemoTagPos) - 1)) | (static_cast<uint64_t>(m) << kStrMemoClenBits);
 }
+constexpr uint64_t kStrMemoKey = ~((1ull << kStrMemoTagPos) - 1) | (((1ull << kStrMemoLenBits) - 1) << kStrMemoClenBits);
 
 struct StrRowsArgs {
 	const StrCol* cols;
@@ -1159,6 +1165,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 		if (mine >= u1 + kStrWarps - 1) { continue; }
 		const StrCol      c    = a.cols[col];
 		ulonglong2* const memo = reinterpret_cast<ulonglong2*>(a.memo + (static_cast<uint64_t>(col) << a.memo_bits));
+		const uint32_t    pairs = (1u << (a.memo_bits - 1)) - 1;
 		__syncthreads(); // the previous column's table is read to the end
 		for (uint32_t k = tid; k < sizeof(StrTab) / 4; k += nt) {
 			reinterpret_cast<uint32_t*>(&S.t)[k] = __ldg(reinterpret_cast<const uint32_t*>(c.tab) + k);
@@ -1198,43 +1205,62 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 					const uint32_t limit = room < 12 ? 0u : room < (1u << 31) ? static_cast<uint32_t>(room) - 11 : 1u << 31;
 					auto load8 = [&](uint32_t p, bool inside) { return inside ? str_load8_inside(c, o0 + p) : str_load8(c, o0 + p); };
 					uint32_t todo = 0;
-					uint32_t at = 0, row = 0, ask = 0; // the look into the memo of the row before
+					uint32_t row = 0, ask = 0; // the look into the memo of the row before
 					uint64_t key = 0;
 					ulonglong2 seen = make_ulonglong2(0, 0);
 					for (uint32_t j = lane; j < unit + 32; j += 32) {
-						uint32_t row_next = j, ask_next = 0, at_next = 0;
+						uint32_t row_next = j, ask_next = 0;
 						uint64_t key_next = 0;
 						ulonglong2 seen_next = make_ulonglong2(0, 0);
 						if (j < unit) {
 							const uint32_t b = off[j], e = off[j + 1], m = e >= b ? e - b : 0;
 							const bool     inside = e < limit;
 							uint64_t       h = kStrHashSeed ^ m;
-							for (uint32_t p = 0; p < m; p += 8) { h = str_hash_step(h, load8(b + p, inside), m - p); }
+							for (uint32_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_row_bytes(load8(b + p, inside), m - p)); }
 							const uint64_t r = r0 + j;
 							c.hash[r]        = h;
 							c.len[r]         = m;
 							sl += m;
 							if ((r & 1023u) % rs == 0) {
-								key_next  = str_memo_key(h, m, a.memo_bits, &at_next);
-								seen_next = __ldcg(memo + at_next);
-								ask_next  = 1;
+								ask_next = m <= kStrMemoLen && e <= room ? 1u : 2u; // 2: no entry, to be matched
+								if (ask_next == 1) {
+									key_next  = str_memo_key(h, m);
+									seen_next = __ldcg(memo + (static_cast<uint32_t>(h) & pairs));
+								}
 							} else {
 								c.clen[r] = 0;
 							}
 						}
-						const uint64_t found = (seen.x & ~0xFFFull) == key ? seen.x : seen.y;
-						const bool     hit   = ask && (found & ~0xFFFull) == key && (found & 0xFFFu) != 0;
+						const uint64_t found = (seen.x & kStrMemoKey) == key ? seen.x : seen.y;
+						bool           hit   = ask == 1 && found != 0 && (found & kStrMemoKey) == key;
+						if (hit) { // the same bytes?
+							const uint64_t q = (found >> kStrMemoAtPos) & (kStrMemoAtEnd - 1);
+							const uint32_t b = off[row], m = static_cast<uint32_t>(key >> kStrMemoClenBits) & kStrMemoLen;
+							const bool     inside = b + m < limit && q + m + 12 <= c.n_bytes;
+							if (inside) { // two words a step: their loads are in flight together
+								for (uint32_t p = 0; p < m && hit; p += 16) {
+									const uint32_t p1 = p + 8 < m ? p + 8 : p;
+									const uint64_t x0 = str_load8_inside(c, o0 + b + p), y0 = str_load8_inside(c, q + p);
+									const uint64_t x1 = str_load8_inside(c, o0 + b + p1), y1 = str_load8_inside(c, q + p1);
+									hit = (str_row_bytes(x0 ^ y0, m - p) | str_row_bytes(x1 ^ y1, m - p1)) == 0;
+								}
+							} else {
+								for (uint32_t p = 0; p < m && hit; p += 8) {
+									hit = str_row_bytes(str_load8(c, o0 + b + p) ^ str_load8(c, q + p), m - p) == 0;
+								}
+							}
+						}
 						if (hit) {
-							const uint32_t cl = static_cast<uint32_t>(found & 0xFFFu) - 1;
+							const uint32_t cl = static_cast<uint32_t>(found & ((1u << kStrMemoClenBits) - 1)) - 1;
 							c.clen[r0 + row]  = cl;
 							sc += cl;
 						}
 						const bool     miss = ask && !hit;
-						const uint32_t slot = seen.x == 0 ? 0u : seen.y == 0 ? 1u : static_cast<uint32_t>(key >> 40) & 1u;
+						const uint32_t slot = seen.x == 0 ? 0u : seen.y == 0 ? 1u : static_cast<uint32_t>(key >> 57) & 1u;
 						const uint32_t m    = __ballot_sync(0xFFFFFFFFu, miss);
 						if (miss) { list[todo + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(row | slot << 15); }
 						todo += __popc(m);
-						row = row_next, ask = ask_next, at = at_next, key = key_next, seen = seen_next;
+						row = row_next, ask = ask_next, key = key_next, seen = seen_next;
 					}
 					__syncwarp();
 					uint32_t next = 0, j = 0, p = 0, left = 0, cl = 0;
@@ -1298,10 +1324,12 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 						const uint32_t i = list[k] & 0x7FFFu;
 						const uint64_t r = r0 + i;
 						const uint32_t l = c.clen[r];
-						const uint32_t b = off[i], e = off[i + 1];
-						key              = str_memo_key(c.hash[r], e >= b ? e - b : 0, a.memo_bits, &at);
-						if (l <= kStrMemoLen) { // into the entry of the pair that was free, or over one of the two
-							__stcg(reinterpret_cast<uint64_t*>(memo + at) + (list[k] >> 15), key | (l + 1));
+						const uint32_t b = off[i], e = off[i + 1], n = e >= b ? e - b : 0;
+						if (n <= kStrMemoLen && l <= kStrMemoClen && e <= room && o0 + b < kStrMemoAtEnd) {
+							// into the entry of the pair that was free, or over one of the two
+							const uint64_t h = c.hash[r];
+							__stcg(reinterpret_cast<uint64_t*>(memo + (static_cast<uint32_t>(h) & pairs)) + (list[k] >> 15),
+							       str_memo_key(h, n) | ((o0 + b) << kStrMemoAtPos) | (l + 1));
 						}
 					}
 				}

@@ -1083,14 +1083,24 @@ __device__ __forceinline__ uint64_t str_row_bytes(uint64_t x, uint64_t left) {
 }
 __device__ __forceinline__ uint64_t str_hash_step(uint64_t h, uint64_t x) { return str_mix(h ^ x) + 0x9E3779B97F4A7C15ull; }
 constexpr uint64_t kStrHashSeed = 0x243F6A8885A308D3ull;
+// The hash of a row of m bytes whose words gave h, the last one x.  A row that ends in a zero byte has its length mixed in
+// once more: the length that h starts from can cancel against a first byte, and a shorter row's words are the same then
+// ("a" and "b\0" shared a hash).  (Another hash for all rows would change their columns' statistics.)
+__device__ __forceinline__ uint64_t str_hash_end(uint64_t h, uint64_t x, uint64_t m) {
+	return m && (x >> (8 * ((m - 1) & 7u)) & 0xFFu) == 0 ? str_mix(h + m * 0x9E3779B97F4A7C15ull) : h;
+}
 
 // A unit whose offsets do not fit 31 bits from its first one (rows of gigabytes, or corrupt offsets), row by row.
 __device__ __noinline__ void str_unit_wide(const StrRowsSmem& S, const StrCol& c, uint64_t r0, uint32_t unit, uint32_t rs,
                                            uint32_t lane, uint64_t* sl, uint64_t* sc) {
 	for (uint32_t j = lane; j < unit; j += 32) {
 		const uint64_t r = r0 + j, b = __ldg(c.offsets + r), e = __ldg(c.offsets + r + 1), m = e >= b ? e - b : 0;
-		uint64_t       h = kStrHashSeed ^ m;
-		for (uint64_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_row_bytes(str_load8(c, b + p), m - p)); }
+		uint64_t       h = kStrHashSeed ^ m, x = 0;
+		for (uint64_t p = 0; p < m; p += 8) {
+			x = str_row_bytes(str_load8(c, b + p), m - p);
+			h = str_hash_step(h, x);
+		}
+		h = str_hash_end(h, x, m);
 		uint32_t cl = 0;
 		if ((r & 1023u) % rs == 0) {
 			for (uint64_t p = 0; p < m;) {
@@ -1216,7 +1226,12 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 							const uint32_t b = off[j], e = off[j + 1], m = e >= b ? e - b : 0;
 							const bool     inside = e < limit;
 							uint64_t       h = kStrHashSeed ^ m;
-							for (uint32_t p = 0; p < m; p += 8) { h = str_hash_step(h, str_row_bytes(load8(b + p, inside), m - p)); }
+							uint64_t       x = 0;
+							for (uint32_t p = 0; p < m; p += 8) {
+								x = str_row_bytes(load8(b + p, inside), m - p);
+								h = str_hash_step(h, x);
+							}
+							h = str_hash_end(h, x, m);
 							const uint64_t r = r0 + j;
 							c.hash[r]        = h;
 							c.len[r]         = m;

@@ -14,6 +14,7 @@
 #include "fls_b200.h"
 #include "fls_cd_queue.cuh"
 #include "fls_select.h"
+#include "fls_smem_limit.h"
 #include "fls_strings.cuh"
 #include "fls_strplan.h"
 
@@ -1364,14 +1365,11 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_items, uint64_t* vlen, uint64_t* vclen,
                             uint32_t rs, uint64_t* memo, uint32_t memo_bits, uint64_t n_cols, cudaStream_t s) {
 	Device* d = current_device();
-	if (!d || d->ordinal < 0 || d->ordinal >= 64) { return cudaErrorInvalidDevice; }
-	static bool set[64] = {};
-	if (!set[d->ordinal]) {
-		const cudaError_t e = cudaFuncSetAttribute(k_str_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(StrRowsSmem));
-		if (e != cudaSuccess) { return e; }
-		set[d->ordinal] = true;
-	}
-	cudaError_t e = cudaMemsetAsync(memo, 0, (n_cols << memo_bits) * 8, s);
+	if (!d) { return cudaErrorInvalidDevice; }
+	static SmemLimit limit;
+	cudaError_t      e = limit.need(reinterpret_cast<const void*>(k_str_rows), sizeof(StrRowsSmem));
+	if (e != cudaSuccess) { return e; }
+	e = cudaMemsetAsync(memo, 0, (n_cols << memo_bits) * 8, s);
 	if (e == cudaSuccess && vlen) { e = cudaMemsetAsync(vlen, 0, n_items * 8, s); }
 	if (e == cudaSuccess && vclen) { e = cudaMemsetAsync(vclen, 0, n_items * 8, s); }
 	if (e != cudaSuccess) { return e; }
@@ -1888,13 +1886,10 @@ cudaError_t forward(cudaStream_t s, const float* params, const float* X, uint64_
 // class probabilities of n rows
 cudaError_t probabilities(cudaStream_t s, const float* params, const float* X, uint64_t n, float* P) {
 	Device* d = current_device();
-	if (!d || d->ordinal < 0 || d->ordinal >= 64) { return cudaErrorInvalidDevice; }
-	static bool set[64] = {};
-	if (!set[d->ordinal]) {
-		const cudaError_t e = cudaFuncSetAttribute(k_mlp, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(MlpSmem));
-		if (e != cudaSuccess) { return e; }
-		set[d->ordinal] = true;
-	}
+	if (!d) { return cudaErrorInvalidDevice; }
+	static SmemLimit  limit;
+	const cudaError_t e = limit.need(reinterpret_cast<const void*>(k_mlp), sizeof(MlpSmem));
+	if (e != cudaSuccess) { return e; }
 	const uint64_t tiles = (n + kMlpRows - 1) / kMlpRows;
 	k_mlp<<<static_cast<unsigned>(std::min<uint64_t>(tiles, d->sm_count)), 256, sizeof(MlpSmem), s>>>(params, X, n, P);
 	++launch_counter();
@@ -1938,12 +1933,9 @@ int grid_for(uint64_t warps_needed) {
 }
 
 cudaError_t launch_features(const ItemArgs& a, float* feat, cudaStream_t s) {
-	static bool set = false;
-	if (!set) {
-		const cudaError_t e = cudaFuncSetAttribute(k_features, cudaFuncAttributeMaxDynamicSharedMemorySize, kFeatSmem);
-		if (e != cudaSuccess) { return e; }
-		set = true;
-	}
+	static SmemLimit  limit;
+	const cudaError_t e = limit.need(reinterpret_cast<const void*>(k_features), kFeatSmem);
+	if (e != cudaSuccess) { return e; }
 	k_features<<<grid_for(a.n_items), kWarps * 32, kFeatSmem, s>>>(a, feat);
 	++launch_counter();
 	return cudaGetLastError();
@@ -2080,14 +2072,8 @@ int wizard_run(fls_sel_plan* p, const std::vector<uint32_t>& subset, uint64_t* d
 	++launch_counter();
 	// dictionary of every chunk: one CTA per chunk, tables in shared memory
 	{
-		static bool attr[64] = {};
-		if (dev->ordinal < 0 || dev->ordinal >= 64) { return FLS_ERR_CUDA; }
-		if (!attr[dev->ordinal]) {
-			if (cudaFuncSetAttribute(k_chunk_dict, cudaFuncAttributeMaxDynamicSharedMemorySize, sizeof(ChunkDictSmem)) != cudaSuccess) {
-				return FLS_ERR_CUDA;
-			}
-			attr[dev->ordinal] = true;
-		}
+		static SmemLimit limit;
+		if (limit.need(reinterpret_cast<const void*>(k_chunk_dict), sizeof(ChunkDictSmem)) != cudaSuccess) { return FLS_ERR_CUDA; }
 		// one CTA per SM, each with its own slot scratch
 		const uint32_t grid = static_cast<uint32_t>(std::min<size_t>(chunks.size(), static_cast<size_t>(dev->sm_count)));
 		if (!p->gtab.need(kCdGBytes * grid + 4)) { return FLS_ERR_CUDA; }

@@ -13,6 +13,7 @@
 #include "fls_decode.cu"
 #include "fls_strings.cuh"
 #include "fls_runtime.h"
+#include "fls_smem_limit.h"
 #include "fls_strplan.h"
 #include "fls_b200.h"
 
@@ -932,26 +933,20 @@ cudaError_t launch_dict_align(const uint8_t* bytes, const uint32_t* rows, const 
 }
 
 // Launch one pass of kernel fn over the column's vectors with `warps` warps per CTA and as many CTAs per SM as
-// shared memory allows (no more CTAs than there are vectors for their warps).  *set / *mu: the kernel's dynamic
-// shared-memory limit set so far and its lock.  sm_count 0: the SM count of the library's per-device state.
+// shared memory allows (no more CTAs than there are vectors for their warps).  limit: the kernel's.  sm_count 0: the SM
+// count of the library's per-device state.
 template <class F>
-static cudaError_t launch_pass(F fn, uint32_t* set, std::mutex* mu, const StrArgs& a, int warps, uint32_t dyn_smem,
-                               cudaStream_t s, int sm_count) {
-	{
-		std::lock_guard<std::mutex> lk(*mu);
-		if (dyn_smem > *set) {
-			const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_smem);
-			if (e != cudaSuccess) { return e; }
-			*set = dyn_smem;
-		}
-	}
+static cudaError_t launch_pass(F fn, SmemLimit* limit, const StrArgs& a, int warps, uint32_t dyn_smem, cudaStream_t s,
+                               int sm_count) {
+	cudaError_t e = limit->need(reinterpret_cast<const void*>(fn), dyn_smem);
+	if (e != cudaSuccess) { return e; }
 	if (sm_count <= 0) {
 		const Device* dev = current_device();
 		if (!dev) { return cudaErrorUnknown; }
 		sm_count = dev->sm_count;
 	}
-	int         per_sm = 0;
-	cudaError_t e      = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, dyn_smem);
+	int per_sm = 0;
+	e          = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, dyn_smem);
 	if (e != cudaSuccess) { return e; }
 	if (per_sm < 1) { return cudaErrorInvalidConfiguration; }
 	const uint64_t need = (a.col.n_vec + warps - 1) / warps;
@@ -965,16 +960,14 @@ static cudaError_t launch_pass(F fn, uint32_t* set, std::mutex* mu, const StrArg
 
 template <int PASS, int KIND, int SM, bool R16 = false>
 static cudaError_t launch_str_kernel(const StrArgs& a, int warps, uint32_t dyn_smem, cudaStream_t s, int sm_count) {
-	static std::mutex mu;
-	static uint32_t   set = 0;
-	return launch_pass(k_str_pass<PASS, KIND, SM, R16>, &set, &mu, a, warps, dyn_smem, s, sm_count);
+	static SmemLimit limit;
+	return launch_pass(k_str_pass<PASS, KIND, SM, R16>, &limit, a, warps, dyn_smem, s, sm_count);
 }
 
 template <int PASS, int KIND>
 static cudaError_t launch_stream_kernel(const StrArgs& a, int warps, uint32_t dyn_smem, cudaStream_t s, int sm_count) {
-	static std::mutex mu;
-	static uint32_t   set = 0;
-	return launch_pass(k_stream_pass<PASS, KIND>, &set, &mu, a, warps, dyn_smem, s, sm_count);
+	static SmemLimit limit;
+	return launch_pass(k_stream_pass<PASS, KIND>, &limit, a, warps, dyn_smem, s, sm_count);
 }
 
 cudaError_t launch_str_lengths(const StrArgs& a, int sm_count, cudaStream_t s) {
@@ -998,24 +991,17 @@ uint32_t dict_pass_smem_per_warp(bool rows16) { return str_rows_bytes(rows16) + 
 
 template <bool R16, bool SMDICT>
 static cudaError_t launch_dict_pass_t(const StrSetArgs& a, int warps, uint32_t dyn_smem, cudaStream_t s, int sm_count) {
-	auto* const       fn = k_dict_pass<R16, SMDICT>;
-	static std::mutex mu;
-	static uint32_t   set = 0;
-	{
-		std::lock_guard<std::mutex> lk(mu);
-		if (dyn_smem > set) {
-			const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, dyn_smem);
-			if (e != cudaSuccess) { return e; }
-			set = dyn_smem;
-		}
-	}
+	auto* const      fn = k_dict_pass<R16, SMDICT>;
+	static SmemLimit limit;
+	cudaError_t      e = limit.need(reinterpret_cast<const void*>(fn), dyn_smem);
+	if (e != cudaSuccess) { return e; }
 	if (sm_count <= 0) {
 		const Device* dev = current_device();
 		if (!dev) { return cudaErrorUnknown; }
 		sm_count = dev->sm_count;
 	}
-	int         per_sm = 0;
-	cudaError_t e      = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, dyn_smem);
+	int per_sm = 0;
+	e          = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, warps * 32, dyn_smem);
 	if (e != cudaSuccess) { return e; }
 	if (per_sm < 1) { return cudaErrorInvalidConfiguration; }
 	// at most a CTA a vector; fewer vectors than warps: so many warps of each CTA take one
@@ -1047,16 +1033,9 @@ static cudaError_t launch_stream_single_t(const StrArgs& a, uint64_t* lb, cudaSt
 	auto* const        fn    = k_stream_single<KIND>;
 	constexpr int      warps = kStrMaxWarps;
 	constexpr uint32_t smem  = warps * kStreamSinglePerWarp;
-	static std::mutex  mu;
-	static bool        set = false;
-	{
-		std::lock_guard<std::mutex> lk(mu);
-		if (!set) {
-			const cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-			if (e != cudaSuccess) { return e; }
-			set = true;
-		}
-	}
+	static SmemLimit   limit;
+	const cudaError_t  e = limit.need(reinterpret_cast<const void*>(fn), smem);
+	if (e != cudaSuccess) { return e; }
 	if (sm_count <= 0) {
 		const Device* dev = current_device();
 		if (!dev) { return cudaErrorUnknown; }

@@ -5,6 +5,7 @@
 #include "fls_decode.cu"
 #include "fls_cd_queue.cuh"
 #include "fls_page.h"
+#include "fls_smem_limit.h"
 #include "fls_strings.cuh"
 #include "fls_b200.h"
 
@@ -338,4 +339,19 @@ extern "C" int emu_cd_queue(const uint64_t* keys, const uint8_t* need, uint32_t 
 		}
 	}
 	return spent ? -1 : most;
+}
+
+// A kernel's shared-memory limit (fls_smem_limit.h) over n launches on the given devices of the given sizes: asked[i] is
+// the limit the runtime was asked to set before launch i (0: it was not asked).
+static int g_emu_device, g_emu_limit;
+cudaError_t cudaGetDevice(int* dev) { *dev = g_emu_device; return cudaSuccess; }
+cudaError_t cudaFuncSetAttribute(const void*, int, int value) { g_emu_limit = value; return cudaSuccess; }
+extern "C" void emu_smem_limit(const int* device, const uint32_t* bytes, int n, int* asked, int* error) {
+	SmemLimit limit;
+	for (int i = 0; i < n; ++i) {
+		g_emu_device = device[i];
+		g_emu_limit  = 0;
+		error[i]     = limit.need(nullptr, bytes[i]);
+		asked[i]     = g_emu_limit;
+	}
 }

@@ -16,6 +16,10 @@
 typedef int           cudaError_t;
 typedef struct CUst_* cudaStream_t;
 #define cudaSuccess 0
+#define cudaErrorInvalidDevice 101
+enum { cudaFuncAttributeMaxDynamicSharedMemorySize = 8 };
+cudaError_t cudaGetDevice(int* dev);                                 // the test's device
+cudaError_t cudaFuncSetAttribute(const void* fn, int attr, int value); // counted
 
 struct uint2 {
 	uint32_t x, y;

@@ -368,7 +368,7 @@ int fls_string_plan_create(const uint8_t* d_page, uint64_t page_size, const uint
 		}
 		p->sp_warps = static_cast<int>(sw < kStrMaxWarps ? sw : kStrMaxWarps);
 		p->sp_smem  = static_cast<uint32_t>(p->sp_warps * pw + (p->sp_dict_cap ? d8 + tab : 0u));
-		if (!p->dargs.alloc(1) || !p->lb.alloc(1ull + pi.vec_c) ||
+		if (!p->dargs.alloc(1) || !p->lb.alloc(2ull + pi.vec_c) ||
 		    cudaMemcpy(p->dargs.p, &a, sizeof(StrArgs), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return FLS_ERR_CUDA;
 		}
@@ -414,7 +414,7 @@ int fls_string_plan_measure(fls_string_plan* p, uint64_t* n_bytes, fls_stream_t 
 static int single_pass_decode(const fls_string_plan* p, uint32_t* d_offsets, uint8_t* d_bytes, uint64_t cap,
                               cudaStream_t s) {
 	const uint32_t n_vec = p->args.col.n_vec;
-	if (cudaMemsetAsync(p->lb.p, 0, 8ull * (1 + n_vec), s) != cudaSuccess) { return FLS_ERR_CUDA; }
+	if (cudaMemsetAsync(p->lb.p, 0, 8ull * (2 + n_vec), s) != cudaSuccess) { return FLS_ERR_CUDA; }
 	StrSetArgs x {};
 	x.cols        = p->dargs.p;
 	x.n_cols      = 1;
@@ -478,7 +478,8 @@ int fls_string_plan_destroy(fls_string_plan* p) {
 struct fls_string_set {
 	std::vector<StrArgs> args;     // every column's arguments: item_base, and the outputs once bound
 	DevArr<StrArgs>      cols;     // the same in device memory
-	DevArr<uint64_t>     lb;       // a ticket per column + one look-back word per vector of every column
+	DevArr<uint64_t>     first;    // every column's first vector among all, and their number
+	DevArr<uint64_t>     lb;       // the cursor, a ticket per column, one look-back word per vector of every column
 	uint64_t             n_items  = 0;
 	int                  warps    = 0;
 	uint32_t             smem = 0, dict_cap = 0, tab_cap = 0;
@@ -492,12 +493,14 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 	if (!out || !plans || n == 0) { return FLS_ERR_ARG; }
 	*out = nullptr;
 	std::unique_ptr<fls_string_set> set(new fls_string_set());
-	uint64_t dict_max = 0, tab_max = 0;
+	uint64_t              dict_max = 0, tab_max = 0;
+	std::vector<uint64_t> first;
 	for (uint32_t i = 0; i < n; ++i) {
 		if (!plans[i]) { return FLS_ERR_ARG; }
 		if (!plans[i]->single) { return FLS_ERR_UNSUPPORTED; } // DICT pages with a packed row table only
 		StrArgs a   = plans[i]->args;
 		a.item_base = set->n_items;
+		first.push_back(set->n_items);
 		set->args.push_back(a);
 		set->n_items += a.col.n_vec;
 		set->rows16 = set->rows16 && a.rows16;
@@ -516,7 +519,11 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 	}
 	set->warps = static_cast<int>(w < kStrMaxWarps ? w : kStrMaxWarps);
 	set->smem  = static_cast<uint32_t>(set->warps * pw + (set->dict_cap ? dict_max + tab : 0u));
-	if (!set->cols.alloc(n) || !set->lb.alloc(n + set->n_items)) { return FLS_ERR_CUDA; }
+	first.push_back(set->n_items);
+	if (!set->cols.alloc(n) || !set->first.alloc(first.size()) || !set->lb.alloc(1 + n + set->n_items) ||
+	    cudaMemcpy(set->first.p, first.data(), 8 * first.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+		return FLS_ERR_CUDA;
+	}
 	*out = set.release();
 	return FLS_OK;
 }
@@ -544,11 +551,12 @@ int fls_string_set_bind(fls_string_set* set, uint32_t* const* d_offsets, uint8_t
 int fls_string_set_decode(const fls_string_set* set, fls_stream_t stream) {
 	if (!set || !set->bound) { return FLS_ERR_ARG; }
 	cudaStream_t s = static_cast<cudaStream_t>(stream);
-	if (cudaMemsetAsync(set->lb.p, 0, 8ull * (set->args.size() + set->n_items), s) != cudaSuccess) { return FLS_ERR_CUDA; }
+	if (cudaMemsetAsync(set->lb.p, 0, 8ull * (1 + set->args.size() + set->n_items), s) != cudaSuccess) { return FLS_ERR_CUDA; }
 	StrSetArgs x {};
 	x.cols      = set->cols.p;
 	x.n_cols    = static_cast<uint32_t>(set->args.size());
 	x.n_items   = set->n_items;
+	x.first     = set->first.p;
 	x.flags     = set->lb.p;
 	x.status    = set->status;
 	x.dict_cap  = set->dict_cap;

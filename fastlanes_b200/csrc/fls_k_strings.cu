@@ -711,29 +711,19 @@ __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const u
 	return vpos;
 }
 
-// The column a CTA starts with: the one that holds its share of all vectors' first (warp 0).
-__device__ __forceinline__ uint32_t first_column(const StrSetArgs& s, uint32_t lane) {
-	const uint64_t x = s.n_items * blockIdx.x / gridDim.x;
-	uint32_t       c = 0;
-	for (uint32_t i = lane; i < s.n_cols; i += 32) {
-		if (s.cols[i].item_base <= x && s.cols[i].col.n_vec) { c = i; }
+// The next column of a CTA (warp 0; n_cols: none).  With as many columns as CTAs or more, a cursor hands them out in
+// order, and a CTA that finds it at the end helps with the fullest column.
+__device__ __forceinline__ uint32_t next_column(const StrSetArgs& s, uint32_t lane, bool first) {
+	if (s.n_cols == 1) { return first ? 0u : 1u; }
+	if (s.n_cols >= gridDim.x) {
+		unsigned long long c = 0;
+		if (lane == 0) { c = atomicAdd(reinterpret_cast<unsigned long long*>(s.flags), 1ull); }
+		c = __shfl_sync(0xFFFFFFFFu, c, 0);
+		if (c < s.n_cols) { return static_cast<uint32_t>(c); }
+	} else if (first) {
+		return share_column(s, blockIdx.x, gridDim.x, lane);
 	}
-	return __reduce_max_sync(0xFFFFFFFFu, c);
-}
-
-// The column with the most vectors not yet taken (warp 0); n_cols when there is none.
-__device__ __forceinline__ uint32_t next_column(const StrSetArgs& s, uint32_t lane) {
-	uint32_t best = 0, at = s.n_cols;
-	for (uint32_t i = lane; i < s.n_cols; i += 32) {
-		const uint64_t taken = ld_acquire_u64(s.flags + i);
-		const uint32_t n = s.cols[i].col.n_vec, left = taken < n ? n - static_cast<uint32_t>(taken) : 0u;
-		if (left > best) {
-			best = left;
-			at   = i;
-		}
-	}
-	const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, best);
-	return __reduce_min_sync(0xFFFFFFFFu, most && best == most ? at : s.n_cols);
+	return fullest_column(s, blockIdx.x, gridDim.x, lane);
 }
 
 // A warp takes vectors by its column's ticket, so that no warp waits for the others of its CTA, and the last vectors
@@ -752,7 +742,7 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 	for (bool first = true;; first = false) {
 		__syncthreads(); // the previous column's dictionary is read to the end
 		if (warp == 0) {
-			const uint32_t c = first ? first_column(s, lane) : next_column(s, lane);
+			const uint32_t c = next_column(s, lane, first);
 			if (lane == 0) { s_col = c; }
 		}
 		__syncthreads();
@@ -770,14 +760,14 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 		}
 		while (warp < s.active) {
 			unsigned long long ticket = 0;
-			if (lane == 0) { ticket = atomicAdd(reinterpret_cast<unsigned long long*>(s.flags + col), 1ull); }
+			if (lane == 0) { ticket = atomicAdd(reinterpret_cast<unsigned long long*>(s.flags + 1 + col), 1ull); }
 			ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
 			if (ticket >= n_vec) { break; }
 			const uint32_t  v       = static_cast<uint32_t>(ticket);
 			const uint2*    dict    = reinterpret_cast<const uint2*>(SMDICT ? sdict : A.dict8);
 			const uint32_t* tab     = SMDICT ? stab : A.rows8;
 			const uint32_t  entry_c = A.entry_c;
-			uint64_t*       words   = s.flags + s.n_cols + A.item_base;
+			uint64_t*       words   = s.flags + 1 + s.n_cols + A.item_base;
 			const Plan      p       = make_plan(A.col, v);
 			bool            bad     = false;
 			bool            ok      = p.ok;
@@ -1009,8 +999,10 @@ static cudaError_t launch_dict_pass_t(const StrSetArgs& a, int warps, uint32_t d
 	uint64_t   grid = static_cast<uint64_t>(sm_count) * per_sm;
 	grid            = grid < a.n_items ? grid : a.n_items;
 	if (grid == 0) { return cudaSuccess; }
-	const uint64_t each = (a.n_items + grid - 1) / grid;
-	b.active            = static_cast<uint32_t>(each < static_cast<uint64_t>(warps) ? each : warps);
+	// (columns' CTAs are whole numbers: a column of one and a half shares may get one CTA)
+	uint64_t each = (a.n_items + grid - 1) / grid;
+	each *= a.n_cols > 1 && each > 1 ? 2 : 1;
+	b.active = static_cast<uint32_t>(each < static_cast<uint64_t>(warps) ? each : warps);
 	fn<<<static_cast<unsigned>(grid), warps * 32, dyn_smem, s>>>(b);
 	++launch_counter();
 	return cudaGetLastError();

@@ -665,4 +665,36 @@ __device__ __forceinline__ uint32_t stream_vector(const uint32_t* rows32, const 
 	return vdec;
 }
 
+// The column a CTA starts with when there are fewer columns than CTAs: the one that holds the first vector of its share of
+// all vectors (warp 0).
+__device__ __forceinline__ uint32_t share_column(const StrSetArgs& s, uint32_t cta, uint32_t ctas, uint32_t lane) {
+	const uint64_t x = s.n_items * cta / ctas;
+	uint32_t       c = 0;
+	for (uint32_t i = lane; i < s.n_cols; i += 32) {
+		if (__ldg(s.first + i) <= x) { c = i; }
+	}
+	return __reduce_max_sync(0xFFFFFFFFu, c);
+}
+
+// The column with the most vectors not yet taken (warp 0); n_cols when there is none.  Every CTA looks from a column of
+// its own on, so that of columns with equally many, as row groups' are, CTAs that ask together take different ones.
+__device__ __forceinline__ uint32_t fullest_column(const StrSetArgs& s, uint32_t cta, uint32_t ctas, uint32_t lane) {
+	const uint32_t from = static_cast<uint32_t>(static_cast<uint64_t>(s.n_cols) * cta / ctas);
+	uint32_t       best = 0, at = 0;
+#pragma unroll 8
+	for (uint32_t i = lane; i < s.n_cols; i += 32) {
+		const uint32_t c     = i + from < s.n_cols ? i + from : i + from - s.n_cols;
+		const uint64_t taken = *reinterpret_cast<const volatile uint64_t*>(s.flags + 1 + c), n = __ldg(s.first + c + 1) - __ldg(s.first + c);
+		const uint32_t left  = taken < n ? static_cast<uint32_t>(n - taken) : 0u;
+		if (left > best) {
+			best = left;
+			at   = i;
+		}
+	}
+	const uint32_t most = __reduce_max_sync(0xFFFFFFFFu, best);
+	if (most == 0) { return s.n_cols; }
+	const uint32_t i = __reduce_min_sync(0xFFFFFFFFu, best == most ? at : ~0u);
+	return i + from < s.n_cols ? i + from : i + from - s.n_cols;
+}
+
 } // namespace flsgpu

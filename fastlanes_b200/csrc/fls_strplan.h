@@ -67,16 +67,17 @@ struct StrArgs {
 
 // One launch of the single-pass DICT decode (k_dict_pass) over the vectors of one or more DICT string columns.
 // Every column has a ticket; a CTA stays with a column, its dictionary in shared memory, while the column's ticket has
-// vectors left, and each of its warps takes them one by one.  Every vector publishes its decoded byte total and, once
-// its predecessors' totals are known, its inclusive prefix (a decoupled look-back within its column), so each vector
-// learns its first output byte without a separate lengths pass.
+// vectors left, and each of its warps takes them one by one; then it goes on to another column.  Every vector publishes
+// its decoded byte total and, once its predecessors' totals are known, its inclusive prefix (a decoupled look-back within
+// its column), so each vector learns its first output byte without a separate lengths pass.
 struct StrSetArgs {
 	const StrArgs*  cols;      // per-column arguments in device memory (each with dict8 and rows8)
 	uint32_t        n_cols;
 	uint32_t        active;    // warps of a CTA that take vectors (fewer for sets of fewer vectors than warps)
 	uint64_t        n_items;   // vectors of all columns
-	uint64_t*       flags;     // [c] the ticket of column c, [n_cols + item_base + v] the look-back word of vector v;
-	                           // zeroed before every launch
+	const uint64_t* first;     // the first vector of every column among all, and n_items behind them (one column: null)
+	uint64_t*       flags;     // [0] the cursor over the columns, [1 + c] the ticket of column c, [1 + n_cols + item_base
+	                           // + v] the look-back word of vector v; zeroed before every launch
 	int*            status;
 	uint32_t*       out_offsets; // one-column launches: the outputs (null: each column's own)
 	uint8_t*        out_bytes;

@@ -355,3 +355,31 @@ extern "C" void emu_smem_limit(const int* device, const uint32_t* bytes, int n, 
 		asked[i]     = g_emu_limit;
 	}
 }
+
+// The columns that CTAs 0 .. ctas - 1 of a string set take when they ask together (fls_strings.cuh): flags as the kernel
+// has them (the cursor, then a ticket a column), first: every column's first vector, and their number.
+extern "C" void emu_set_columns(const uint64_t* first, uint64_t* flags, uint32_t n_cols, uint32_t ctas, uint32_t* share,
+                                uint32_t* fullest) {
+	StrSetArgs s {};
+	s.n_cols  = n_cols;
+	s.n_items = first[n_cols];
+	s.first   = first;
+	s.flags   = flags;
+	std::barrier<>           bar(32);
+	EmuWarp                  w {&bar, {}, {}};
+	std::vector<std::thread> th;
+	for (uint32_t t = 0; t < 32; ++t) {
+		th.emplace_back([&, t] {
+			g_emu_warp = &w;
+			g_emu_lane = static_cast<int>(t);
+			for (uint32_t c = 0; c < ctas; ++c) {
+				const uint32_t x = share_column(s, c, ctas, t), y = fullest_column(s, c, ctas, t);
+				if (t == 0) {
+					share[c]   = x;
+					fullest[c] = y;
+				}
+			}
+		});
+	}
+	for (auto& x : th) { x.join(); }
+}

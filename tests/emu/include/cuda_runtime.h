@@ -97,6 +97,15 @@ inline unsigned __reduce_or_sync(unsigned, unsigned v) {
 	__syncwarp();
 	return r;
 }
+inline unsigned __reduce_max_sync(unsigned, unsigned v) {
+	g_emu_warp->xch[g_emu_lane] = v;
+	__syncwarp();
+	unsigned r = 0;
+	for (int i = 0; i < 32; ++i) { r = g_emu_warp->xch[i] > r ? static_cast<unsigned>(g_emu_warp->xch[i]) : r; }
+	__syncwarp();
+	return r;
+}
+inline unsigned __reduce_min_sync(unsigned m, unsigned v) { return ~__reduce_max_sync(m, ~v); }
 inline int __popc(unsigned x) { return __builtin_popcount(x); }
 inline int __popcll(unsigned long long x) { return __builtin_popcountll(x); }
 inline int __ffsll(long long x) { return __builtin_ffsll(x); }

@@ -161,8 +161,7 @@ struct fls_string_plan {
 	bool                     single   = false;
 	DevArr<StrArgs>          dargs;    // the plan's arguments in device memory (item_base 0)
 	DevArr<uint64_t>         lb;       // ticket + one look-back word per vector, zeroed before every decode
-	int                      sp_warps = 0;
-	uint32_t                 sp_smem  = 0, sp_dict_cap = 0, sp_tab_cap = 0;
+	DictLayout               layout {};
 	// single-pass FSST / BYTE_ARR decode (k_stream_single), look-back words in lb
 	bool                     stream_single = false;
 	// a measure() whose per-vector totals and bases the next decode() takes over (the usual measure, allocate,
@@ -355,19 +354,8 @@ int fls_string_plan_create(const uint8_t* d_page, uint64_t page_size, const uint
 	p->warps    = static_cast<int>(w < kStrMaxWarps ? w : kStrMaxWarps);
 	p->dyn_smem = static_cast<uint32_t>(p->warps * per_warp + (a.dict_in_smem ? dict_sm : 0u));
 	if (a.kind == STR_DICT && a.dict_rows && pi.vec_c > 0) {
-		// single-pass decode: the dictionary and its row table in shared memory when at least 8 warps still fit
-		p->single            = true;
-		const uint32_t   pw  = dict_pass_smem_per_warp(a.rows16);
-		const uint64_t   tab = (4ull * a.entry_c + 15) & ~15ull;
-		const uint64_t   all = kDictPassSmem, d8 = a.dict8_n;
-		uint64_t         sw  = all / pw;
-		if (d8 + tab < all && (all - d8 - tab) / pw >= 8) {
-			p->sp_dict_cap = static_cast<uint32_t>(d8);
-			p->sp_tab_cap  = a.entry_c;
-			sw             = (all - d8 - tab) / pw;
-		}
-		p->sp_warps = static_cast<int>(sw < kStrMaxWarps ? sw : kStrMaxWarps);
-		p->sp_smem  = static_cast<uint32_t>(p->sp_warps * pw + (p->sp_dict_cap ? d8 + tab : 0u));
+		p->single = true;
+		p->layout = dict_layout(a.dict8_n, a.entry_c, a.dict_bytes_n / a.entry_c, a.rows16);
 		if (!p->dargs.alloc(1) || !p->lb.alloc(2ull + pi.vec_c) ||
 		    cudaMemcpy(p->dargs.p, &a, sizeof(StrArgs), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return FLS_ERR_CUDA;
@@ -424,9 +412,7 @@ static int single_pass_decode(const fls_string_plan* p, uint32_t* d_offsets, uin
 	x.out_offsets = d_offsets;
 	x.out_bytes   = d_bytes;
 	x.out_cap     = cap;
-	x.dict_cap    = p->sp_dict_cap;
-	x.tab_cap     = p->sp_tab_cap;
-	return launch_dict_pass(x, p->args.rows16, p->sp_warps, p->sp_smem, s) == cudaSuccess ? FLS_OK : FLS_ERR_CUDA;
+	return launch_dict_pass(x, p->args.rows16, p->layout, s) == cudaSuccess ? FLS_OK : FLS_ERR_CUDA;
 }
 
 int fls_string_plan_decode(const fls_string_plan* p, uint32_t* d_offsets, uint8_t* d_bytes, uint64_t bytes_cap,
@@ -481,8 +467,7 @@ struct fls_string_set {
 	DevArr<uint64_t>     first;    // every column's first vector among all, and their number
 	DevArr<uint64_t>     lb;       // the cursor, a ticket per column, one look-back word per vector of every column
 	uint64_t             n_items  = 0;
-	int                  warps    = 0;
-	uint32_t             smem = 0, dict_cap = 0, tab_cap = 0;
+	DictLayout           layout {};
 	bool                 rows16 = true, bound = false;
 	int*                 status = nullptr;
 };
@@ -493,7 +478,7 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 	if (!out || !plans || n == 0) { return FLS_ERR_ARG; }
 	*out = nullptr;
 	std::unique_ptr<fls_string_set> set(new fls_string_set());
-	uint64_t              dict_max = 0, tab_max = 0;
+	uint64_t              dict_max = 0, packed_sum = 0, tab_max = 0, entry_sum = 0;
 	std::vector<uint64_t> first;
 	for (uint32_t i = 0; i < n; ++i) {
 		if (!plans[i]) { return FLS_ERR_ARG; }
@@ -506,19 +491,11 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 		set->rows16 = set->rows16 && a.rows16;
 		dict_max    = std::max<uint64_t>(dict_max, a.dict8_n);
 		tab_max     = std::max<uint64_t>(tab_max, a.entry_c);
+		packed_sum += a.dict_bytes_n;
+		entry_sum += a.entry_c;
 		set->status = a.status;
 	}
-	const uint32_t pw  = dict_pass_smem_per_warp(set->rows16);
-	const uint64_t tab = (4 * tab_max + 15) & ~15ull;
-	const uint64_t all = kDictPassSmem;
-	uint64_t       w   = all / pw;
-	if (dict_max + tab < all && (all - dict_max - tab) / pw >= 8) {
-		set->dict_cap = static_cast<uint32_t>(dict_max);
-		set->tab_cap  = static_cast<uint32_t>(tab_max);
-		w             = (all - dict_max - tab) / pw;
-	}
-	set->warps = static_cast<int>(w < kStrMaxWarps ? w : kStrMaxWarps);
-	set->smem  = static_cast<uint32_t>(set->warps * pw + (set->dict_cap ? dict_max + tab : 0u));
+	set->layout = dict_layout(dict_max, tab_max, packed_sum / entry_sum, set->rows16);
 	first.push_back(set->n_items);
 	if (!set->cols.alloc(n) || !set->first.alloc(first.size()) || !set->lb.alloc(1 + n + set->n_items) ||
 	    cudaMemcpy(set->first.p, first.data(), 8 * first.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
@@ -556,12 +533,10 @@ int fls_string_set_decode(const fls_string_set* set, fls_stream_t stream) {
 	x.cols      = set->cols.p;
 	x.n_cols    = static_cast<uint32_t>(set->args.size());
 	x.n_items   = set->n_items;
-	x.first     = set->first.p;
 	x.flags     = set->lb.p;
 	x.status    = set->status;
-	x.dict_cap  = set->dict_cap;
-	x.tab_cap   = set->tab_cap;
-	return launch_dict_pass(x, set->rows16, set->warps, set->smem, s) == cudaSuccess ? FLS_OK : FLS_ERR_CUDA;
+	x.first     = set->first.p;
+	return launch_dict_pass(x, set->rows16, set->layout, s) == cudaSuccess ? FLS_OK : FLS_ERR_CUDA;
 }
 
 int fls_string_set_destroy(fls_string_set* set) {

@@ -129,10 +129,6 @@ constexpr uint32_t kStrPB      = 4;
 constexpr uint32_t kStrRows    = 4096 + 128; // >= 1055 padded row words, >= 128 * (32 + 1) staged bytes
 constexpr uint32_t kStrRows16  = 2048 + 128; // >= 1086 padded 16-bit rows, >= 128 * (16 + 1) staged bytes
 constexpr uint32_t kStrWindow  = 2048;
-// k_dict_pass: three quarters of it, for more warps beside the dictionary (16 Mi rows over 4,096 entries: 243 us with 24
-// warps and 2 KB, 232 us with 28 and 1.5 KB)
-constexpr uint32_t kDictWindow = 1536;
-
 enum : int { STR_PASS_LENGTHS = 0, STR_PASS_MATERIALIZE = 1 };
 
 // per-warp shared memory of the single-pass FSST / BYTE_ARR kernel: rows, then the window (no plan ring)
@@ -630,7 +626,7 @@ __device__ __forceinline__ uint64_t lookback(const uint64_t* words, uint32_t v, 
 // row per lane, positions by a warp scan) into the warp's output window (put_row), which leaves in 16-byte
 // stores.  tab: the row table ((start / 8) | length << 24) of the dictionary's entry_c entries.  Returns the
 // bytes written; *bad for codes outside the dictionary (such rows are empty).
-template <bool R16>
+template <bool R16, uint32_t WINDOW>
 __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const uint32_t* tab, uint32_t entry_c,
                                                     const uint2* dict, uint8_t* win, uint32_t* offs, uint8_t* bytes,
                                                     uint64_t vbase, uint32_t lane, bool* bad) {
@@ -685,24 +681,32 @@ __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const u
 		const uint32_t o   = vpos + inc - fl;
 		const uint32_t T   = __shfl_sync(0xFFFFFFFFu, inc, 31);
 		offs[32 * b + lane] = static_cast<uint32_t>(vbase + o);
-		if (fill + T > kDictWindow) { flush(false); }
-		if (fill + T <= kDictWindow) {
-			uint32_t   hk = 0, head = 0;
-			const bool mid = put_row8(win32, fill + (o - vpos), dict + fs, fl, &hk, &head);
+		// the rows of the lanes that have one here, the batch's byte `from` at the window's byte `fill`
+		auto put = [&](bool mine, uint32_t from) {
+			uint32_t       hk = 0, head = 0;
+			bool           mid = false;
+			const uint32_t d = fill + (o - vpos - from), n = mine ? fl : 0u;
+			mid = put_row8(win32, d, dict + fs, n, &hk, &head);
 			__syncwarp(); // every word's whole store lands before the rows that start inside it OR in
 			if (mid) { atomicOr(win32 + hk, head); }
+		};
+		if (fill + T > WINDOW) { flush(false); }
+		if (fill + T <= WINDOW) {
+			put(true, 0);
 			fill += T;
 		} else {
-			// a batch larger than the window: straight to global memory after the window's pending bytes
-			flush(true);
-			uint8_t* dst = bytes + vbase + o;
-			for (uint32_t i = 0; i < fl; ++i) { dst[i] = reinterpret_cast<const uint8_t*>(dict + fs)[i]; }
-			const uint64_t pos = vbase + vpos + T;
-			W                  = pos & ~15ull;
-			fill               = static_cast<uint32_t>(pos & 15u);
-			lo                 = pos;
-			__syncwarp();
-			if (lane == 0) { win32[fill >> 2] = 0; }
+			// more than the window takes at a time (rows of more than 47 or 63 bytes on average): as many rows as fit, until
+			// all are out (a row of up to 255 bytes always fits).  12 Mi rows of 60 to 140 bytes: 9,949 us when such a
+			// batch went to global memory byte by byte, 546 us so.
+			for (uint32_t done = 0; done < T;) {
+				const uint32_t room = done + WINDOW - fill;
+				const uint32_t upto = T <= room ? T : __reduce_max_sync(0xFFFFFFFFu, inc <= room ? inc : 0u);
+				put(inc <= upto && inc - fl >= done, done);
+				__syncwarp();
+				fill += upto - done;
+				done = upto;
+				if (done < T) { flush(false); }
+			}
 		}
 		vpos += T;
 		__syncwarp();
@@ -729,12 +733,12 @@ __device__ __forceinline__ uint32_t next_column(const StrSetArgs& s, uint32_t la
 // A warp takes vectors by its column's ticket, so that no warp waits for the others of its CTA, and the last vectors
 // of a set are spread over all SMs (a CTA that took 28 vectors at a time left 107 of 148 SMs idle for the second
 // half of a 5,280-vector set: 120 us in all, 87 us so; 200 vectors of one column: 60 us a decode, 41 us so).
-template <bool R16, bool SMDICT>
+template <bool R16, bool SMDICT, uint32_t WINDOW>
 __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArgs s) {
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ uint32_t s_col;
 	const uint32_t      lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
-	constexpr uint32_t  kPerWarp = str_rows_bytes(R16) + kDictWindow;
+	constexpr uint32_t  kPerWarp = str_rows_bytes(R16) + WINDOW;
 	uint8_t*            rows     = smem + warp * kPerWarp;
 	uint8_t*            win      = rows + str_rows_bytes(R16);
 	uint8_t*            sdict    = smem + nwarps * kPerWarp;
@@ -800,7 +804,7 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 			} else if (!ok) {
 				for (uint32_t r = lane; r < kVec; r += 32) { offs[r] = static_cast<uint32_t>(P); }
 			} else {
-				const uint32_t got = dict_vector_out<R16>(rows, tab, entry_c, dict, win, offs, bytes, P, lane, &bad);
+				const uint32_t got = dict_vector_out<R16, WINDOW>(rows, tab, entry_c, dict, win, offs, bytes, P, lane, &bad);
 				if (got != T) { bad = true; }
 			}
 			if (lane == 0 && v + 1 == n_vec) { offsets[static_cast<uint64_t>(n_vec) * kVec] = static_cast<uint32_t>(P + T); }
@@ -977,11 +981,9 @@ cudaError_t launch_str_lengths(const StrArgs& a, int sm_count, cudaStream_t s) {
 	}
 }
 
-uint32_t dict_pass_smem_per_warp(bool rows16) { return str_rows_bytes(rows16) + kDictWindow; }
-
-template <bool R16, bool SMDICT>
+template <bool R16, bool SMDICT, uint32_t WINDOW>
 static cudaError_t launch_dict_pass_t(const StrSetArgs& a, int warps, uint32_t dyn_smem, cudaStream_t s, int sm_count) {
-	auto* const      fn = k_dict_pass<R16, SMDICT>;
+	auto* const      fn = k_dict_pass<R16, SMDICT, WINDOW>;
 	static SmemLimit limit;
 	cudaError_t      e = limit.need(reinterpret_cast<const void*>(fn), dyn_smem);
 	if (e != cudaSuccess) { return e; }
@@ -1008,16 +1010,22 @@ static cudaError_t launch_dict_pass_t(const StrSetArgs& a, int warps, uint32_t d
 	return cudaGetLastError();
 }
 
-cudaError_t launch_dict_pass(const StrSetArgs& a, bool rows16, int warps, uint32_t dyn_smem, cudaStream_t s,
-                             int sm_count) {
-	if (warps < 1 || warps > kStrMaxWarps) { return cudaErrorInvalidValue; }
-	const bool sm = a.dict_cap != 0;
-	if (rows16) {
-		return sm ? launch_dict_pass_t<true, true>(a, warps, dyn_smem, s, sm_count)
-		          : launch_dict_pass_t<true, false>(a, warps, dyn_smem, s, sm_count);
+template <bool R16, uint32_t WINDOW>
+static cudaError_t launch_dict_pass_w(const StrSetArgs& a, const DictLayout& l, cudaStream_t s, int sm_count) {
+	const int w = static_cast<int>(l.warps);
+	return l.mode == DICT_SMEM8 ? launch_dict_pass_t<R16, true, WINDOW>(a, w, l.smem, s, sm_count)
+	                            : launch_dict_pass_t<R16, false, WINDOW>(a, w, l.smem, s, sm_count);
+}
+
+cudaError_t launch_dict_pass(const StrSetArgs& args, bool rows16, const DictLayout& l, cudaStream_t s, int sm_count) {
+	if (l.warps < 1 || l.warps > static_cast<uint32_t>(kStrMaxWarps)) { return cudaErrorInvalidValue; }
+	StrSetArgs a = args;
+	a.dict_cap   = l.dict_cap;
+	if (l.window == kDictWindow) {
+		return rows16 ? launch_dict_pass_w<true, kDictWindow>(a, l, s, sm_count) : launch_dict_pass_w<false, kDictWindow>(a, l, s, sm_count);
 	}
-	return sm ? launch_dict_pass_t<false, true>(a, warps, dyn_smem, s, sm_count)
-	          : launch_dict_pass_t<false, false>(a, warps, dyn_smem, s, sm_count);
+	return rows16 ? launch_dict_pass_w<true, kDictWideWindow>(a, l, s, sm_count)
+	              : launch_dict_pass_w<false, kDictWideWindow>(a, l, s, sm_count);
 }
 
 template <int KIND>

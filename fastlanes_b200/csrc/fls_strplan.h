@@ -82,17 +82,49 @@ struct StrSetArgs {
 	uint32_t*       out_offsets; // one-column launches: the outputs (null: each column's own)
 	uint8_t*        out_bytes;
 	uint64_t        out_cap;
-	uint32_t        dict_cap; // shared memory held for a dictionary's bytes (16-byte multiple; 0: dictionaries in
-	                          // global memory)
-	uint32_t        tab_cap;  // entries held for the packed row table (with dict_cap)
+	uint32_t        dict_cap; // shared memory held for a dictionary's bytes (a multiple of 16)
 };
 
 // dynamic shared memory of a k_dict_pass CTA (227 KB less its static words)
 constexpr uint32_t kDictPassSmem = 226 * 1024;
-// per-warp shared memory of k_dict_pass: the vector's rows and the output window
-uint32_t dict_pass_smem_per_warp(bool rows16);
-cudaError_t launch_dict_pass(const StrSetArgs& a, bool rows16, int warps, uint32_t dyn_smem, cudaStream_t s,
-                             int sm_count = 0);
+// of a warp of it beside its window: the vector's rows
+constexpr uint32_t kDictRows16 = 2048 + 128, kDictRows32 = 4096 + 128;
+
+constexpr uint32_t kDictWindow = 1536, kDictWideWindow = 2048; // a warp's output window
+
+// Where k_dict_pass has its dictionaries (entries on 8-byte boundaries: dict8, rows8): in global or shared memory.
+enum : uint32_t { DICT_GLOBAL, DICT_SMEM8 };
+
+struct DictLayout {
+	uint32_t mode, warps, window;
+	uint32_t dict_cap, smem; // shared memory held for the dictionary's bytes, and in all
+};
+
+// How a k_dict_pass CTA is laid out for dictionaries of at most `d8` bytes (entries padded to 8), `entries` entries and
+// `mean` bytes an entry: in shared memory when at least 8 warps fit beside them.  Window (columns of 12,000 vectors,
+// us): 2 KB costs warps, 1.5 KB splits the batches of long rows.  Entries of 40 to 60 bytes (2,000 of them): 267 with 27
+// warps of 2 KB, 355 with 31 of 1.5 KB; of 5 to 40 bytes (4,096): 191 with 25, 181 with 29.  So 2 KB for means of 40 bytes
+// on, and wherever 32 warps fit all the same (20 to 40 bytes, 300 entries: 198 against 204).
+inline DictLayout dict_layout(uint64_t d8, uint64_t entries, uint64_t mean, bool rows16) {
+	const uint64_t tab = (4 * entries + 15) & ~15ull;
+	d8                 = (d8 + 15) & ~15ull;
+	DictLayout l {};
+	auto       warps = [&](uint64_t held) { // that fit beside `held` bytes
+		const uint64_t w = held < kDictPassSmem ? (kDictPassSmem - held) / ((rows16 ? kDictRows16 : kDictRows32) + l.window) : 0;
+		return w < static_cast<uint64_t>(kStrMaxWarps) ? w : static_cast<uint64_t>(kStrMaxWarps);
+	};
+	for (const uint32_t window : {kDictWideWindow, kDictWindow}) {
+		l.window   = window;
+		l.mode     = warps(d8 + tab) >= 8 ? DICT_SMEM8 : DICT_GLOBAL;
+		l.dict_cap = static_cast<uint32_t>(l.mode == DICT_SMEM8 ? d8 : 0);
+		const uint64_t held = l.mode == DICT_GLOBAL ? 0 : l.dict_cap + tab;
+		l.warps             = static_cast<uint32_t>(warps(held));
+		l.smem              = static_cast<uint32_t>(held) + l.warps * ((rows16 ? kDictRows16 : kDictRows32) + window);
+		if (mean >= 40 || (l.mode != DICT_GLOBAL && l.warps == static_cast<uint32_t>(kStrMaxWarps))) { break; }
+	}
+	return l;
+}
+cudaError_t launch_dict_pass(const StrSetArgs& a, bool rows16, const DictLayout& l, cudaStream_t s, int sm_count = 0);
 
 // The dictionary's entries (rows: start | length << 24) from bytes to their places in bytes8 (rows8), zero behind them.
 cudaError_t launch_dict_align(const uint8_t* bytes, const uint32_t* rows, const uint32_t* rows8, uint32_t entry_c,

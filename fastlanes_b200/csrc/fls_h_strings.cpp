@@ -355,7 +355,7 @@ int fls_string_plan_create(const uint8_t* d_page, uint64_t page_size, const uint
 	p->dyn_smem = static_cast<uint32_t>(p->warps * per_warp + (a.dict_in_smem ? dict_sm : 0u));
 	if (a.kind == STR_DICT && a.dict_rows && pi.vec_c > 0) {
 		p->single = true;
-		p->layout = dict_layout(a.dict8_n, a.entry_c, a.dict_bytes_n / a.entry_c, a.rows16);
+		p->layout = dict_layout(a.dict8_n, a.dict_bytes_n, a.entry_c, a.dict_bytes_n / a.entry_c, a.rows16);
 		if (!p->dargs.alloc(1) || !p->lb.alloc(2ull + pi.vec_c) ||
 		    cudaMemcpy(p->dargs.p, &a, sizeof(StrArgs), cudaMemcpyHostToDevice) != cudaSuccess) {
 			return FLS_ERR_CUDA;
@@ -478,7 +478,7 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 	if (!out || !plans || n == 0) { return FLS_ERR_ARG; }
 	*out = nullptr;
 	std::unique_ptr<fls_string_set> set(new fls_string_set());
-	uint64_t              dict_max = 0, packed_sum = 0, tab_max = 0, entry_sum = 0;
+	uint64_t              dict_max = 0, packed_max = 0, packed_sum = 0, tab_max = 0, entry_sum = 0;
 	std::vector<uint64_t> first;
 	for (uint32_t i = 0; i < n; ++i) {
 		if (!plans[i]) { return FLS_ERR_ARG; }
@@ -490,12 +490,13 @@ int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_s
 		set->n_items += a.col.n_vec;
 		set->rows16 = set->rows16 && a.rows16;
 		dict_max    = std::max<uint64_t>(dict_max, a.dict8_n);
+		packed_max  = std::max<uint64_t>(packed_max, a.dict_bytes_n);
 		tab_max     = std::max<uint64_t>(tab_max, a.entry_c);
 		packed_sum += a.dict_bytes_n;
 		entry_sum += a.entry_c;
 		set->status = a.status;
 	}
-	set->layout = dict_layout(dict_max, tab_max, packed_sum / entry_sum, set->rows16);
+	set->layout = dict_layout(dict_max, packed_max, tab_max, packed_sum / entry_sum, set->rows16);
 	first.push_back(set->n_items);
 	if (!set->cols.alloc(n) || !set->first.alloc(first.size()) || !set->lb.alloc(1 + n + set->n_items) ||
 	    cudaMemcpy(set->first.p, first.data(), 8 * first.size(), cudaMemcpyHostToDevice) != cudaSuccess) {

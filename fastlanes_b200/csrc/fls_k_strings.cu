@@ -624,11 +624,12 @@ __device__ __forceinline__ uint64_t lookback(const uint64_t* words, uint32_t v, 
 
 // Rows of one DICT vector into Arrow offsets and bytes from the first output byte vbase: 32 rows at a time (a
 // row per lane, positions by a warp scan) into the warp's output window (put_row), which leaves in 16-byte
-// stores.  tab: the row table ((start / 8) | length << 24) of the dictionary's entry_c entries.  Returns the
-// bytes written; *bad for codes outside the dictionary (such rows are empty).
-template <bool R16, uint32_t WINDOW>
+// stores.  tab: the row table of the dictionary's entry_c entries (start | length << 24; the start in units of 8 bytes
+// when the entries lie on 8-byte boundaries, MODE).  Returns the bytes written; *bad for codes outside the dictionary
+// (such rows are empty).
+template <bool R16, int MODE, uint32_t WINDOW>
 __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const uint32_t* tab, uint32_t entry_c,
-                                                    const uint2* dict, uint8_t* win, uint32_t* offs, uint8_t* bytes,
+                                                    const uint8_t* dict, uint8_t* win, uint32_t* offs, uint8_t* bytes,
                                                     uint64_t vbase, uint32_t lane, bool* bad) {
 	uint32_t* win32 = reinterpret_cast<uint32_t*>(win);
 	uint64_t  W     = vbase & ~15ull; // output position of win[0]
@@ -686,7 +687,11 @@ __device__ __forceinline__ uint32_t dict_vector_out(const uint8_t* rows, const u
 			uint32_t       hk = 0, head = 0;
 			bool           mid = false;
 			const uint32_t d = fill + (o - vpos - from), n = mine ? fl : 0u;
-			mid = put_row8(win32, d, dict + fs, n, &hk, &head);
+			if constexpr (MODE == DICT_SMEM_PACKED) {
+				mid = put_row(win32, d, reinterpret_cast<const uint32_t*>(dict), fs, n, &hk, &head);
+			} else {
+				mid = put_row8(win32, d, reinterpret_cast<const uint2*>(dict) + fs, n, &hk, &head);
+			}
 			__syncwarp(); // every word's whole store lands before the rows that start inside it OR in
 			if (mid) { atomicOr(win32 + hk, head); }
 		};
@@ -733,7 +738,7 @@ __device__ __forceinline__ uint32_t next_column(const StrSetArgs& s, uint32_t la
 // A warp takes vectors by its column's ticket, so that no warp waits for the others of its CTA, and the last vectors
 // of a set are spread over all SMs (a CTA that took 28 vectors at a time left 107 of 148 SMs idle for the second
 // half of a 5,280-vector set: 120 us in all, 87 us so; 200 vectors of one column: 60 us a decode, 41 us so).
-template <bool R16, bool SMDICT, uint32_t WINDOW>
+template <bool R16, int MODE, uint32_t WINDOW>
 __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArgs s) {
 	extern __shared__ __align__(128) uint8_t smem[];
 	__shared__ uint32_t s_col;
@@ -754,12 +759,14 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 		if (col >= s.n_cols) { break; }
 		const StrArgs& A     = s.cols[col];
 		const uint32_t n_vec = A.col.n_vec;
-		if constexpr (SMDICT) {
-			// the column's aligned dictionary (cudaMalloc'd, a multiple of 16 bytes) and row table
-			const uint32_t nb16 = static_cast<uint32_t>((A.dict8_n + 15) / 16);
-			const uint4*   src  = reinterpret_cast<const uint4*>(A.dict8);
+		const uint8_t*  gdict = MODE == DICT_SMEM_PACKED ? A.dict_bytes : A.dict8;
+		const uint32_t* gtab  = MODE == DICT_SMEM_PACKED ? A.dict_rows : A.rows8;
+		if constexpr (MODE != DICT_GLOBAL) {
+			// the column's dictionary (cudaMalloc'd, with 16 bytes of slack) and row table
+			const uint32_t nb16 = static_cast<uint32_t>(((MODE == DICT_SMEM_PACKED ? A.dict_bytes_n : A.dict8_n) + 15) / 16);
+			const uint4*   src  = reinterpret_cast<const uint4*>(gdict);
 			for (uint32_t i = threadIdx.x; i < nb16; i += blockDim.x) { reinterpret_cast<uint4*>(sdict)[i] = __ldg(src + i); }
-			for (uint32_t i = threadIdx.x; i < A.entry_c; i += blockDim.x) { stab[i] = __ldg(A.rows8 + i); }
+			for (uint32_t i = threadIdx.x; i < A.entry_c; i += blockDim.x) { stab[i] = __ldg(gtab + i); }
 			__syncthreads();
 		}
 		while (warp < s.active) {
@@ -768,8 +775,8 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 			ticket = __shfl_sync(0xFFFFFFFFu, ticket, 0);
 			if (ticket >= n_vec) { break; }
 			const uint32_t  v       = static_cast<uint32_t>(ticket);
-			const uint2*    dict    = reinterpret_cast<const uint2*>(SMDICT ? sdict : A.dict8);
-			const uint32_t* tab     = SMDICT ? stab : A.rows8;
+			const uint8_t*  dict    = MODE == DICT_GLOBAL ? gdict : sdict;
+			const uint32_t* tab     = MODE == DICT_GLOBAL ? gtab : stab;
 			const uint32_t  entry_c = A.entry_c;
 			uint64_t*       words   = s.flags + 1 + s.n_cols + A.item_base;
 			const Plan      p       = make_plan(A.col, v);
@@ -804,7 +811,7 @@ __global__ void __launch_bounds__(kStrMaxWarps * 32) k_dict_pass(const StrSetArg
 			} else if (!ok) {
 				for (uint32_t r = lane; r < kVec; r += 32) { offs[r] = static_cast<uint32_t>(P); }
 			} else {
-				const uint32_t got = dict_vector_out<R16, WINDOW>(rows, tab, entry_c, dict, win, offs, bytes, P, lane, &bad);
+				const uint32_t got = dict_vector_out<R16, MODE, WINDOW>(rows, tab, entry_c, dict, win, offs, bytes, P, lane, &bad);
 				if (got != T) { bad = true; }
 			}
 			if (lane == 0 && v + 1 == n_vec) { offsets[static_cast<uint64_t>(n_vec) * kVec] = static_cast<uint32_t>(P + T); }
@@ -981,9 +988,10 @@ cudaError_t launch_str_lengths(const StrArgs& a, int sm_count, cudaStream_t s) {
 	}
 }
 
-template <bool R16, bool SMDICT, uint32_t WINDOW>
+
+template <bool R16, int MODE, uint32_t WINDOW>
 static cudaError_t launch_dict_pass_t(const StrSetArgs& a, int warps, uint32_t dyn_smem, cudaStream_t s, int sm_count) {
-	auto* const      fn = k_dict_pass<R16, SMDICT, WINDOW>;
+	auto* const      fn = k_dict_pass<R16, MODE, WINDOW>;
 	static SmemLimit limit;
 	cudaError_t      e = limit.need(reinterpret_cast<const void*>(fn), dyn_smem);
 	if (e != cudaSuccess) { return e; }
@@ -1013,8 +1021,11 @@ static cudaError_t launch_dict_pass_t(const StrSetArgs& a, int warps, uint32_t d
 template <bool R16, uint32_t WINDOW>
 static cudaError_t launch_dict_pass_w(const StrSetArgs& a, const DictLayout& l, cudaStream_t s, int sm_count) {
 	const int w = static_cast<int>(l.warps);
-	return l.mode == DICT_SMEM8 ? launch_dict_pass_t<R16, true, WINDOW>(a, w, l.smem, s, sm_count)
-	                            : launch_dict_pass_t<R16, false, WINDOW>(a, w, l.smem, s, sm_count);
+	switch (l.mode) {
+	case DICT_SMEM8: return launch_dict_pass_t<R16, DICT_SMEM8, WINDOW>(a, w, l.smem, s, sm_count);
+	case DICT_SMEM_PACKED: return launch_dict_pass_t<R16, DICT_SMEM_PACKED, WINDOW>(a, w, l.smem, s, sm_count);
+	default: return launch_dict_pass_t<R16, DICT_GLOBAL, WINDOW>(a, w, l.smem, s, sm_count);
+	}
 }
 
 cudaError_t launch_dict_pass(const StrSetArgs& args, bool rows16, const DictLayout& l, cudaStream_t s, int sm_count) {

@@ -92,34 +92,46 @@ constexpr uint32_t kDictRows16 = 2048 + 128, kDictRows32 = 4096 + 128;
 
 constexpr uint32_t kDictWindow = 1536, kDictWideWindow = 2048; // a warp's output window
 
-// Where k_dict_pass has its dictionaries (entries on 8-byte boundaries: dict8, rows8): in global or shared memory.
-enum : uint32_t { DICT_GLOBAL, DICT_SMEM8 };
+// Where k_dict_pass has its dictionaries: entries on 8-byte boundaries (dict8, rows8) in global or shared memory, or
+// byte after byte (dict_bytes, dict_rows) in shared memory.
+enum : uint32_t { DICT_GLOBAL, DICT_SMEM8, DICT_SMEM_PACKED };
 
 struct DictLayout {
 	uint32_t mode, warps, window;
 	uint32_t dict_cap, smem; // shared memory held for the dictionary's bytes, and in all
 };
 
-// How a k_dict_pass CTA is laid out for dictionaries of at most `d8` bytes (entries padded to 8), `entries` entries and
-// `mean` bytes an entry: in shared memory when at least 8 warps fit beside them.  Window (columns of 12,000 vectors,
-// us): 2 KB costs warps, 1.5 KB splits the batches of long rows.  Entries of 40 to 60 bytes (2,000 of them): 267 with 27
-// warps of 2 KB, 355 with 31 of 1.5 KB; of 5 to 40 bytes (4,096): 191 with 25, 181 with 29.  So 2 KB for means of 40 bytes
-// on, and wherever 32 warps fit all the same (20 to 40 bytes, 300 entries: 198 against 204).
-inline DictLayout dict_layout(uint64_t d8, uint64_t entries, uint64_t mean, bool rows16) {
-	const uint64_t tab = (4 * entries + 15) & ~15ull;
-	d8                 = (d8 + 15) & ~15ull;
+// How a k_dict_pass CTA is laid out for dictionaries of at most `d8` bytes (entries padded to 8) or `packed` bytes
+// (unpadded), `entries` entries and `mean` bytes an entry.  Measured on columns of 12,000 vectors (us):
+//   window   2 KB costs warps, 1.5 KB splits the batches of long rows.  Entries of 40 to 60 bytes (2,000 of them): 267 with
+//            27 warps of 2 KB, 355 with 31 of 1.5 KB; of 5 to 40 bytes (4,096): 191 with 25, 181 with 29.  So 2 KB for
+//            means of 40 bytes on, and wherever 32 warps fit all the same (20 to 40 bytes, 300 entries: 198 against 204).
+//   mode     whole 8-byte loads pay for entries of some length: 173 against 189 packed (5 to 40 bytes, 300 entries), 400
+//            against 445 (5 to 20 bytes, 200 columns of 500 entries and 200 vectors), but 146 against 138 (9 bytes),
+//            120 against 109 (1 byte).  The padding costs warps: 204 with 17 against 165
+//            with 28 packed (6,000 of 17 bytes), 251 with 14 against 243 with 19 (6,000 of 5 to 40 bytes).  So padded
+//            from 10 bytes on, if four fifths of the packed form's warps fit.
+//   global   below about 13 warps the dictionary does better in the L1 and L2 caches: 302 against 409 with 8 (7,500
+//            of 5 to 40 bytes), 224 against 323 with 8 (10,000 of 9 bytes, padded); with 18 warps 214 against 173
+//            (18,000 of 5 bytes), with 14 304 against 251.
+inline DictLayout dict_layout(uint64_t d8, uint64_t packed, uint64_t entries, uint64_t mean, bool rows16) {
+	constexpr uint64_t kMinWarps = 13;
+	const uint64_t     tab = (4 * entries + 15) & ~15ull;
+	d8     = (d8 + 15) & ~15ull;
+	packed = (packed + 15) & ~15ull;
 	DictLayout l {};
 	auto       warps = [&](uint64_t held) { // that fit beside `held` bytes
 		const uint64_t w = held < kDictPassSmem ? (kDictPassSmem - held) / ((rows16 ? kDictRows16 : kDictRows32) + l.window) : 0;
 		return w < static_cast<uint64_t>(kStrMaxWarps) ? w : static_cast<uint64_t>(kStrMaxWarps);
 	};
 	for (const uint32_t window : {kDictWideWindow, kDictWindow}) {
-		l.window   = window;
-		l.mode     = warps(d8 + tab) >= 8 ? DICT_SMEM8 : DICT_GLOBAL;
-		l.dict_cap = static_cast<uint32_t>(l.mode == DICT_SMEM8 ? d8 : 0);
+		l.window          = window;
+		const uint64_t w8 = warps(d8 + tab), wp = warps(packed + tab);
+		l.mode            = mean >= 10 && w8 >= kMinWarps && 5 * w8 >= 4 * wp ? DICT_SMEM8 : wp >= kMinWarps ? DICT_SMEM_PACKED : DICT_GLOBAL;
+		l.dict_cap        = static_cast<uint32_t>(l.mode == DICT_SMEM8 ? d8 : l.mode == DICT_SMEM_PACKED ? packed : 0);
 		const uint64_t held = l.mode == DICT_GLOBAL ? 0 : l.dict_cap + tab;
-		l.warps             = static_cast<uint32_t>(warps(held));
-		l.smem              = static_cast<uint32_t>(held) + l.warps * ((rows16 ? kDictRows16 : kDictRows32) + window);
+		l.warps           = static_cast<uint32_t>(warps(held));
+		l.smem            = static_cast<uint32_t>(held) + l.warps * ((rows16 ? kDictRows16 : kDictRows32) + window);
 		if (mean >= 40 || (l.mode != DICT_GLOBAL && l.warps == static_cast<uint32_t>(kStrMaxWarps))) { break; }
 	}
 	return l;

@@ -385,8 +385,8 @@ extern "C" void emu_set_columns(const uint64_t* first, uint64_t* flags, uint32_t
 }
 
 // The layout of the single-pass DICT decode (dict_layout): mode, warps, window, dict_cap, smem, and a warp's rows.
-extern "C" void emu_dict_layout(uint64_t d8, uint64_t, uint64_t entries, uint64_t mean, int rows16, uint32_t* out) {
-	const DictLayout l = dict_layout(d8, entries, mean, rows16 != 0);
+extern "C" void emu_dict_layout(uint64_t d8, uint64_t packed, uint64_t entries, uint64_t mean, int rows16, uint32_t* out) {
+	const DictLayout l = dict_layout(d8, packed, entries, mean, rows16 != 0);
 	const uint32_t   x[6] = {l.mode, l.warps, l.window, l.dict_cap, l.smem, rows16 ? kDictRows16 : kDictRows32};
 	std::memcpy(out, x, sizeof(x));
 }

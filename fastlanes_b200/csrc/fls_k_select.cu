@@ -1157,10 +1157,19 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 	const uint64_t n      = a.fill ? n_fill : a.n_items - n_fill;
 	auto           item   = [&](uint64_t i) { return a.fill ? i * a.stride : a.stride == 1 ? i : i + i / (a.stride - 1) + 1; };
 	const uint64_t gw = static_cast<uint64_t>(blockIdx.x) * kStrWarps, nw = static_cast<uint64_t>(gridDim.x) * kStrWarps;
-	// units are dealt to the warps round robin, over the columns' borders
-	for (uint64_t first = 0; first < n;) {
-		const uint32_t col = a.items[item(first)].col;
-		uint64_t       lo = first + 1, hi = n; // the column's end among them: the first item of another column
+	// units are dealt to the warps round robin, over the columns' borders; a CTA goes from the column of its first unit to
+	// that of its first unit past it
+	for (uint64_t u0 = 0;;) {
+		const uint64_t turn = u0 % nw; // whose unit u0 is
+		u0 += turn < gw ? gw - turn : turn < gw + kStrWarps ? 0 : nw - turn + gw;
+		if (u0 >= n << per) { break; }
+		const uint32_t col = a.items[item(u0 >> per)].col;
+		// the column's end among the items, the first of another column: by doubling steps, then halving
+		uint64_t lo = (u0 >> per) + 1, hi = lo;
+		for (uint64_t d = 1; hi < n && a.items[item(hi)].col == col; d *= 2) {
+			lo = hi + 1;
+			hi = lo + d < n ? lo + d : n;
+		}
 		while (lo < hi) {
 			const uint64_t mid = (lo + hi) / 2;
 			if (a.items[item(mid)].col == col) {
@@ -1169,11 +1178,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 				hi = mid;
 			}
 		}
-		const uint64_t u0 = first << per, u1 = lo << per;
-		first             = lo;
-		// the CTA's first unit of the column at or after u0: one of warp gw .. gw + kStrWarps - 1 (mod nw)
-		const uint64_t mine = u0 + (gw + kStrWarps - 1 + nw - u0 % nw) % nw; // of the CTA's last warp
-		if (mine >= u1 + kStrWarps - 1) { continue; }
+		const uint64_t    u1   = lo << per;
 		const StrCol      c    = a.cols[col];
 		ulonglong2* const memo = reinterpret_cast<ulonglong2*>(a.memo + (static_cast<uint64_t>(col) << a.memo_bits));
 		const uint32_t    pairs = (1u << (a.memo_bits - 1)) - 1;
@@ -1357,6 +1362,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 				if (a.vclen) { atomicAdd(reinterpret_cast<unsigned long long*>(a.vclen + it), static_cast<unsigned long long>(sc * rs)); }
 			}
 		}
+		u0 = u1;
 	}
 }
 

@@ -1027,32 +1027,34 @@ __device__ __forceinline__ uint64_t str_load8_inside(const StrCol& c, uint64_t p
 // row, the exact figure the wizard's sizes need; rs > 1, the learned selector's features: the other rows'
 // compressed lengths are written as 0 and the vector's sum is scaled by rs).  The CTAs go through the columns one
 // after the other, a warp taking units of kStrUnit rows.
-//   memo     rows that another row of the column equals (dictionary-like columns: nearly all) take its compressed
-//            length from the column's part of a table in global memory, cleared for every call: an entry says where
-//            a row's bytes are, and both rows' bytes are compared.  A first launch over every `stride`-th vector fills
-//            it: all units start at once, so that without it nothing would be found.  With one table for all columns,
-//            those whose rows all differ would push the others' entries out;
+//   memo     rows that another row of the column equals take its compressed length from the column's part of a table in
+//            global memory, cleared for every call: an entry says where a row's bytes are, and both rows' bytes are
+//            compared (nothing follows from a hash).  A first launch over every `stride`-th vector fills it -- all
+//            units start at once, so that it finds nothing -- and counts the rows that it would have found; columns
+//            whose rows repeat (a quarter of those) look theirs up in the second launch.  With one table for all
+//            columns, those whose rows all differ would push the others' entries out;
 //   match    greedy matching looks at the next two bytes in a 64 KB table in shared memory (what they start: nothing,
 //            a one- or two-byte symbol, or a group of longer ones), so that only the few symbols of one group are
 //            compared, where the symbols sharing a first byte were walked one after the other;
 //   lanes    draw rows from the warp's list as they finish (8 at a time), four codes between two looks: rows of 1 to 20
 //            codes would otherwise leave most lanes idle.
-// 5.7 M rows of 6 columns (a third of the rows all different, 17 codes each): 1,677 us by rows and first-byte lists; for
-// the two launches 128 + 481 us with one memo for all columns, 123 + 255 us with one each and eight bytes loaded for
-// four codes, 57 + 298 us with units of 32 rows in the first launch.  Bound by instructions and the latency of the rows'
-// loads (issue slots half used, registers full).
+// 5.7 M rows of 6 columns (a third of the rows all different, 17 codes each): 1,677 us by rows and first-byte lists,
+// 45 + 312 us so.  Bound by instructions and the latency of the rows' loads (issue slots half used, registers full).  Whole
+// calls: the memo is worth 1,156 against 930 us for those (and 28 integer columns); of 4.6 M rows all different it
+// would cost 709 us where 488 are needed, so the columns are told apart.
 constexpr int      kStrWarps = 16;
-constexpr uint32_t kStrPer = 3, kStrUnit = 1024 >> kStrPer; // rows a warp takes at a time (log2 of a vector's units)
-constexpr uint32_t kStrFillPer = 5, kStrFillUnit = 1024 >> kStrFillPer; // one a lane in the launch that fills the memo
+// log2 of a vector's units: of 128 rows, and of 32, one a lane, where those would leave warps without one
+constexpr uint32_t kStrPer = 3, kStrUnit = 1024 >> kStrPer, kStrSmallPer = 5;
 // log2 of a column's memo entries: as many as the largest column has rows, at most 1 MB, and (down to the least) all
 // columns' at most 8 MB, which is cleared in a few microseconds and stays in L2
 constexpr uint32_t kStrMemoMin = 13, kStrMemoMax = 17, kStrMemoAll = 20;
+constexpr uint32_t kStrMemoVecs = 8; // a column's vectors, on average, in the launch that fills its part
 struct StrRowsSmem {
 	// by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g; behind them, by a row's last byte
 	uint8_t  pair[65536 + 256];
 	StrTab   t;
 	uint32_t off[kStrWarps][kStrUnit + 1]; // a unit's row offsets from its first row's
-	uint16_t list[kStrWarps][kStrUnit];    // rows to match; bit 15: which of its pair's memo entries a row takes
+	uint16_t list[kStrWarps][kStrUnit];    // rows to match
 };
 
 // What the string bytes in x, `left` of them still in the row, start (an entry of pair; its first two bytes are read).
@@ -1139,23 +1141,25 @@ struct StrRowsArgs {
 	const Item*   items; // by column
 	uint64_t      n_items;
 	uint64_t *    vlen, *vclen; // optional: sums of every item, zero before the first launch
-	uint64_t*     memo; // 1 << memo_bits entries for every column
+	uint64_t*     memo;   // 1 << memo_bits entries for every column; null: no memo
+	uint32_t*     repeats; // with it, for every column: rows of the launch that fills the memo, and how many another equals
 	uint32_t      memo_bits;
 	uint32_t      rs;
-	uint32_t      stride; // every stride-th item in the launch that fills the memo, the others in the next one
-	uint32_t      fill;
+	uint32_t      stride; // every stride-th item in the first launch, the others in the next one
+	uint32_t      first;
+	uint32_t      per; // log2 of a vector's units
 };
 
 __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArgs a) {
 	extern __shared__ __align__(16) uint8_t smem[];
 	StrRowsSmem&       S  = *reinterpret_cast<StrRowsSmem*>(smem);
 	constexpr uint32_t nt = kStrWarps * 32;
-	const uint32_t     unit = a.fill ? kStrFillUnit : kStrUnit, per = a.fill ? kStrFillPer : kStrPer; // rows; log2 of units
+	const uint32_t     per = a.per, unit = 1024u >> per; // rows of a unit
 	const uint32_t     tid = threadIdx.x, lane = tid & 31u, warp = tid >> 5, rs = a.rs;
-	// this launch's items: i * stride (fill), or the others in order; number i of them
-	const uint64_t n_fill = (a.n_items + a.stride - 1) / a.stride;
-	const uint64_t n      = a.fill ? n_fill : a.n_items - n_fill;
-	auto           item   = [&](uint64_t i) { return a.fill ? i * a.stride : a.stride == 1 ? i : i + i / (a.stride - 1) + 1; };
+	// this launch's items: i * stride (first), or the others in order; number i of them
+	const uint64_t n_first = (a.n_items + a.stride - 1) / a.stride;
+	const uint64_t n       = a.first ? n_first : a.n_items - n_first;
+	auto           item    = [&](uint64_t i) { return a.first ? i * a.stride : a.stride == 1 ? i : i + i / (a.stride - 1) + 1; };
 	const uint64_t gw = static_cast<uint64_t>(blockIdx.x) * kStrWarps, nw = static_cast<uint64_t>(gridDim.x) * kStrWarps;
 	// units are dealt to the warps round robin, over the columns' borders; a CTA goes from the column of its first unit to
 	// that of its first unit past it
@@ -1182,6 +1186,9 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 		const StrCol      c    = a.cols[col];
 		ulonglong2* const memo = reinterpret_cast<ulonglong2*>(a.memo + (static_cast<uint64_t>(col) << a.memo_bits));
 		const uint32_t    pairs = (1u << (a.memo_bits - 1)) - 1;
+		// rows are looked up only where the first launch found that they repeat
+		const bool look = a.memo && !a.first && a.repeats[2 * col + 1] >= a.repeats[2 * col] / 4;
+		uint32_t   rows = 0, repeats = 0;
 		__syncthreads(); // the previous column's table is read to the end
 		for (uint32_t k = tid; k < sizeof(StrTab) / 4; k += nt) {
 			reinterpret_cast<uint32_t*>(&S.t)[k] = __ldg(reinterpret_cast<const uint32_t*>(c.tab) + k);
@@ -1243,7 +1250,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 							c.len[r]         = m;
 							sl += m;
 							if ((r & 1023u) % rs == 0) {
-								ask_next = m <= kStrMemoLen && e <= room ? 1u : 2u; // 2: no entry, to be matched
+								ask_next = look && m <= kStrMemoLen && e <= room ? 1u : 2u; // 2: not looked up, to be matched
 								if (ask_next == 1) {
 									key_next  = str_memo_key(h, m);
 									seen_next = __ldcg(memo + (static_cast<uint32_t>(h) & pairs));
@@ -1277,9 +1284,8 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 							sc += cl;
 						}
 						const bool     miss = ask && !hit;
-						const uint32_t slot = seen.x == 0 ? 0u : seen.y == 0 ? 1u : static_cast<uint32_t>(key >> 57) & 1u;
 						const uint32_t m    = __ballot_sync(0xFFFFFFFFu, miss);
-						if (miss) { list[todo + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(row | slot << 15); }
+						if (miss) { list[todo + __popc(m & ((1u << lane) - 1u))] = static_cast<uint16_t>(row); }
 						todo += __popc(m);
 						row = row_next, ask = ask_next, key = key_next, seen = seen_next;
 					}
@@ -1293,7 +1299,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 								const uint32_t k = next + __popc(idle & ((1u << lane) - 1u));
 								have             = k < todo;
 								if (have) {
-									j                = list[k] & 0x7FFFu;
+									j                = list[k];
 									p                = off[j];
 									const uint32_t e = off[j + 1];
 									left             = e >= p ? e - p : 0;
@@ -1341,16 +1347,22 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 						}
 					}
 					__syncwarp();
-					for (uint32_t k = lane; k < todo; k += 32) { // what was matched, for the rows to come
-						const uint32_t i = list[k] & 0x7FFFu;
+					for (uint32_t k = a.memo && (a.first || look) ? lane : todo; k < todo; k += 32) { // what was matched, for the rows to come
+						const uint32_t i = list[k];
 						const uint64_t r = r0 + i;
 						const uint32_t l = c.clen[r];
 						const uint32_t b = off[i], e = off[i + 1], n = e >= b ? e - b : 0;
+						++rows;
 						if (n <= kStrMemoLen && l <= kStrMemoClen && e <= room && o0 + b < kStrMemoAtEnd) {
-							// into the entry of the pair that was free, or over one of the two
-							const uint64_t h = c.hash[r];
-							__stcg(reinterpret_cast<uint64_t*>(memo + (static_cast<uint32_t>(h) & pairs)) + (list[k] >> 15),
-							       str_memo_key(h, n) | ((o0 + b) << kStrMemoAtPos) | (l + 1));
+							const uint64_t   h = c.hash[r], k = str_memo_key(h, n);
+							ulonglong2*      at = memo + (static_cast<uint32_t>(h) & pairs);
+							const ulonglong2 had = __ldcg(at);
+							if ((had.x != 0 && (had.x & kStrMemoKey) == k) || (had.y != 0 && (had.y & kStrMemoKey) == k)) {
+								++repeats;
+							} else { // into the entry of the pair that is free, or over one of the two
+								const uint32_t slot = had.x == 0 ? 0u : had.y == 0 ? 1u : static_cast<uint32_t>(h >> 57) & 1u;
+								__stcg(reinterpret_cast<uint64_t*>(at) + slot, k | ((o0 + b) << kStrMemoAtPos) | (l + 1));
+							}
 						}
 					}
 				}
@@ -1362,12 +1374,20 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 				if (a.vclen) { atomicAdd(reinterpret_cast<unsigned long long*>(a.vclen + it), static_cast<unsigned long long>(sc * rs)); }
 			}
 		}
+		if (a.memo && a.first) {
+			rows    = warp_sum(rows);
+			repeats = warp_sum(repeats);
+			if (lane == 0 && rows) {
+				atomicAdd(a.repeats + 2 * col, rows);
+				atomicAdd(a.repeats + 2 * col + 1, repeats);
+			}
+		}
 		u0 = u1;
 	}
 }
 
-// k_str_rows over n_items vectors, two CTAs a SM: the launch that fills the memo over as many vectors as give every
-// warp a unit, then the rest.
+// k_str_rows over n_items vectors, two CTAs a SM; with the memo in two launches, the first over as many vectors as give
+// every warp a unit of 32 rows.
 cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_items, uint64_t* vlen, uint64_t* vclen,
                             uint32_t rs, uint64_t* memo, uint32_t memo_bits, uint64_t n_cols, cudaStream_t s) {
 	Device* d = current_device();
@@ -1375,17 +1395,22 @@ cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_it
 	static SmemLimit limit;
 	cudaError_t      e = limit.need(reinterpret_cast<const void*>(k_str_rows), sizeof(StrRowsSmem));
 	if (e != cudaSuccess) { return e; }
-	e = cudaMemsetAsync(memo, 0, (n_cols << memo_bits) * 8, s);
-	if (e == cudaSuccess && vlen) { e = cudaMemsetAsync(vlen, 0, n_items * 8, s); }
+	if (vlen) { e = cudaMemsetAsync(vlen, 0, n_items * 8, s); }
 	if (e == cudaSuccess && vclen) { e = cudaMemsetAsync(vclen, 0, n_items * 8, s); }
+	const uint64_t most = static_cast<uint64_t>(d->sm_count) * 2, warps = most * kStrWarps; // CTAs, warps
+	uint64_t       step = std::max<uint64_t>(1, ((n_items << kStrSmallPer) + warps - 1) / warps);
+	// the memo pays from some vectors a column in the first launch on, and when every row is matched
+	const bool keep = memo && rs == 1 && step > 1 && n_items / n_cols >= kStrMemoVecs * step;
+	step            = keep ? step : 1;
+	if (e == cudaSuccess && keep) { e = cudaMemsetAsync(memo, 0, (n_cols << memo_bits) * 8 + n_cols * 8, s); }
 	if (e != cudaSuccess) { return e; }
-	const uint64_t warps = static_cast<uint64_t>(d->sm_count) * 2 * kStrWarps, step = ((n_items << kStrFillPer) + warps - 1) / warps;
-	StrRowsArgs    a {cols, items, n_items, vlen, vclen, memo, memo_bits, rs, static_cast<uint32_t>(std::max<uint64_t>(1, step)), 1};
-	for (const uint32_t fill : {1u, 0u}) {
-		const uint64_t n_fill = (n_items + a.stride - 1) / a.stride, n = fill ? n_fill : n_items - n_fill;
-		const uint64_t units  = n << (fill ? kStrFillPer : kStrPer);
-		const uint64_t ctas   = std::min((units + kStrWarps - 1) / kStrWarps, static_cast<uint64_t>(d->sm_count) * 2);
-		a.fill                = fill;
+	StrRowsArgs a {cols, items, n_items, vlen, vclen, keep ? memo : nullptr, reinterpret_cast<uint32_t*>(memo + (n_cols << memo_bits)),
+	               memo_bits, rs, static_cast<uint32_t>(step), 1, 0};
+	for (const uint32_t first : {1u, 0u}) {
+		const uint64_t n_first = (n_items + step - 1) / step, n = first ? n_first : n_items - n_first;
+		a.first = first;
+		a.per   = (n << kStrPer) < warps ? kStrSmallPer : kStrPer;
+		const uint64_t ctas = std::min(((n << a.per) + kStrWarps - 1) / kStrWarps, most);
 		if (ctas) {
 			k_str_rows<<<static_cast<unsigned>(ctas), kStrWarps * 32, sizeof(StrRowsSmem), s>>>(a);
 			++launch_counter();
@@ -2300,7 +2325,12 @@ int fls_sel_plan_create_strings(const fls_sel_str_column* cols, uint32_t n_cols,
 	                                        (static_cast<uint64_t>(n_cols) << own->memo_bits) > (1ull << kStrMemoAll))) {
 		--own->memo_bits;
 	}
-	if (!own->str_memo.alloc((static_cast<uint64_t>(n_cols ? n_cols : 1) << own->memo_bits) * 8)) { return FLS_ERR_CUDA; }
+	// (of more columns the launch that fills the memo has too few vectors each: no memo)
+	const Device* dev = current_device();
+	if (n_cols && dev && static_cast<uint64_t>(n_cols) * kStrMemoVecs <= (static_cast<uint64_t>(dev->sm_count) * 2 * kStrWarps) >> kStrSmallPer &&
+	    !own->str_memo.alloc(((static_cast<uint64_t>(n_cols) << own->memo_bits) + n_cols) * 8)) {
+		return FLS_ERR_CUDA;
+	}
 	own->str   = true;
 	own->scols = sc;
 	own->hash_d.p = hash.p, hash.p = nullptr;

@@ -55,3 +55,50 @@ def test_rows_of_one_hash(cuda, n_vec):
         assert int(sizes[c, 0]) == frame + int(lens[part].sum()) + 4096 * nv
     assert P.device_status() == 0
     plan.close()
+
+
+def _plan_of(cuda, n_cols, n_vec, rng):
+    import torch
+
+    from fastlanes_b200 import select as SL
+
+    symbols = TABLES["long"]
+    rows = [bytes(rng.choice(np.frombuffer(b"abcdefghx", np.uint8), int(n))) for n in rng.integers(0, 30, n_vec * 1024)]
+    offs = np.concatenate([[0], np.cumsum([len(r) for r in rows])]).astype(np.int64)
+    data = torch.from_numpy(np.frombuffer(b"".join(rows), np.uint8).copy()).to(cuda)
+    return SL.StrSelectionPlan([(data, torch.from_numpy(offs).to(cuda), _table(symbols))] * n_cols), rows, symbols
+
+
+def _launches(call):
+    import torch
+
+    from fastlanes_b200._lib import lib
+
+    lib.fls_gpu_launch_count(1)
+    call()
+    torch.cuda.synchronize()
+    return lib.fls_gpu_launch_count(0)
+
+
+def test_statistics_take_every_fourth_row(cuda):
+    """The compressed share of a vector (statistic 1) is that of its rows 0, 4, 8, ..., in one launch over the rows."""
+    plan, rows, symbols = _plan_of(cuda, 1, 200, np.random.default_rng(2))
+    feat = plan.features(3)[0].cpu().numpy()
+    assert _launches(lambda: plan.features(3)) == 3  # rows, integer statistics, string statistics
+    for i, v in enumerate(v for c in range(0, 200, 64) for v in range(c, min(c + 64, 200), 3)):
+        part = rows[v * 1024:(v + 1) * 1024]
+        want = 4.0 * sum(_compressed(r, symbols) for r in part[::4]) / sum(map(len, part))
+        assert abs(feat[i, 1] - want) < 1e-6 * want  # whole numbers below 2^24 in float32, one division
+    plan.close()
+
+
+@pytest.mark.parametrize("n_cols,n_vec,launches", [(1, 100, 1), (1, 400, 2), (18, 90, 2), (18, 20, 1), (30, 90, 1)])
+def test_first_launch_only_where_it_pays(cuda, n_cols, n_vec, launches):
+    """The launch that fills the memo runs for few columns of many vectors alone (on 148 SMs)."""
+    import torch
+
+    if torch.cuda.get_device_properties(cuda).multi_processor_count != 148:
+        pytest.skip("the limits are those of 148 SMs")
+    plan, _, _ = _plan_of(cuda, n_cols, n_vec, np.random.default_rng(3))
+    assert _launches(plan.wizard) == launches + 3  # parts, dictionaries, sizes
+    plan.close()

@@ -390,3 +390,47 @@ extern "C" void emu_dict_layout(uint64_t d8, uint64_t packed, uint64_t entries, 
 	const uint32_t   x[6] = {l.mode, l.warps, l.window, l.dict_cap, l.smem, rows16 ? kDictRows16 : kDictRows32};
 	std::memcpy(out, x, sizeof(x));
 }
+
+// One FSST vector as the single-pass kernel (k_stream_single) decodes it, on an emulated warp: its total by fsst_total, by
+// the general walk where that does not stand, then offsets (1025) and bytes from position vbase.  Returns the total the
+// vector publishes; *got what was written, *lone whether its escapes stood alone.
+extern "C" uint64_t emu_stream_single(const uint64_t* sym, const uint8_t* len, const uint32_t* ends, const uint8_t* comp,
+                                      uint32_t n, uint64_t vbase, uint32_t* offsets, uint8_t* out, uint64_t* got, int* lone) {
+	std::vector<uint32_t> rows(kVec + kVec / 32 + 32, 0);
+	for (uint32_t r = 0; r < kVec; ++r) { rows[r + r / 32] = ends[r]; }
+	std::vector<uint64_t> tsym(sym, sym + 256);
+	std::vector<uint8_t>  tlen(len, len + 256);
+	tsym[255] = 0; // the kernel's shared copy: the escape with an empty entry
+	tlen[255] = 0;
+	std::vector<uint8_t> win_buf(2048 + 64, 0xA5);
+	uint8_t*             win = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(win_buf.data()) + 15) & ~uintptr_t(15));
+	uint32_t             total = 0, wrote = 0;
+	std::barrier<>       bar(32);
+	EmuWarp              w {&bar, {}, {}};
+	std::vector<std::thread> th;
+	for (uint32_t t = 0; t < 32; ++t) {
+		th.emplace_back([&, t] {
+			g_emu_warp = &w;
+			g_emu_lane = static_cast<int>(t);
+			bool           bad = false;
+			const uint32_t L   = stream_rows_length(rows.data(), n, t, &bad);
+			uint32_t       T   = L;
+			const bool     one = fsst_total<true>(rows.data(), comp, L, tlen.data(), t, &T);
+			if (!one) {
+				StreamOut o {};
+				T = stream_vector<false, true, 2048>(rows.data(), comp, n, tsym.data(), tlen.data(), t, o, &bad);
+			}
+			StreamOut      o {offsets, out, vbase, win};
+			const uint32_t x = stream_vector<true, true, 2048>(rows.data(), comp, n, tsym.data(), tlen.data(), t, o, &bad, one);
+			if (t == 0) {
+				total = T;
+				wrote = x;
+				*lone = one ? 1 : 0;
+			}
+		});
+	}
+	for (auto& x : th) { x.join(); }
+	offsets[kVec] = static_cast<uint32_t>(vbase + wrote);
+	*got          = wrote;
+	return total;
+}

@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(1024) k_pack_offsets(const uint8_t* __restrict
 		const uint64_t u1  = u0 + 1024 * 1024 < v0 ? u0 + 1024 * 1024 : v0;
 		uint32_t       sum = 0;
 		for (uint64_t u = u0 + tid * 16; u < u1; u += 1024 * 16) {
-			uint8_t b[16];
+			__align__(16) uint8_t b[16];
 			if (wide) {
 				*reinterpret_cast<uint4*>(b) = __ldg(reinterpret_cast<const uint4*>(bw + u));
 			} else {
@@ -338,8 +338,11 @@ FLS_ENC2(uint64_t, 64)
 int fls_gpu_pack_offsets(const uint8_t* d_bw, uint64_t n_vec, uint32_t width, uint64_t* d_byte_off, uint64_t* d_total,
                          fls_stream_t stream) {
 	if (!d_total || ((!d_bw || !d_byte_off) && n_vec)) { return FLS_ERR_ARG; }
+	const Device* d = current_device();
+	if (!d) { return FLS_ERR_CUDA; }
 	// stretches of whole turns, as many as there are turns up to one a SM
-	const uint64_t turns = (n_vec + kPoTurn - 1) / kPoTurn, per = kPoTurn * ((turns + 147) / 148);
+	const uint64_t sms = static_cast<uint64_t>(d->sm_count), turns = (n_vec + kPoTurn - 1) / kPoTurn;
+	const uint64_t per = kPoTurn * ((turns + sms - 1) / sms);
 	const unsigned grid  = static_cast<unsigned>(per ? (n_vec + per - 1) / per : 1);
 	k_pack_offsets<<<grid, 1024, 0, static_cast<cudaStream_t>(stream)>>>(d_bw, n_vec, width, d_byte_off, d_total, per);
 	++launch_counter();

@@ -187,12 +187,13 @@ __device__ __forceinline__ uint32_t pack_parts(const Parts& p) {
 // ---------------------------------------------------------------------------------------------------------
 constexpr uint32_t kHSlots = 2048;
 
+// the odd multipliers are xxHash's 32-bit primes 1, 2 and 3 (Collet)
 template <class T>
 __device__ __forceinline__ uint32_t feat_hash(T x) {
 	uint32_t a = static_cast<uint32_t>(x) * 0x9E3779B1u;
 	if constexpr (sizeof(T) == 8) { a += static_cast<uint32_t>(x >> 32) * 0x85EBCA77u; }
 	a ^= a >> 15;
-	a *= 0x2C1B3C6Du;
+	a *= 0xC2B2AE3Du;
 	return a ^ (a >> 13);
 }
 

@@ -1049,7 +1049,8 @@ constexpr uint32_t kStrPer = 3, kStrUnit = 1024 >> kStrPer, kStrSmallPer = 5;
 // log2 of a column's memo entries: as many as the largest column has rows, at most 1 MB, and (down to the least) all
 // columns' at most 8 MB, which is cleared in a few microseconds and stays in L2
 constexpr uint32_t kStrMemoMin = 13, kStrMemoMax = 17, kStrMemoAll = 20;
-constexpr uint32_t kStrMemoVecs = 8; // a column's vectors, on average, in the launch that fills its part
+// a column's vectors, on average: at least for a memo, and in the launch that fills it
+constexpr uint32_t kStrMemoVecs = 32, kStrMemoFill = 8;
 struct StrRowsSmem {
 	// by the next two bytes: 0 escape, 1 / 2 a symbol of that length, kStrGroup + g; behind them, by a row's last byte
 	uint8_t  pair[65536 + 256];
@@ -1388,7 +1389,7 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 }
 
 // k_str_rows over n_items vectors, two CTAs a SM; with the memo in two launches, the first over as many vectors as give
-// every warp a unit of 32 rows.
+// every warp a unit of 32 rows, or more.
 cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_items, uint64_t* vlen, uint64_t* vclen,
                             uint32_t rs, uint64_t* memo, uint32_t memo_bits, uint64_t n_cols, cudaStream_t s) {
 	Device* d = current_device();
@@ -1400,9 +1401,10 @@ cudaError_t launch_str_rows(const StrCol* cols, const Item* items, uint64_t n_it
 	if (e == cudaSuccess && vclen) { e = cudaMemsetAsync(vclen, 0, n_items * 8, s); }
 	const uint64_t most = static_cast<uint64_t>(d->sm_count) * 2, warps = most * kStrWarps; // CTAs, warps
 	uint64_t       step = std::max<uint64_t>(1, ((n_items << kStrSmallPer) + warps - 1) / warps);
-	// the memo pays from some vectors a column in the first launch on, and when every row is matched
-	const bool keep = memo && rs == 1 && step > 1 && n_items / n_cols >= kStrMemoVecs * step;
-	step            = keep ? step : 1;
+	// the memo pays for columns of some vectors, when every row is matched; the first launch takes at least some of each
+	const uint64_t vecs = n_items / n_cols;
+	const bool     keep = memo && rs == 1 && step > 1 && vecs >= kStrMemoVecs;
+	step                = keep ? std::min<uint64_t>(step, vecs / kStrMemoFill) : 1;
 	if (e == cudaSuccess && keep) { e = cudaMemsetAsync(memo, 0, (n_cols << memo_bits) * 8 + n_cols * 8, s); }
 	if (e != cudaSuccess) { return e; }
 	StrRowsArgs a {cols, items, n_items, vlen, vclen, keep ? memo : nullptr, reinterpret_cast<uint32_t*>(memo + (n_cols << memo_bits)),
@@ -2326,9 +2328,7 @@ int fls_sel_plan_create_strings(const fls_sel_str_column* cols, uint32_t n_cols,
 	                                        (static_cast<uint64_t>(n_cols) << own->memo_bits) > (1ull << kStrMemoAll))) {
 		--own->memo_bits;
 	}
-	// (of more columns the launch that fills the memo has too few vectors each: no memo)
-	const Device* dev = current_device();
-	if (n_cols && dev && static_cast<uint64_t>(n_cols) * kStrMemoVecs <= (static_cast<uint64_t>(dev->sm_count) * 2 * kStrWarps) >> kStrSmallPer &&
+	if (n_cols && rows / 1024 / n_cols >= kStrMemoVecs &&
 	    !own->str_memo.alloc(((static_cast<uint64_t>(n_cols) << own->memo_bits) + n_cols) * 8)) {
 		return FLS_ERR_CUDA;
 	}

@@ -92,9 +92,10 @@ def test_statistics_take_every_fourth_row(cuda):
     plan.close()
 
 
-@pytest.mark.parametrize("n_cols,n_vec,launches", [(1, 100, 1), (1, 400, 2), (18, 90, 2), (18, 20, 1), (30, 90, 1)])
+@pytest.mark.parametrize("n_cols,n_vec,launches", [(1, 100, 1), (1, 400, 2), (18, 90, 2), (40, 30, 1), (40, 33, 2)])
 def test_first_launch_only_where_it_pays(cuda, n_cols, n_vec, launches):
-    """The launch that fills the memo runs for few columns of many vectors alone (on 148 SMs)."""
+    """The launch that fills the memo runs for columns of 32 vectors and more, and not for so few vectors that one launch over
+    all of them is all there is (on 148 SMs)."""
     import torch
 
     if torch.cuda.get_device_properties(cuda).multi_processor_count != 148:

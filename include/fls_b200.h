@@ -346,7 +346,7 @@ int fls_string_plan_destroy(fls_string_plan* plan);
  *   another kind).  bind: each column's outputs (as fls_string_plan_decode's: n_rows + 1 u32 offsets, 16-byte
  *   aligned bytes, capacity < 4 GiB); synchronous, once.  decode: asynchronous, no allocation, capturable in a
  *   CUDA graph; decodes of one set whose work overlaps on the GPU race on its scratch.  Device memory a set
- *   holds: 8 bytes per vector and per column.
+ *   holds: 8 bytes per vector and 16 per column.
  * ------------------------------------------------------------------------------------------------------- */
 typedef struct fls_string_set fls_string_set;
 int fls_string_set_create(const fls_string_plan* const* plans, uint32_t n, fls_string_set** out_set);

@@ -1356,14 +1356,14 @@ __global__ void __launch_bounds__(kStrWarps * 32, 2) k_str_rows(const StrRowsArg
 						const uint32_t b = off[i], e = off[i + 1], n = e >= b ? e - b : 0;
 						++rows;
 						if (n <= kStrMemoLen && l <= kStrMemoClen && e <= room && o0 + b < kStrMemoAtEnd) {
-							const uint64_t   h = c.hash[r], k = str_memo_key(h, n);
+							const uint64_t   h = c.hash[r], key = str_memo_key(h, n);
 							ulonglong2*      at = memo + (static_cast<uint32_t>(h) & pairs);
 							const ulonglong2 had = __ldcg(at);
-							if ((had.x != 0 && (had.x & kStrMemoKey) == k) || (had.y != 0 && (had.y & kStrMemoKey) == k)) {
+							if ((had.x != 0 && (had.x & kStrMemoKey) == key) || (had.y != 0 && (had.y & kStrMemoKey) == key)) {
 								++repeats;
 							} else { // into the entry of the pair that is free, or over one of the two
 								const uint32_t slot = had.x == 0 ? 0u : had.y == 0 ? 1u : static_cast<uint32_t>(h >> 57) & 1u;
-								__stcg(reinterpret_cast<uint64_t*>(at) + slot, k | ((o0 + b) << kStrMemoAtPos) | (l + 1));
+								__stcg(reinterpret_cast<uint64_t*>(at) + slot, key | ((o0 + b) << kStrMemoAtPos) | (l + 1));
 							}
 						}
 					}

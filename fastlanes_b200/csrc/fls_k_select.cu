@@ -469,7 +469,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_features(ItemArgs a, float* 
 //             position of its first occurrence seen so far (the chunk's values stay in L2, so the key itself is read
 //             back from that position when the hash bits agree).  A slot of 4 bytes instead of a 64-bit key and a
 //             position (12) is what lets one table hold most of a chunk of distinct values;
-//   queue     a warp takes whole vectors, and every step looks at one slot for each of 32 keys from the warp's queue
+//   queue     a warp takes whole vectors (in chunks of few, some rows of one), and every step looks at one slot for each
+//             of 32 keys from the warp's queue
 //             in shared memory; keys that have to look further go back on it.  So runs, other parts' keys and long
 //             probes cost no idle lanes (a loop of its own for every warp of keys went round for its unluckiest
 //             lane, 200 to 300 instructions a step);
@@ -657,7 +658,12 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 	volatile uint32_t* over = &S.over;
 	uint64_t           sw0 = 0, sw1 = 0; // weights of the first positions this thread finds
 	CdQueue<T>         Q {reinterpret_cast<T*>(S.qkey[warp]), S.qpos[warp], S.qslot[warp], S.qtag[warp], nullptr, 0, 0, 0};
-	constexpr uint32_t kPer = kMaxVecPerChunk / kCdWarps; // vectors of a warp: warp, warp + kCdWarps
+	// a warp's units: warp, warp + kCdWarps.  A unit is a vector, or some of its rows where there are fewer vectors than
+	// half the warps (4,096 chunks of one vector: 973 us with a warp each, 293 so)
+	constexpr uint32_t kPer  = kMaxVecPerChunk / kCdWarps;
+	const uint32_t     split = nv < kCdWarps ? 31 - __clz(kCdWarps / nv) : 0; // log2 of a vector's units
+	const uint32_t     units = nv << split, unit_rows = 32u >> split;
+	auto               first_row = [&](uint32_t u) { return (u << (5 - split)) & 31u; };
 	uint32_t           listed[kPer];
 	auto clear = [&](uint32_t words) { // of the table
 		for (uint32_t k = tid; k < words / 4; k += kCdThreads) {
@@ -672,22 +678,23 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 		}
 		sw0 = sw1 = 0;
 	};
-	// row r of vector v: this lane's value, and whether it starts a run (a vector's first value counts as one)
+	// row r of vector v: this lane's value, and whether it starts a run (the first value of row r0, a unit's first, counts
+	// as one)
 	T    last = 0;
-	auto row  = [&](uint32_t v, uint32_t r, T* x) {
+	auto row  = [&](uint32_t v, uint32_t r, uint32_t r0, T* x) {
 		*x     = __ldg(vals + v * 1024 + r * 32 + lane);
 		T prev = __shfl_up_sync(0xFFFFFFFFu, *x, 1);
 		if (lane == 0) { prev = last; }
 		last = __shfl_sync(0xFFFFFFFFu, *x, 31);
-		return *x != prev || (r == 0 && lane == 0);
+		return *x != prev || (r == r0 && lane == 0);
 	};
 	// the ranges of the warp's vectors from their slots (the table holds the first positions), and the first positions
 	// themselves; the table is read to the end at the closing barrier
 	auto collect = [&](uint32_t n_slots) {
 #pragma unroll
 		for (uint32_t j = 0; j < kPer; ++j) {
-			const uint32_t  v    = warp + j * kCdWarps;
-			const uint16_t* list = slots + v * 1024;
+			const uint32_t  u    = warp + j * kCdWarps;
+			const uint16_t* list = slots + u * unit_rows * 32;
 			uint32_t        lo = ~0u, hi = 0u;
 #pragma unroll 4
 			for (uint32_t i = lane; i < listed[j]; i += 32) {
@@ -697,9 +704,9 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 			}
 			lo = __reduce_min_sync(0xFFFFFFFFu, lo);
 			hi = __reduce_max_sync(0xFFFFFFFFu, hi);
-			if (lane == 0 && lo != ~0u) { // (the parts' turns are one after the other)
-				S.vrange[v][0] = min(S.vrange[v][0], lo);
-				S.vrange[v][1] = max(S.vrange[v][1], hi);
+			if (lane == 0 && lo != ~0u) {
+				atomicMin(&S.vrange[u >> split][0], lo);
+				atomicMax(&S.vrange[u >> split][1], hi);
 			}
 		}
 #pragma unroll 4
@@ -723,28 +730,28 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 		clear(kCdSlots);
 		__syncthreads();
 		auto entry = [&](T x) { return S.table + static_cast<uint32_t>(static_cast<T>((x ^ flip) - low)); };
-		for (uint32_t v = warp; v < nv; v += kCdWarps) {
+		for (uint32_t u = warp; u < units; u += kCdWarps) {
 #pragma unroll 8
-			for (uint32_t r = 0; r < 32; ++r) {
-				const uint32_t pos = v * 1024 + r * 32 + lane;
+			for (uint32_t r = 0; r < unit_rows; ++r) {
+				const uint32_t pos = (u * unit_rows + r) * 32 + lane;
 				uint32_t*      e   = entry(__ldg(vals + pos));
 				if (pos < *reinterpret_cast<volatile uint32_t*>(e)) { atomicMin(e, pos); }
 			}
 		}
 		__syncthreads();
-		for (uint32_t v = warp; v < nv; v += kCdWarps) {
+		for (uint32_t u = warp; u < units; u += kCdWarps) {
 			uint32_t lo = ~0u, hi = 0u;
 #pragma unroll 8
-			for (uint32_t r = 0; r < 32; ++r) {
-				const uint32_t f = *entry(__ldg(vals + v * 1024 + r * 32 + lane));
+			for (uint32_t r = 0; r < unit_rows; ++r) {
+				const uint32_t f = *entry(__ldg(vals + (u * unit_rows + r) * 32 + lane));
 				lo               = min(lo, f);
 				hi               = max(hi, f);
 			}
 			lo = __reduce_min_sync(0xFFFFFFFFu, lo);
 			hi = __reduce_max_sync(0xFFFFFFFFu, hi);
 			if (lane == 0) {
-				S.vrange[v][0] = lo;
-				S.vrange[v][1] = hi;
+				atomicMin(&S.vrange[u >> split][0], lo);
+				atomicMax(&S.vrange[u >> split][1], hi);
 			}
 		}
 #pragma unroll
@@ -766,7 +773,7 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 #pragma unroll
 				for (uint32_t i = 0; i < 4; ++i) {
 					T          x;
-					const bool start = row(v, r0 + i, &x);
+					const bool start = row(v, r0 + i, 0, &x);
 					uint32_t   place, other;
 					cd_hash(x, &place, &other);
 					const uint32_t b = place >> 12;
@@ -802,7 +809,7 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 				for (uint32_t r = 0; r < 32 && v < nv; ++r) {
 					if (__any_sync(0xFFFFFFFFu, *over != 0)) { break; } // one answer for the whole warp
 					T          x;
-					const bool start = row(v, r, &x);
+					const bool start = row(v, r, 0, &x);
 					uint32_t   place, other;
 					cd_hash(x, &place, &other);
 					const uint32_t pos  = v * 1024 + r * 32 + lane;
@@ -846,14 +853,14 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 			__syncthreads();
 #pragma unroll
 			for (uint32_t j = 0; j < kPer; ++j) {
-				const uint32_t v    = warp + j * kCdWarps;
+				const uint32_t u = warp + j * kCdWarps, v = u >> split, r0 = first_row(u), r1 = r0 + unit_rows;
 				uint32_t       rows = 0;
-				Q.list = slots + v * 1024;
+				Q.list = slots + u * unit_rows * 32;
 				Q.q = Q.n = 0;
-				for (uint32_t r = 0; r < 32 && v < nv; ++r) {
+				for (uint32_t r = r0; r < r1 && v < nv; ++r) {
 					if (__any_sync(0xFFFFFFFFu, *over != 0)) { break; } // one answer for the whole warp
 					T        x;
-					bool     need = row(v, r, &x);
+					bool     need = row(v, r, r0, &x);
 					uint32_t place, other;
 					cd_hash(x, &place, &other);
 					need = need && cd_part(other, parts_log) == part;
@@ -866,12 +873,12 @@ __device__ __forceinline__ void chunk_dict(const ChunkDictArgs& a, const Col& co
 						Q.push(need, x, pos, s, tag, lane);
 						looked = Q.q >= 32;
 					}
-					if (!Q.drain(S.table, kCdSlots, vals, r == 31, lane, &fresh)) {
+					if (!Q.drain(S.table, kCdSlots, vals, r + 1 == r1, lane, &fresh)) {
 						if (lane == 0) { S.spent = *over = 1; }
 						break;
 					}
 					++rows;
-					if (lane == 0 && (looked || r == 31)) {
+					if (lane == 0 && (looked || r + 1 == r1)) {
 						// room left, and room for the chunk if the keys go on coming at this rate?
 						const uint32_t now = atomicAdd(&S.count, (rows << 16) + fresh) + (rows << 16) + fresh;
 						const uint32_t n = now & 0xFFFFu, done = now >> 16;

@@ -470,17 +470,16 @@ __global__ void __launch_bounds__(kWarps * 32, 2) k_features(ItemArgs a, float* 
 //             back from that position when the hash bits agree).  A slot of 4 bytes instead of a 64-bit key and a
 //             position (12) is what lets one table hold most of a chunk of distinct values;
 //   queue     a warp takes whole vectors (in chunks of few, some rows of one), and every step looks at one slot for each
-//             of 32 keys from the warp's queue
-//             in shared memory; keys that have to look further go back on it.  So runs, other parts' keys and long
-//             probes cost no idle lanes (a loop of its own for every warp of keys went round for its unluckiest
-//             lane, 200 to 300 instructions a step);
+//             of 32 keys from the warp's queue in shared memory; keys that have to look further go back on it.  So
+//             runs, other parts' keys and long probes cost no idle lanes (a loop of its own for every warp of keys
+//             went round for its unluckiest lane, 200 to 300 instructions a step);
 //   parts     a chunk of more distinct values goes through the table in parts of the hash space (2, then 4); the count
 //             beside the rows done says early whether it will;
 //   sort      keys that crowd, whatever the reason (every hash has such keys), spend a warp's looks or overflow four
 //             parts: their chunk's positions are sorted by value instead.
 // Exact for every chunk: the hash only decides how long it takes.  Instruction-bound.  28 integer columns (30 M values, 462
-// chunks): 1,855 us with 16 Ki slots of keys and positions and a bucket pass through global memory, 284 us so; 5.7 M
-// string hashes (90 chunks): 710 us, 138 us.
+// chunks): 1,855 us with 16 Ki slots of keys and positions and a bucket pass through global memory, 275 us so; 5.7 M
+// string hashes (90 chunks): 710 us, 139 us.
 // ---------------------------------------------------------------------------------------------------------
 constexpr uint32_t kCdThreads = 1024;
 constexpr uint32_t kCdWarps   = kCdThreads / 32;
@@ -567,7 +566,7 @@ __device__ __forceinline__ void cd_choose(const ChunkDictArgs& a, uint32_t i0, u
 // First positions and vector ranges of a chunk without a hash: its positions (order: space for them in global memory)
 // sorted by value and then position with Batcher's merge exchange (Knuth, The Art of Computer Programming 3, algorithm
 // 5.2.2M), so that the positions of a value stand side by side, the first one in front.  136 passes over 65,536
-// positions: some milliseconds a chunk, however its keys are made.
+// positions: 15 ms for a chunk with the looks spent before, however its keys are made (0.13 ms for keys that spread).
 template <class T>
 __device__ __noinline__ void cd_sort(const T* vals, uint32_t nv, uint16_t* order, const uint32_t* w0, const uint32_t* w1,
                                      ChunkDictSmem& S) {

@@ -13,18 +13,41 @@ namespace {
 // Positions of the set bits of the vector's bitmap (lane l holds word l, bits 32l .. 32l + 31) in ascending
 // order into idx (global, 1024 entries); returns the count (every lane).  s: the warp's 1024 entries of shared
 // memory, 16-byte aligned.
-// One bitmap word a step, a bit a lane: a word's positions land side by side, so the shared-memory stores have no
-// bank conflicts (a lane walking its own word's bits stored 2 bytes at a stride of up to 64), words without a
-// bit cost nothing, and the list leaves in 16-byte stores.  16,001 vectors, half of the bits set: 57.5 us
-// before, 12.4 us now (both from cold caches).
+// A lane walks its own word's bits, as many steps as the fullest word has bits: straight to global memory when those are
+// few, else into shared memory, from where the list leaves in 16-byte stores.  Where fewer words hold a bit than the
+// fullest has bits (nearly all bits set, or clusters), one word a step, a bit a lane: its positions land side by side,
+// without bank conflicts, and words without a bit cost nothing.  40,000 vectors (us, lanes walking to global memory / a
+// word a step / now): 3 % of the bits set 12.3 / 34.8 / 12.3, 15 % 22.5 / 49.2 / 18.4, half 121 / 49 / 27, all 266 / 49 / 21.
 __device__ __forceinline__ uint32_t compact_bits(uint32_t word, uint32_t lane, uint16_t* s, uint16_t* idx) {
+	if (__all_sync(0xFFFFFFFFu, word == ~0u)) { // the whole vector, as a filter of sorted values has it
+		if ((reinterpret_cast<uintptr_t>(idx) & 15u) == 0) {
+#pragma unroll
+			for (uint32_t j = 0; j < 4; ++j) {
+				const uint32_t i = j * 32 + lane, x = i * 0x00080008u + 0x00010000u; // positions 8 i, 8 i + 1
+				reinterpret_cast<uint4*>(idx)[i] = make_uint4(x, x + 0x00020002u, x + 0x00040004u, x + 0x00060006u);
+			}
+		} else {
+			for (uint32_t i = lane; i < 1024; i += 32) { idx[i] = static_cast<uint16_t>(i); }
+		}
+		return 1024;
+	}
 	uint32_t       n    = 0;
 	const uint32_t some = __ballot_sync(0xFFFFFFFFu, word != 0); // words that hold a bit
-	for (uint32_t rest = some; rest; rest &= rest - 1) {
-		const uint32_t k = __ffs(rest) - 1;
-		const uint32_t w = __shfl_sync(0xFFFFFFFFu, word, k);
-		if ((w >> lane) & 1u) { s[n + __popc(w & ((1u << lane) - 1u))] = static_cast<uint16_t>(32 * k + lane); }
-		n += __popc(w);
+	const uint32_t mine = __popc(word), most = __reduce_max_sync(0xFFFFFFFFu, mine);
+	const bool     direct = most <= 8;
+	if (direct || most < static_cast<uint32_t>(__popc(some))) {
+		const uint32_t inc = warp_inclusive_scan(mine, lane);
+		uint16_t*      to  = direct ? idx : s;
+		for (uint32_t at = inc - mine; word; word &= word - 1) { to[at++] = static_cast<uint16_t>(32 * lane + __ffs(word) - 1); }
+		n = __shfl_sync(0xFFFFFFFFu, inc, 31);
+		if (direct) { return n; }
+	} else {
+		for (uint32_t rest = some; rest; rest &= rest - 1) {
+			const uint32_t k = __ffs(rest) - 1;
+			const uint32_t w = __shfl_sync(0xFFFFFFFFu, word, k);
+			if ((w >> lane) & 1u) { s[n + __popc(w & ((1u << lane) - 1u))] = static_cast<uint16_t>(32 * k + lane); }
+			n += __popc(w);
+		}
 	}
 	__syncwarp();
 	if ((reinterpret_cast<uintptr_t>(idx) & 15u) == 0) {
@@ -39,8 +62,10 @@ __device__ __forceinline__ uint32_t compact_bits(uint32_t word, uint32_t lane, u
 	return n;
 }
 
-__global__ void __launch_bounds__(256) k_bitmap_to_selection(const uint32_t* __restrict__ bm, uint64_t n_vec,
-                                                             uint16_t* __restrict__ idx, uint16_t* __restrict__ count) {
+// (8 CTAs an SM, 32 registers a thread, here and in the next kernel: with 6 of them the intersection of full lists took 399
+// us, 313 so)
+__global__ void __launch_bounds__(256, 8) k_bitmap_to_selection(const uint32_t* __restrict__ bm, uint64_t n_vec,
+                                                                uint16_t* __restrict__ idx, uint16_t* __restrict__ count) {
 	__shared__ __align__(16) uint16_t list[8][1024];
 	const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x / 32;
 	const uint64_t nw   = static_cast<uint64_t>(gridDim.x) * (blockDim.x / 32);
@@ -78,9 +103,9 @@ __device__ __forceinline__ bool list_bits(const uint16_t* idx, uint32_t n, uint3
 	return !__any_sync(0xFFFFFFFFu, bad);
 }
 
-__global__ void k_selection_and(const uint16_t* __restrict__ i0, const uint16_t* __restrict__ c0,
-                                const uint16_t* __restrict__ i1, const uint16_t* __restrict__ c1, uint16_t* io,
-                                uint16_t* co, uint64_t n_vec, int* status) {
+__global__ void __launch_bounds__(256, 8) k_selection_and(const uint16_t* __restrict__ i0, const uint16_t* __restrict__ c0,
+                                                          const uint16_t* __restrict__ i1, const uint16_t* __restrict__ c1,
+                                                          uint16_t* io, uint16_t* co, uint64_t n_vec, int* status) {
 	__shared__ uint32_t               bits[8][2][32];
 	__shared__ __align__(16) uint16_t list[8][1024];
 	const uint32_t      lane = threadIdx.x & 31u, warp = threadIdx.x / 32;
